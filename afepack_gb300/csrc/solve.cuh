@@ -86,8 +86,10 @@ void permute_csr(const afp_context* ctx, int64_t m, const int* rowptr, const int
                  DevBuf<double>& out_vals);
 // d_j = a_jj + sum_{k in [r0,r1), k != j} |a_jk| for j in [r0, r1)
 void l1_diag(const afp_context* ctx, const CSRView<double>& A, int64_t r0, int64_t r1, double* d);
-// Dense inverse of the n x n CSR matrix by Gauss-Jordan elimination with
-// partial pivoting; returns false when a pivot is zero.
+// Inverts the dense symmetric positive definite n x n M in place
+// (spd_inverse.cu); false, with M undefined, when it is not.
+bool spd_inverse(const afp_context* ctx, int64_t n, double* M);
+// Dense inverse of the n x n CSR matrix; returns false when it is singular.
 bool dense_inverse(const afp_context* ctx, const CSRView<double>& A, double* inv);
 
 }  // namespace afp

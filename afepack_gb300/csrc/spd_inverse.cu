@@ -1,0 +1,530 @@
+// Dense inverse of a symmetric positive definite matrix (the coarsest level
+// of the hierarchy), with the cubic work on the tensor cores.
+//
+// Block sweep in place on the lower triangle, kB pivots at a time.  With the
+// pivot block P, Q = P^-1, the panel C (rows of the panel's columns; for rows
+// already swept the panel's rows, transposed) and the rest S,
+//   S_ij <- S_ij -+ (C_i Q) C_j^T,   C_i <- -+ C_i Q,   P <- Q
+// (minus for rows below the panel, plus for rows already swept), which after
+// the last panel leaves the inverse.  Symmetry halves the work; a positive
+// definite matrix needs no pivoting, as every block pivot is a Schur
+// complement of it.
+//
+// FP64 arithmetic runs at 2 multiply-adds a clock and SM here, so the n^3
+// part of a 6,744-row inverse is at least 0.25 s in FP64 even with symmetry.
+// The two products of a panel are therefore formed from exact pieces on the
+// tensor cores (Ozaki, Ogita, Oishi, Rump, Numer. Algorithms 59, 2012): every
+// row is scaled by a power of two and cut into kS = 9 signed digits of 7 bits
+// (|d| <= 64; the cut rounds at 2^-63 of the row's scale), digit i stored
+// times 2^-7i in BF16, which holds it exactly.  In units of their weight a
+// product of two digits is at most 2^12 and a sum over kB = 256 inner indices
+// and up to 8 digit pairs of one weight at most 2^23, so the FP32
+// accumulators of the weights 0..7 are exact.  Weight 8 shares the last
+// accumulator (its rounding is 2^-24 of weight 7); the pairs below are left
+// out.  An entry's eight sums are put together in 64-bit integers and FP64.
+// On grid matrices of 576 rows with coefficients of contrast 1, 1e4 and 1e8
+// the inverse is as far from an extended-precision one as the same sweep with
+// FP64 products: 2.2e-15, 8e-14 and 2e-11 of its norm on either side; with
+// 8 digits the small entries of the last two were 40 and more times worse.
+//
+// Measured (GB300, whole inverse): 6,744 rows 49 ms against 706 ms with the
+// pivoted FP64 sweep of solve.cu (two launches per pivot, FP64 products);
+// 2,196 rows 4.5 against 68 ms.  At 6,744 rows the trailing updates take 36
+// of the 49 ms, the panels' own inverses 8.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "common.cuh"
+#include "solve.cuh"
+
+namespace afp {
+namespace {
+
+constexpr int kB = 256;         // panel width
+constexpr int kS = 9;           // digits per number
+constexpr int kAcc = 8;         // accumulators of an output tile
+constexpr int kKC = 32;         // inner indices per pipeline stage
+constexpr int kNK = kB / kKC;   // stages of one product
+constexpr int kTM = 128, kTN = 64;  // output tile of a block: kAcc accumulators of kTN columns fill tensor memory
+constexpr int kSub = 16;        // pivots per step of the panel's own inverse
+
+// ------------------------------------------------------------- eligibility
+// flag |= 1 unless the matrix is symmetric to rounding with a positive
+// diagonal in [2^-400, 2^400] (the digits' scales stay normal numbers)
+__global__ void k_spd_check(int64_t n, const double* __restrict__ M, int* __restrict__ flag) {
+  __shared__ double tr[32][33];
+  const int64_t i0 = (int64_t)blockIdx.y * 32, j0 = (int64_t)blockIdx.x * 32;
+  if (j0 > i0) return;
+  for (int r = threadIdx.y; r < 32; r += 8) {
+    const int64_t i = j0 + r, j = i0 + threadIdx.x;
+    tr[r][threadIdx.x] = (i < n && j < n) ? M[i * n + j] : 0.0;
+  }
+  __syncthreads();
+  bool bad = false;
+  for (int r = threadIdx.y; r < 32; r += 8) {
+    const int64_t i = i0 + r, j = j0 + threadIdx.x;
+    if (i >= n || j >= n || j > i) continue;
+    const double a = M[i * n + j];
+    const double di = M[i * n + i], dj = M[j * n + j];
+    if (!(fabs(a - tr[threadIdx.x][r]) <= 1e-12 * sqrt(di * dj))) bad = true;
+    if (i == j && !(a >= 0x1p-400 && a <= 0x1p400)) bad = true;
+  }
+  if (__any_sync(0xffffffffu, bad) && threadIdx.x == 0) atomicOr(flag, 1);
+}
+
+// ----------------------------------------------------- the panel's inverse
+// P (kB x kB, full) <- the pivot block from the lower triangle, the identity
+// beyond pb
+__global__ void k_spd_pivot_block(int64_t n, int64_t k0, int pb, const double* __restrict__ M,
+                                  double* __restrict__ P) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = t / kB, c = t % kB;
+  double v = r == c ? 1.0 : 0.0;
+  if (r < pb && c < pb) v = r >= c ? M[(k0 + r) * n + k0 + c] : M[(k0 + c) * n + k0 + r];
+  P[t] = v;
+}
+
+// One step of the block Gauss-Jordan inverse of P: kSub pivots, from `in` to
+// `out`.  A block owns 32 rows x kSub columns and inverts the kSub x kSub
+// pivot itself: 2 us of FP64 latency in every block instead of one more
+// launch in the chain.
+__global__ void __launch_bounds__(128) k_spd_sweep(int kk, const double* __restrict__ in, double* __restrict__ out,
+                                                   int* __restrict__ flag) {
+  __shared__ double D[kSub][kSub + 1], R[kSub][kSub + 1], T[kSub][kSub + 1], Cc[32][kSub + 1];
+  const int tid = threadIdx.x;
+  const int jb = blockIdx.x, ib = blockIdx.y;
+  const int p0 = kk * kSub, c0 = jb * kSub, r0 = ib * 32;
+  for (int t = tid; t < kSub * kSub; t += 128) {
+    const int r = t / kSub, c = t % kSub;
+    D[r][c] = in[(p0 + r) * kB + p0 + c];
+    R[r][c] = in[(p0 + r) * kB + c0 + c];
+  }
+  for (int t = tid; t < 32 * kSub; t += 128) Cc[t / kSub][t % kSub] = in[(r0 + t / kSub) * kB + p0 + t % kSub];
+  __syncthreads();
+  // in-place inverse: thread t holds entries (r, c) and (r + 8, c)
+  const int r = tid / kSub, c = tid % kSub;
+  for (int q = 0; q < kSub; ++q) {
+    const double p = D[q][q];
+    const double ip = 1.0 / p;
+    if (!(p > 0.0) && tid == 0) atomicOr(flag, 1);
+    const double rowv = (c == q ? 1.0 : D[q][c]) * ip;
+    const double f0 = D[r][q], f1 = D[r + 8][q];
+    const double a0 = c == q ? 0.0 : D[r][c], a1 = c == q ? 0.0 : D[r + 8][c];
+    __syncthreads();
+    D[r][c] = r == q ? rowv : a0 - f0 * rowv;
+    D[r + 8][c] = r + 8 == q ? rowv : a1 - f1 * rowv;
+    __syncthreads();
+  }
+  // T = Q R_j, or Q itself in the pivot's own columns
+  for (int h = 0; h < 2; ++h) {
+    double s = 0;
+    for (int q = 0; q < kSub; ++q) s += D[r + 8 * h][q] * R[q][c];
+    T[r + 8 * h][c] = jb == kk ? D[r + 8 * h][c] : s;
+  }
+  __syncthreads();
+  for (int h = 0; h < 4; ++h) {
+    const int rr = r + 8 * h, row = r0 + rr;
+    double v;
+    if (row >= p0 && row < p0 + kSub) {
+      v = T[row - p0][c];
+    } else {
+      v = jb == kk ? 0.0 : in[row * kB + c0 + c];
+      for (int q = 0; q < kSub; ++q) v -= Cc[rr][q] * T[q][c];
+    }
+    out[row * kB + c0 + c] = v;
+  }
+}
+
+// --------------------------------------------------------------- the digits
+// Digit arrays: [stage kc][digit][8-row group][octet of kKC][8 rows][8
+// inner], BF16: any run of row groups of one stage and digit is contiguous in
+// the core-matrix order the tensor cores read (8 rows x 16 bytes, next octet
+// 128 bytes on, next row group 512 bytes on), so a tile is one bulk copy.
+__device__ __forceinline__ size_t digit_offset(int64_t groups, int kc, int s, int64_t row, int octet) {
+  return ((((size_t)kc * kS + s) * groups + row / 8) * (kKC / 8) + octet) * 64 + (row % 8) * 8;
+}
+
+// One warp cuts one row: lane l holds inner indices 8 l .. 8 l + 7.
+__device__ __forceinline__ void cut_row(const double (&v)[8], int lane, int64_t groups, int64_t row,
+                                        __nv_bfloat16* __restrict__ dig, double* __restrict__ scale) {
+  double mx = 0.0;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) mx = fmax(mx, fabs(v[e]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  // 2^ex > mx, from the exponent bits; a row below 2^-900 counts as zeros
+  const int ex = min(900, max(-900, (int)((__double2hiint(mx) >> 20) & 0x7ff) - 1022));
+  const double up = __hiloint2double((1023 + 7 * kS - 1 - ex) << 20, 0);
+  long long w[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = __double2ll_rn(v[e] * up);
+#pragma unroll
+  for (int s = kS - 1; s >= 0; --s) {
+    __align__(16) __nv_bfloat16 d[8];
+    const float unit = __int_as_float((127 - 7 * s) << 23);  // 2^-7s
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      long long g = w[e];
+      if (s > 0) {
+        g = ((w[e] + 64) & 127) - 64;
+        w[e] = (w[e] - g) >> 7;
+      }
+      d[e] = __float2bfloat16_rn((float)(int)g * unit);
+    }
+    *reinterpret_cast<uint4*>(dig + digit_offset(groups, lane / 4, s, row, lane % 4)) =
+        *reinterpret_cast<const uint4*>(d);
+  }
+  if (lane == 0) *scale = __hiloint2double((1023 + ex) << 20, 0);
+}
+
+// C of the panel [k0, k0 + pb) cut into digits; a block takes one 8-row group.
+// Rows below the panel read their own columns, rows above it the panel's rows
+// transposed, the panel's rows and the padding are zeros.
+__global__ void __launch_bounds__(256) k_spd_cut_panel(int64_t n, int64_t k0, int pb, const double* __restrict__ M,
+                                                       int64_t groups, __nv_bfloat16* __restrict__ dig,
+                                                       double* __restrict__ scale) {
+  __shared__ double tile[8][kB + 1];
+  const int64_t i0 = (int64_t)blockIdx.x * 8;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t row = i0 + w;
+  double v[8];
+  if (i0 < k0) {  // k0 is a multiple of 8: the whole group is above the panel
+    const int j = threadIdx.x;
+    if (j < pb) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) tile[e][j] = M[(k0 + j) * n + i0 + e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) tile[e][j] = 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = tile[w][8 * lane + e];
+  } else {
+    const bool on = row >= k0 + pb && row < n;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int j = 8 * lane + e;
+      v[e] = (on && j < pb) ? M[row * n + k0 + j] : 0.0;
+    }
+  }
+  cut_row(v, lane, groups, row, dig, scale + row);
+}
+
+// A dense `rows` x kB array cut into digits; with M, its rows also go back
+// into the panel of the lower triangle: -Z below, +Z^T into the panel's rows
+// for the rows above.
+__global__ void __launch_bounds__(256) k_spd_cut_dense(int64_t n, int64_t k0, int pb, const double* __restrict__ Z,
+                                                       double* __restrict__ M, int64_t groups,
+                                                       __nv_bfloat16* __restrict__ dig, double* __restrict__ scale) {
+  __shared__ double tile[8][kB + 1];
+  const int64_t i0 = (int64_t)blockIdx.x * 8;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t row = i0 + w;
+  double v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = Z[row * kB + 8 * lane + e];
+  cut_row(v, lane, groups, row, dig, scale + row);
+  if (M == nullptr) return;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) tile[w][8 * lane + e] = v[e];
+  __syncthreads();
+  const int j = threadIdx.x;
+  if (i0 < k0) {
+    if (j < pb)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) M[(k0 + j) * n + i0 + e] = tile[e][j];
+  } else if (j < pb) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (i0 + e >= k0 + pb && i0 + e < n) M[(i0 + e) * n + k0 + j] = -tile[e][j];
+  }
+}
+
+// the pivot block back into the lower triangle
+__global__ void k_spd_put_pivot(int64_t n, int64_t k0, int pb, const double* __restrict__ Q, double* __restrict__ M) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = t / kB, c = t % kB;
+  if (r < pb && c <= r) M[(k0 + r) * n + k0 + c] = Q[t];
+}
+
+// upper triangle <- lower triangle
+__global__ void k_spd_mirror(int64_t n, double* __restrict__ M) {
+  __shared__ double tr[32][33];
+  const int64_t i0 = (int64_t)blockIdx.y * 32, j0 = (int64_t)blockIdx.x * 32;
+  if (j0 > i0) return;
+  for (int r = threadIdx.y; r < 32; r += 8) {
+    const int64_t i = i0 + r, j = j0 + threadIdx.x;
+    tr[r][threadIdx.x] = (i < n && j < n) ? M[i * n + j] : 0.0;
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32; r += 8) {
+    const int64_t i = j0 + r, j = i0 + threadIdx.x;  // (i, j) above the diagonal
+    if (i < n && j < n && j > i) M[i * n + j] = tr[threadIdx.x][r];
+  }
+}
+
+// -------------------------------------------------------- the digit product
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void bar_init(uint64_t* b, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t* b, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+// false when the phase does not complete within the bound (seconds at most)
+__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t phase) {
+  for (int it = 0; it < (1 << 22); ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(phase)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* b) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(smem_u32(b))
+               : "memory");
+}
+// Shared-memory matrix descriptor: no swizzle, K-major, next octet 128 bytes
+// on (leading offset), next 8-row group 512 bytes on (stride offset).
+__device__ __forceinline__ uint64_t mat_desc(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
+         ((uint64_t)1 << 46);
+}
+// FP32 accumulators, both operands BF16 and K-major, kTM x kTN
+constexpr uint32_t kInstr = (1u << 4) | (1u << 7) | (1u << 10) | ((kTN / 8) << 17) | ((kTM / 16) << 24);
+
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+      "l"(a), "l"(b), "r"(kInstr), "r"((uint32_t)accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* b) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(addr));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+constexpr uint32_t kABytes = kTM * kKC * 2, kBBytes = kTN * kKC * 2;  // one digit's tile of a stage
+constexpr uint32_t kStageBytes = kS * (kABytes + kBBytes);
+constexpr int kStages = 2;
+constexpr size_t kProdSmem = kStages * kStageBytes + 1024;
+constexpr int kProdThreads = 192;
+
+// The exact sums over digit pairs of a kTM x kTN tile of A B^T (A, B digit
+// arrays of kB inner indices).  UPDATE: subtracted from (rows >= k0) or added
+// to the tiles of the lower triangle of `out` (row stride ld) that the panel
+// [k0, k0 + kB) does not own; otherwise stored to `out`.  One tile per block:
+// warp 4 streams the digits, warp 5 issues the products, warps 0-3 put the
+// sums together.  A tile is 720 products of 128 x 64 x 16 (23K clocks) and
+// 8,192 entries of five FP64-rate operations (20K clocks), which bounds it.
+template <bool UPDATE>
+__global__ void __launch_bounds__(kProdThreads) k_spd_product(const __nv_bfloat16* __restrict__ A, int64_t groups_a,
+                                                              const double* __restrict__ sa,
+                                                              const __nv_bfloat16* __restrict__ B, int64_t groups_b,
+                                                              const double* __restrict__ sb, int64_t rows,
+                                                              int64_t cols, int64_t k0, double* __restrict__ out,
+                                                              int64_t ld, int* __restrict__ error) {
+  const int64_t i0 = (int64_t)blockIdx.x * kTM, j0 = (int64_t)blockIdx.y * kTN;
+  if (UPDATE) {
+    if (j0 > i0 + kTM - 1) return;
+    if ((i0 >= k0 && i0 < k0 + kB) || (j0 >= k0 && j0 < k0 + kB)) return;
+  }
+  extern __shared__ unsigned char prod_raw[];
+  __shared__ uint64_t full[kStages], empty[kStages], done;
+  __shared__ uint32_t tmem_slot;
+  const uint32_t base = (smem_u32(prod_raw) + 1023u) & ~1023u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      bar_init(&full[s], 1);
+      bar_init(&empty[s], 1);
+    }
+    bar_init(&done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  if (warp == 4 && lane == 0) {
+    int issued = 0;
+    for (int kc = 0; kc < kNK; ++kc) {
+      const int st = kc % kStages;
+      if (kc >= kStages && !bar_wait(&empty[st], ((kc / kStages) - 1) & 1)) {
+        atomicOr(error, 2);
+        break;
+      }
+      bar_expect(&full[st], kStageBytes);
+      const uint32_t dst = base + st * kStageBytes;
+      for (int s = 0; s < kS; ++s) {
+        bulk_load(dst + s * kABytes, A + (((size_t)kc * kS + s) * groups_a + i0 / 8) * (kKC * 8), kABytes, &full[st]);
+        bulk_load(dst + kS * kABytes + s * kBBytes, B + (((size_t)kc * kS + s) * groups_b + j0 / 8) * (kKC * 8),
+                  kBBytes, &full[st]);
+      }
+      ++issued;
+    }
+    // copies in flight end before the block does
+    for (int kc = issued > kStages ? issued - kStages : 0; kc < issued; ++kc)
+      if (!bar_wait(&full[kc % kStages], (kc / kStages) & 1)) atomicOr(error, 2);
+  } else if (warp == 5 && lane == 0) {
+    for (int kc = 0; kc < kNK; ++kc) {
+      const int st = kc % kStages;
+      if (!bar_wait(&full[st], (kc / kStages) & 1)) {
+        atomicOr(error, 2);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t ab = base + st * kStageBytes, bb = ab + kS * kABytes;
+#pragma unroll 1
+      for (int i = 0; i < kS; ++i)
+        for (int j = 0; i + j < kS; ++j)
+#pragma unroll
+          for (int q = 0; q < kKC / 16; ++q)
+            mma(tmem + min(i + j, kAcc - 1) * kTN, mat_desc(ab + i * kABytes + q * 256), mat_desc(bb + j * kBBytes + q * 256),
+                kc > 0 || i > 0 || q > 0);
+      mma_commit(&empty[st]);
+    }
+    mma_commit(&done);
+  } else if (warp < 4) {
+    const bool ok = bar_wait(&done, 0);
+    if (!ok) {
+      if (lane == 0) atomicOr(error, 2);
+    } else {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // the stages are free: warp w keeps its 32 rows of the tile there
+      double* tile = reinterpret_cast<double*>(prod_raw + (base - smem_u32(prod_raw))) + warp * 32 * (kTN + 1);
+      const int64_t row = i0 + warp * 32 + lane;
+      const double rs = sa[row] * 0x1p-68;  // 2^-12 of the digits' scale, 2^-56 of the units of `lo`
+      for (int c = 0; c < kTN; c += 8) {
+        float v[kAcc][8];
+#pragma unroll
+        for (int s = 0; s < kAcc; ++s) tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + s * kTN + c, v[s]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          long long hi = 0, lo = 0;
+#pragma unroll
+          for (int s = 0; s < 4; ++s) hi = hi * 128 + __float2int_rn(v[s][e] * __int_as_float((127 + 7 * s) << 23));
+#pragma unroll
+          for (int s = 4; s < 7; ++s) lo = lo * 128 + __float2int_rn(v[s][e] * __int_as_float((127 + 7 * s) << 23));
+          lo = lo * 16384 + __float2int_rn(v[7][e] * 0x1p56f);
+          tile[lane * (kTN + 1) + c + e] = fma((double)hi, 0x1p35, (double)lo) * rs;
+        }
+      }
+      __syncwarp();
+      const double c0 = sb[j0 + lane], c1 = sb[j0 + 32 + lane];
+      const int64_t ja = j0 + lane, jb = j0 + 32 + lane;
+      for (int r = 0; r < 32; ++r) {
+        const int64_t i = i0 + warp * 32 + r;
+        if (i >= rows) break;
+        double* o = out + i * ld;
+        const double ta = tile[r * (kTN + 1) + lane] * c0, tb = tile[r * (kTN + 1) + 32 + lane] * c1;
+        if (UPDATE) {
+          const double sg = i0 >= k0 ? -1.0 : 1.0;
+          if (ja <= i) o[ja] += sg * ta;
+          if (jb <= i) o[jb] += sg * tb;
+        } else {
+          if (ja < cols) o[ja] = ta;
+          if (jb < cols) o[jb] = tb;
+        }
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  __syncthreads();
+  if (warp == 5) {
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+}
+
+}  // namespace
+
+bool spd_inverse(const afp_context* ctx, int64_t n, double* M) {
+  DevBuf<int> flag(ctx, 2);
+  flag.zero();
+  const dim3 g32((unsigned)((n + 31) / 32), (unsigned)((n + 31) / 32)), b32(32, 8);
+  k_spd_check<<<g32, b32, 0, ctx->stream>>>(n, M, flag.get());
+  check_launch(ctx, "spd check");
+  int hf[2] = {0, 0};
+  flag.download(hf, 2);
+  sync(ctx);
+  if (hf[0]) return false;
+  const int64_t np = (n + kTM - 1) / kTM * kTM, groups = np / 8;
+  const bool one = n <= kB;
+  DevBuf<double> P0(ctx, kB * kB), P1(ctx, kB * kB), Z, sc, sz, sq;
+  DevBuf<__nv_bfloat16> dc, dz, dq;
+  if (!one) {
+    Z.alloc(ctx, np * kB);
+    sc.alloc(ctx, np);
+    sz.alloc(ctx, np);
+    sq.alloc(ctx, kB);
+    dc.alloc(ctx, (size_t)np * kB * kS);
+    dz.alloc(ctx, (size_t)np * kB * kS);
+    dq.alloc(ctx, (size_t)kB * kB * kS);
+    AFP_CUDA(cudaFuncSetAttribute(k_spd_product<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdSmem));
+    AFP_CUDA(cudaFuncSetAttribute(k_spd_product<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdSmem));
+  }
+  for (int64_t k0 = 0; k0 < n; k0 += kB) {
+    const int pb = (int)std::min<int64_t>(kB, n - k0);
+    k_spd_pivot_block<<<kB * kB / 256, 256, 0, ctx->stream>>>(n, k0, pb, M, P0.get());
+    check_launch(ctx, "spd pivot block");
+    double *in = P0.get(), *out = P1.get();
+    for (int kk = 0; kk * kSub < pb; ++kk) {
+      k_spd_sweep<<<dim3(kB / kSub, kB / 32), 128, 0, ctx->stream>>>(kk, in, out, flag.get());
+      check_launch(ctx, "spd panel sweep");
+      std::swap(in, out);
+    }
+    if (!one) {
+      k_spd_cut_dense<<<kB / 8, 256, 0, ctx->stream>>>(n, k0, pb, in, nullptr, kB / 8, dq.get(), sq.get());
+      check_launch(ctx, "spd cut pivot inverse");
+      k_spd_cut_panel<<<(unsigned)groups, 256, 0, ctx->stream>>>(n, k0, pb, M, groups, dc.get(), sc.get());
+      check_launch(ctx, "spd cut panel");
+      k_spd_product<false><<<dim3((unsigned)(np / kTM), kB / kTN), kProdThreads, kProdSmem, ctx->stream>>>(
+          dc.get(), groups, sc.get(), dq.get(), kB / 8, sq.get(), np, kB, k0, Z.get(), kB, flag.get() + 1);
+      check_launch(ctx, "spd panel product");
+      k_spd_cut_dense<<<(unsigned)groups, 256, 0, ctx->stream>>>(n, k0, pb, Z.get(), M, groups, dz.get(), sz.get());
+      check_launch(ctx, "spd cut panel product");
+      k_spd_product<true><<<dim3((unsigned)(np / kTM), (unsigned)(np / kTN)), kProdThreads, kProdSmem, ctx->stream>>>(
+          dz.get(), groups, sz.get(), dc.get(), groups, sc.get(), n, n, k0, M, n, flag.get() + 1);
+      check_launch(ctx, "spd update");
+    }
+    k_spd_put_pivot<<<kB * kB / 256, 256, 0, ctx->stream>>>(n, k0, pb, in, M);
+    check_launch(ctx, "spd put pivot");
+  }
+  k_spd_mirror<<<g32, b32, 0, ctx->stream>>>(n, M);
+  check_launch(ctx, "spd mirror");
+  flag.download(hf, 2);
+  sync(ctx);
+  AFP_REQUIRE(hf[1] == 0, AFP_ERR_TIMEOUT, "dense inverse: a bounded wait ran out");
+  return hf[0] == 0;
+}
+
+}  // namespace afp
