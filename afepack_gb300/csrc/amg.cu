@@ -518,7 +518,7 @@ void setup(afp_amg* h, afp_matrix* A, bool lazy) {
       DevBuf<int> drp(ctx, ns + 1), dci(ctx, sci.size());
       drp.upload(srp.data(), ns + 1);
       dci.upload(sci.data(), sci.size());
-      const int64_t nnz_s = galerkin_nnz(ctx, ns, P.m, drp.get(), dci.get(), arp, aci, dT.rp.get(), dT.ci.get());
+      const int64_t nnz_s = galerkin_nnz(ctx, ns, P.n, P.m, drp.get(), dci.get(), arp, aci, dT.rp.get(), dT.ci.get());
       try_dense = (double)nnz_s / ((double)ns * (double)P.m) >= 0.5 * kDenseTailDensity;
     }
     if (try_dense) {

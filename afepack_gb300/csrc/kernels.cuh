@@ -18,18 +18,19 @@ void galerkin_product(const afp_context* ctx, int64_t n_c, int64_t n_f, const in
                       DevBuf<double>& out_vals);
 
 // Stored entries of the n_rows rows of P A P^T that the given rows of P
-// produce (its symbolic count alone; n_c = columns of the product), to
-// decide how to form a level before forming it.
-int64_t galerkin_nnz(const afp_context* ctx, int64_t n_rows, int64_t n_c, const int* p_rowptr, const int* p_cols,
+// produce (its symbolic count alone; n_f = fine rows, n_c = columns of the
+// product), to decide how to form a level before forming it.
+int64_t galerkin_nnz(const afp_context* ctx, int64_t n_rows, int64_t n_f, int64_t n_c, const int* p_rowptr, const int* p_cols,
                      const int* a_rowptr, const int* a_cols, const int* pt_rowptr, const int* pt_cols);
 
 // Reserves afp_matrix_vmult_noalloc's static staging array on `device` (the
 // current device); called once per context creation (noalloc.cu).
 void noalloc_reserve(int device);
 
-// The same product through a dense intermediate (n_f x n_c and n_c x n_c
-// FP64 arrays), for the dense-tail level only: deterministic, but not
+// The same product as A P^T, then P times it (a sparse intermediate and an
+// n_c x n_c FP64 array), for the dense-tail level only: deterministic, but not
 // getPMPt's accumulation order; exact zeros other than the diagonal dropped.
+// n_c is at most 16384.
 void galerkin_product_dense(const afp_context* ctx, int64_t n_c, int64_t n_f, const int* p_rowptr,
                             const int* p_cols, const double* p_vals, const int* a_rowptr, const int* a_cols,
                             const double* a_vals, const int* pt_rowptr, const int* pt_cols, const double* pt_vals,
