@@ -7,10 +7,9 @@
 // * Pass 1 (lines 39-68) makes row i a C point iff no earlier C point j < i
 //   holds i as a strong neighbour in its own row (|a_ji| >= beta_j).  That
 //   is the lexicographically first independent set of the graph j -> i
-//   (j < i, strong in row j); it is computed in rounds: a row becomes F as
-//   soon as one such j is C, and C once all of them are F.  The lowest
-//   undecided row decides in every round, so the rounds end; on mesh
-//   matrices they number a few times the mesh's grid width.
+//   (j < i, strong in row j).  It spreads as a wave: a row without such j is
+//   C; a row that became C makes every row it holds F; a row that became F
+//   counts down the rows it holds, and one whose count reaches zero is C.
 // * Pass 2 (lines 74-126) promotes an F point i to C when some strong F
 //   neighbour k > i has no C point in its row that is also a strong C
 //   neighbour of i.  The C points i sees are the pass-1 C points and the
@@ -18,12 +17,22 @@
 //   that set, which can only turn i's answer from "promote" to "keep", so a
 //   row that would not be promoted against the pass-1 C points alone is
 //   final, and a remaining candidate is decided once its candidate strong
-//   neighbours below it are decided.  Again rounds, over the (few) candidates.
+//   neighbours below it are decided.  Again a wave, over the (few) candidates.
+//
+//   A wave is up to a few hundred steps of little work each (192 on the
+//   finest level of a 64^3 mesh, 512 of a 256^2 one), so each pass is one
+//   kernel of one thread-block cluster: a step costs a cluster barrier
+//   (hardware, well under a microsecond) and a few dependent loads, instead of a
+//   launch that looks through all rows.  Only rows decided in the step
+//   before are touched.  64^3 hierarchy, all levels: pass 1 5.2 ms against
+//   17 ms of launches, pass 2 15 against 53 ms.
 // * P and P^T (lines 127-216): every fine row's weights are accumulated by
-//   one thread in the reference's order (the same additions into the same
-//   entries), so the values are the reference's.
+//   one thread (a warp where rows are long) in the reference's order (the
+//   same additions into the same entries), so the values are the reference's.
 //
 // Compiled with -fmad=false: every product and quotient rounds as on the host.
+#include <cooperative_groups.h>
+
 #include <cstdint>
 
 #include "common.cuh"
@@ -34,6 +43,7 @@ namespace afp {
 namespace {
 
 constexpr int kRoundsPerCheck = 16;
+constexpr int kWaveThreads = 1024;  // threads per block of a wave's cluster
 
 // the reference's strength test: "if (fabs(a) < beta) continue" skips weak entries
 __device__ __forceinline__ bool strong(double a, double beta) { return !(fabs(a) < beta); }
@@ -61,7 +71,7 @@ __device__ __forceinline__ int find_sorted(const int* __restrict__ ci, int b, in
   return (b < end && ci[b] == c) ? b : -1;
 }
 
-__device__ __forceinline__ int8_t vload(const int8_t* p) { return *(const volatile int8_t*)p; }
+__device__ __forceinline__ int vload(const int* p) { return *(const volatile int*)p; }
 
 // beta_i = alpha * max_j |a_ij| over the off-diagonal entries; one warp per row
 __global__ void k_cf_beta(int m, const int* __restrict__ rp, const double* __restrict__ va, double alpha,
@@ -81,52 +91,85 @@ __global__ void k_cf_beta(int m, const int* __restrict__ rp, const double* __res
   if (lane == 0) beta[i] = b * alpha;
 }
 
-// in_edge[e] for an off-diagonal entry e = (i, j), j < i: row j holds i as a
-// strong neighbour, so a C point j makes i an F point in pass 1
-__global__ void k_cf_in_edges(int m, const int* __restrict__ rp, const int* __restrict__ ci,
-                              const double* __restrict__ va, const double* __restrict__ beta,
-                              uint8_t* __restrict__ in_edge) {
-  const int i = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+// cnt[i] = number of rows j < i that hold i as a strong neighbour; one warp per row j
+__global__ void k_cf_count_in(int m, const int* __restrict__ rp, const int* __restrict__ ci,
+                              const double* __restrict__ va, const double* __restrict__ beta, int* __restrict__ cnt) {
+  const int j = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
-  if (i >= m) return;
-  for (int e = rp[i] + 1 + lane; e < rp[i + 1]; e += 32) {
-    const int j = ci[e];
-    uint8_t f = 0;
-    if (j < i) {
-      const int p = find_offd(rp, ci, j, i);
-      f = (p >= 0 && strong(va[p], beta[j])) ? 1 : 0;
-    }
-    in_edge[e] = f;
-  }
+  if (j >= m) return;
+  const double bj = beta[j];
+  for (int e = rp[j] + 1 + lane; e < rp[j + 1]; e += 32)
+    if (ci[e] > j && strong(va[e], bj)) atomicAdd(cnt + ci[e], 1);
 }
 
-// one round of pass 1; st: 0 undecided, -1 C, 1 F.  Rows read their lower
-// neighbours' states while those may be written in the same round: a state
-// only ever leaves 0 once, so a stale read delays a decision but never changes it.
-__global__ void k_cf_pass1(int m, const int* __restrict__ rp, const int* __restrict__ ci,
-                           const uint8_t* __restrict__ in_edge, int8_t* st, int* undecided) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool pending = false;
-  if (i < m && vload(st + i) == 0) {
-    int8_t out = -1;
-    for (int e = rp[i] + 1; e < rp[i + 1]; ++e) {
-      const int j = ci[e];
-      if (j >= i) break;
-      if (!in_edge[e]) continue;
-      const int8_t s = vload(st + j);
-      if (s == -1) {
-        out = 1;
-        pending = false;
-        break;
+// Appends i of the lanes with `push` to list[*count ...]; the whole warp calls it.
+__device__ __forceinline__ void push_rows(bool push, int i, int* list, int* count) {
+  const unsigned b = __ballot_sync(0xffffffffu, push);
+  if (b == 0) return;
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (lane == __ffs(b) - 1) base = atomicAdd(count, __popc(b));
+  base = __shfl_sync(0xffffffffu, base, __ffs(b) - 1);
+  if (push) list[base + __popc(b & ((1u << lane) - 1u))] = i;
+}
+
+// Pass 1 as a wave.  st: 0 undecided, -1 C, 1 F; cnt from k_cf_count_in;
+// list: two arrays of m rows (this step's and the next one's); counts[3]
+// zeroed.  A row is listed once, when it is decided: F by the compare-and-swap
+// that changed it, C by the decrement that reached zero (a row held by a C
+// point never gets there, since that point does not count down).  The lists
+// and counts are read past the L1 cache, and the cluster barrier orders a
+// step's writes before the next step's reads.  G lanes take a row: a step is
+// a chain of dependent loads, so short rows go four to a warp.
+template <int G>
+__global__ void __launch_bounds__(kWaveThreads) k_cf_pass1_wave(int m, const int* __restrict__ rp,
+                                                                const int* __restrict__ ci,
+                                                                const double* __restrict__ va,
+                                                                const double* __restrict__ beta, int* st, int* cnt,
+                                                                int* list, int* counts, int* steps) {
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  for (int i0 = 0; i0 < m; i0 += nt) {
+    const int i = i0 + tid;
+    const bool c = i < m && cnt[i] == 0;
+    if (c) st[i] = -1;
+    push_rows(c, i, list, counts);
+  }
+  __threadfence();
+  cluster.sync();
+  int step = 0;
+  for (;; ++step) {
+    const int n = __ldcg(counts + step % 3);
+    if (n == 0) break;
+    const int* cur = list + (size_t)(step & 1) * m;
+    int* next = list + (size_t)((step + 1) & 1) * m;
+    int* ncount = counts + (step + 1) % 3;
+    if (tid == 0) counts[(step + 2) % 3] = 0;
+    for (int w = warp * (32 / G); w < n; w += nw * (32 / G)) {
+      const int at = w + lane / G;
+      const int j = at < n ? __ldcg(cur + at) : -1;
+      const bool is_c = j >= 0 && __ldcg(st + j) == -1;
+      const double bj = j >= 0 ? beta[j] : 0.0;
+      const int e1 = j >= 0 ? rp[j + 1] : 0;
+      for (int e = j >= 0 ? rp[j] + 1 + lane % G : 0; __any_sync(0xffffffffu, e < e1); e += G) {
+        const int i = e < e1 ? ci[e] : -1;
+        bool push = false;
+        if (i > j && strong(va[e], bj)) {
+          if (is_c) {
+            push = __ldcg(st + i) == 0 && atomicCAS(st + i, 0, 1) == 0;
+          } else if (atomicSub(cnt + i, 1) == 1) {
+            st[i] = -1;
+            push = true;
+          }
+        }
+        push_rows(push, i, next, ncount);
       }
-      if (s == 0) pending = true;
     }
-    if (!pending) st[i] = out;
+    __threadfence();
+    cluster.sync();
   }
-  if (undecided != nullptr) {
-    const unsigned b = __ballot_sync(0xffffffffu, pending);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(undecided, __popc(b));
-  }
+  if (tid == 0) *steps = step;
 }
 
 // Pass 2's test for an F point i (one warp): is there a strong neighbour
@@ -134,51 +177,211 @@ __global__ void k_cf_pass1(int m, const int* __restrict__ rp, const int* __restr
 // neighbour of i?  C points below i are the pass-1 ones and the promoted
 // (s2 == 2); above i only the pass-1 ones count (the reference has not
 // reached them yet).  With s2 == nullptr no promotion is counted.
+//
+// i's strong C neighbours go into a hash set in shared memory (`table`,
+// kSet slots of the warp's own) and four rows k at a time are looked through,
+// 8 lanes each: a binary search of row i in global memory for every entry of
+// every row k was 8 dependent loads instead of one shared one.  Rows of more
+// strong C neighbours than the set holds are searched that way.
+constexpr int kSet = 512;
+
+__device__ __forceinline__ unsigned set_slot(int key) { return ((unsigned)key * 2654435761u) >> 23; }
+
+__device__ __forceinline__ bool strong_c(int j, double a, double bi, int i, const int* __restrict__ st1,
+                                         const int* s2) {
+  return strong(a, bi) && (st1[j] == -1 || (s2 != nullptr && j < i && __ldcg(s2 + j) == 2));
+}
+
+// A block of several warps (WPR) shares the set and splits the rows k, 8 of
+// i's entries to a warp at a time; each warp answers for its own.
+template <int WPR>
 __device__ bool cf_promote(int i, const int* __restrict__ rp, const int* __restrict__ ci,
                            const double* __restrict__ va, const double* __restrict__ beta,
-                           const int8_t* __restrict__ st1, const int8_t* s2, int lane) {
+                           const int* __restrict__ st1, const int* s2, int* table, int lane) {
   const double bi = beta[i];
-  for (int e = rp[i] + 1; e < rp[i + 1]; ++e) {
-    const int k = ci[e];
-    if (k < i || st1[k] == -1 || !strong(va[e], bi)) continue;
-    bool common = false;
-    for (int b0 = rp[k] + 1; b0 < rp[k + 1] && !common; b0 += 32) {
-      bool hit = false;
-      const int j1 = b0 + lane;
-      if (j1 < rp[k + 1]) {
-        const int k1 = ci[j1];
-        bool c = st1[k1] == -1;
-        if (!c && s2 != nullptr && k1 < i) c = vload(s2 + k1) == 2;
-        if (c) {
-          const int p = find_offd(rp, ci, i, k1);
-          hit = p >= 0 && strong(va[p], bi);
+  const int b = rp[i] + 1, e = rp[i + 1];
+  const int w = WPR > 1 ? threadIdx.x >> 5 : 0;
+  int n = 0;
+  for (int q = b + lane; q < e; q += 32) n += strong_c(ci[q], va[q], bi, i, st1, s2);
+  n = __reduce_add_sync(0xffffffffu, n);
+  const bool set = n <= kSet * 3 / 4;
+  if (set) {
+    if (WPR > 1) __syncthreads();
+    for (int t = w * 32 + lane; t < kSet; t += WPR * 32) table[t] = -1;
+    if (WPR > 1) __syncthreads();
+    else __syncwarp();
+    for (int q = b + w * 32 + lane; q < e; q += WPR * 32) {
+      const int j = ci[q];
+      if (!strong_c(j, va[q], bi, i, st1, s2)) continue;
+      unsigned h = set_slot(j);
+      while (atomicCAS(table + h, -1, j) != -1) h = (h + 1) & (kSet - 1);
+    }
+    if (WPR > 1) __syncthreads();
+    else __syncwarp();
+  }
+  const int sub = lane >> 3, sl = lane & 7;
+  constexpr int CH = WPR > 1 ? 8 : 32;  // i's entries to a warp at a time
+  constexpr int U = 4;                  // entries of a row k in flight per lane
+  for (int q0 = b + w * CH; q0 < e; q0 += WPR * CH) {
+    const int q = q0 + lane;
+    const int k = lane < CH && q < e ? ci[q] : -1;
+    const bool sel = k > i && st1[k] != -1 && strong(va[q], bi);
+    const int kb = sel ? rp[k] + 1 : 0, ke = sel ? rp[k + 1] : 0;
+    for (unsigned todo = __ballot_sync(0xffffffffu, sel); todo != 0;) {
+      unsigned t = todo;
+      for (int s = 0; s < sub; ++s) t &= t - 1;
+      const int src = t ? __ffs(t) - 1 : 0;
+      int at = __shfl_sync(0xffffffffu, kb, src) + sl;
+      const int end = __shfl_sync(0xffffffffu, ke, src);
+      bool open = t != 0;  // the same for a row's 8 lanes
+      bool lacks = false;
+      while (__any_sync(0xffffffffu, open)) {
+        bool hit = false;
+        int k1[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) k1[u] = open && at + 8 * u < end ? ci[at + 8 * u] : -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (k1[u] < 0) continue;
+          if (set) {
+            unsigned h = set_slot(k1[u]);
+            int v;
+            while ((v = table[h]) != -1 && v != k1[u]) h = (h + 1) & (kSet - 1);
+            hit |= v == k1[u];
+          } else {
+            const int p = find_offd(rp, ci, i, k1[u]);
+            hit |= p >= 0 && strong_c(k1[u], va[p], bi, i, st1, s2);
+          }
+        }
+        const unsigned any = (__ballot_sync(0xffffffffu, hit) >> (sub * 8)) & 0xffu;
+        at += 8 * U;
+        if (open && any) open = false;
+        if (open && at - sl >= end) {
+          lacks = true;
+          open = false;
         }
       }
-      common = __any_sync(0xffffffffu, hit);
+      if (__any_sync(0xffffffffu, lacks)) return true;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) todo &= todo - 1;
     }
-    if (!common) return true;
   }
   return false;
 }
 
 // s2 for every pass-1 F point: 1 (candidate) if it would be promoted against
 // the pass-1 C points alone, else 0 (final: promotions below can only add C points)
-__global__ void k_cf_pass2_candidates(int m, const int* __restrict__ rp, const int* __restrict__ ci,
-                                      const double* __restrict__ va, const double* __restrict__ beta,
-                                      const int8_t* __restrict__ st1, int8_t* __restrict__ s2) {
+__global__ void __launch_bounds__(256) k_cf_pass2_candidates(int m, const int* __restrict__ rp,
+                                                             const int* __restrict__ ci,
+                                                             const double* __restrict__ va,
+                                                             const double* __restrict__ beta,
+                                                             const int* __restrict__ st1, int* __restrict__ s2) {
+  __shared__ int tables[8][kSet];
   const int i = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= m) return;
   bool cand = false;
-  if (st1[i] == 1) cand = cf_promote(i, rp, ci, va, beta, st1, nullptr, lane);
+  if (st1[i] == 1) cand = cf_promote<1>(i, rp, ci, va, beta, st1, nullptr, tables[threadIdx.x >> 5], lane);
   if (lane == 0) s2[i] = cand ? 1 : 0;
 }
 
-// one round of pass 2 over the candidates (s2 == 1); s2 becomes 2 (promoted)
-// or 0 once every candidate strong neighbour below i is decided
-__global__ void k_cf_pass2_round(int m, const int* __restrict__ rp, const int* __restrict__ ci,
+// cnt[i] = candidate strong neighbours below candidate i
+__global__ void k_cf_pass2_count(int m, const int* __restrict__ rp, const int* __restrict__ ci,
                                  const double* __restrict__ va, const double* __restrict__ beta,
-                                 const int8_t* __restrict__ st1, int8_t* s2, int* undecided) {
+                                 const int* __restrict__ s2, int* __restrict__ cnt) {
+  const int i = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= m) return;
+  int n = 0;
+  if (s2[i] == 1) {
+    const double bi = beta[i];
+    for (int e = rp[i] + 1 + lane; e < rp[i + 1]; e += 32) n += ci[e] < i && s2[ci[e]] == 1 && strong(va[e], bi);
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0) cnt[i] = n;
+}
+
+// Pass 2 as a wave over the candidates; s2 becomes 2 (promoted) or 0 as they
+// are decided.  A decided row j tells the candidates above it that hold it as
+// a strong neighbour, found through its own row; where the pattern is not
+// symmetric some are not found and stay 1 (*left counts them) for
+// k_cf_pass2_round.  Lists and counts as in k_cf_pass1_wave.  A warp takes a
+// row, or a whole block while a step has no more than `block_rows` rows: on
+// levels of long rows (285 entries: 55 us a row to one warp, and 250 steps
+// one after the other) a row's own time is what a step waits for.
+__global__ void __launch_bounds__(kWaveThreads) k_cf_pass2_wave(int m, const int* __restrict__ rp,
+                                                                const int* __restrict__ ci,
+                                                                const double* __restrict__ va,
+                                                                const double* __restrict__ beta,
+                                                                const int* __restrict__ st1, int* s2, int* cnt,
+                                                                int* list, int* counts, int* steps, int* left, int block_rows) {
+  extern __shared__ int wave_sets[];
+  int(*tables)[kSet] = reinterpret_cast<int(*)[kSet]>(wave_sets);
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  int* table = tables[threadIdx.x >> 5];
+  for (int i0 = 0; i0 < m; i0 += nt) {
+    const int i = i0 + tid;
+    push_rows(i < m && s2[i] == 1 && cnt[i] == 0, i, list, counts);
+  }
+  __threadfence();
+  cluster.sync();
+  int step = 0;
+  for (;; ++step) {
+    const int n = __ldcg(counts + step % 3);
+    if (n == 0) break;
+    const int* cur = list + (size_t)(step & 1) * m;
+    int* next = list + (size_t)((step + 1) & 1) * m;
+    int* ncount = counts + (step + 1) % 3;
+    if (tid == 0) counts[(step + 2) % 3] = 0;
+    // tells the candidates above j; `warps` warps share its row, this is number w
+    auto notify = [&](int j, int w, int warps) {
+      const int e1 = rp[j + 1];
+      for (int e0 = rp[j] + 1 + w * 32; e0 < e1; e0 += warps * 32) {
+        const int i = e0 + lane < e1 ? ci[e0 + lane] : -1;
+        bool push = false;
+        if (i > j && __ldcg(s2 + i) == 1) {
+          const int q = find_offd(rp, ci, i, j);
+          push = q >= 0 && strong(va[q], beta[i]) && atomicSub(cnt + i, 1) == 1;
+        }
+        push_rows(push, i, next, ncount);
+      }
+    };
+    if (n <= block_rows) {
+      for (int w = blockIdx.x; w < n; w += gridDim.x) {
+        const int j = __ldcg(cur + w);
+        const bool mine = cf_promote<kWaveThreads / 32>(j, rp, ci, va, beta, st1, s2, tables[0], lane);
+        const bool p = __syncthreads_or(mine);
+        if (threadIdx.x == 0) s2[j] = p ? 2 : 0;
+        notify(j, threadIdx.x >> 5, kWaveThreads / 32);
+      }
+    } else {
+      for (int w = warp; w < n; w += nw) {
+        const int j = __ldcg(cur + w);
+        const bool p = cf_promote<1>(j, rp, ci, va, beta, st1, s2, table, lane);
+        if (lane == 0) s2[j] = p ? 2 : 0;
+        notify(j, 0, 1);
+      }
+    }
+    __threadfence();
+    cluster.sync();
+  }
+  if (tid == 0) *steps = step;
+  int n = 0;
+  for (int i = tid; i < m; i += nt) n += __ldcg(s2 + i) == 1;
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0 && n) atomicAdd(left, n);
+}
+
+// one round of pass 2 over the candidates left (s2 == 1), whatever the
+// pattern; s2 becomes 2 (promoted) or 0 once every candidate strong neighbour
+// below i is decided
+__global__ void __launch_bounds__(256) k_cf_pass2_round(int m, const int* __restrict__ rp,
+                                                        const int* __restrict__ ci, const double* __restrict__ va,
+                                                        const double* __restrict__ beta,
+                                                        const int* __restrict__ st1, int* s2, int* undecided) {
+  __shared__ int tables[8][kSet];
   const int i = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= m || vload(s2 + i) != 1) return;
@@ -192,11 +395,11 @@ __global__ void k_cf_pass2_round(int m, const int* __restrict__ rp, const int* _
     if (lane == 0 && undecided != nullptr) atomicAdd(undecided, 1);
     return;
   }
-  const bool p = cf_promote(i, rp, ci, va, beta, st1, s2, lane);
+  const bool p = cf_promote<1>(i, rp, ci, va, beta, st1, s2, tables[threadIdx.x >> 5], lane);
   if (lane == 0) s2[i] = p ? 2 : 0;
 }
 
-__global__ void k_cf_flags(int m, const int8_t* __restrict__ st1, const int8_t* __restrict__ s2,
+__global__ void k_cf_flags(int m, const int* __restrict__ st1, const int* __restrict__ s2,
                            int* __restrict__ is_c) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) is_c[i] = (st1[i] == -1 || s2[i] == 2) ? 1 : 0;
@@ -321,6 +524,114 @@ __global__ void k_cf_weights(int m, const int* __restrict__ rp, const int* __res
   }
 }
 
+// The same with a warp per row, for long rows (a thread per row walks the
+// P^T row of every strong F neighbour alone: 43 ms on the 31,833-row level of
+// a 64^3 hierarchy, 285 entries a row; 4.2 ms this way).  The lanes take a P^T row's entries;
+// the sums whose order is the reference's (aii, d, and an entry's own
+// additions) are still added one term at a time: matched terms of a 32-entry
+// chunk are passed round in order.  Rows of P^T longer than kPtCap accumulate
+// and search in global memory.
+constexpr int kPtCap = 256;
+constexpr double kWarpWeightsLen = 24.0;  // mean row length above which a warp takes a row
+
+// acc + the values v of the lanes in `which`, added in lane order
+__device__ __forceinline__ double add_in_order(double acc, double v, unsigned which) {
+  while (which) {
+    const int src = __ffs(which) - 1;
+    which &= which - 1;
+    acc += __shfl_sync(0xffffffffu, v, src);
+  }
+  return acc;
+}
+
+__global__ void __launch_bounds__(128) k_cf_weights_warp(int m, const int* __restrict__ rp,
+                                                         const int* __restrict__ ci, const double* __restrict__ va,
+                                                         const double* __restrict__ beta,
+                                                         const int* __restrict__ is_c,
+                                                         const int* __restrict__ core_at,
+                                                         const int* __restrict__ pt_rp,
+                                                         const int* __restrict__ pt_ci,
+                                                         const double* __restrict__ a_lc, double* pt_va) {
+  __shared__ int scol[4][kPtCap];
+  __shared__ double sacc[4][kPtCap];
+  const int i = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (i >= m) return;
+  const int tb = pt_rp[i], tn = pt_rp[i + 1] - tb;
+  if (is_c[i]) {
+    if (lane == 0) {
+      const int q = find_sorted(pt_ci, tb, tb + tn, core_at[i]);
+      if (q >= 0) pt_va[q] += 1.0;
+    }
+    return;
+  }
+  const bool in_smem = tn <= kPtCap;
+  const int* tcol = in_smem ? scol[w] : pt_ci + tb;
+  double* acc = in_smem ? sacc[w] : pt_va + tb;
+  if (in_smem)
+    for (int q = lane; q < tn; q += 32) {
+      scol[w][q] = pt_ci[tb + q];
+      sacc[w][q] = pt_va[tb + q];
+    }
+  __syncwarp();
+  const double bi = beta[i];
+  const int b = rp[i] + 1, e1 = rp[i + 1];
+  double aii = rp[i] < e1 ? va[rp[i]] : 0.0;
+  for (int e0 = b; e0 < e1; e0 += 32) {
+    const int e = e0 + lane;
+    const double v = e < e1 ? va[e] : 0.0;
+    aii = add_in_order(aii, v, __ballot_sync(0xffffffffu, e < e1 && fabs(v) < bi));
+  }
+  for (int e0 = b; e0 < e1; e0 += 32) {
+    const int e = e0 + lane;
+    const double v = e < e1 ? va[e] : 0.0;
+    const int l = e < e1 ? ci[e] : 0;
+    const bool st = e < e1 && !(fabs(v) < bi);
+    const int core = st && is_c[l] ? core_at[l] : -1;
+    const int lb = st && core < 0 ? pt_rp[l] : 0, le = st && core < 0 ? pt_rp[l + 1] : 0;
+    for (unsigned todo = __ballot_sync(0xffffffffu, st); todo != 0; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const double ve = __shfl_sync(0xffffffffu, v, src);
+      const int c = __shfl_sync(0xffffffffu, core, src);
+      const int pb = __shfl_sync(0xffffffffu, lb, src), pe = __shfl_sync(0xffffffffu, le, src);
+      if (c >= 0) {
+        if (lane == 0) {
+          const int q = find_sorted(tcol, 0, tn, c);
+          if (q >= 0) acc[q] += fabs(ve / aii);
+        }
+        __syncwarp();
+        continue;
+      }
+      double d = 0.0, a0 = 0.0;
+      int q0 = -1;  // the first chunk's match is kept for the second pass
+      for (int p0 = pb; p0 < pe; p0 += 32) {
+        const bool on = p0 + lane < pe;
+        const double a = on ? a_lc[p0 + lane] : 0.0;
+        const int q = on ? find_sorted(tcol, 0, tn, pt_ci[p0 + lane]) : -1;
+        if (p0 == pb) {
+          a0 = a;
+          q0 = q;
+        }
+        d = add_in_order(d, a, __ballot_sync(0xffffffffu, q >= 0));
+      }
+      if (fabs(d * aii) < 1e-16) continue;
+      for (int p0 = pb; p0 < pe; p0 += 32) {
+        double a = a0;
+        int q = q0;
+        if (p0 != pb) {
+          const bool on = p0 + lane < pe;
+          a = on ? a_lc[p0 + lane] : 0.0;
+          q = on ? find_sorted(tcol, 0, tn, pt_ci[p0 + lane]) : -1;
+        }
+        if (q >= 0) acc[q] += fabs(ve * a / (d * aii));
+      }
+      __syncwarp();
+    }
+  }
+  if (in_smem)
+    for (int q = lane; q < tn; q += 32) pt_va[tb + q] = sacc[w][q];
+}
+
 // P(c, i) received the same additions as P^T(i, c)
 __global__ void k_cf_p_vals(int nc, const int* __restrict__ p_rp, const int* __restrict__ p_ci,
                             const int* __restrict__ pt_rp, const int* __restrict__ pt_ci,
@@ -335,7 +646,7 @@ __global__ void k_cf_p_vals(int nc, const int* __restrict__ p_rp, const int* __r
 }
 
 // launches `launch(counter)` in batches, the last of each batch counting the
-// rows left; returns the number of rounds run
+// rows left, until none are; returns the number of rounds run
 template <class F>
 int run_rounds(const afp_context* ctx, int m, DevBuf<int>& counter, F launch, const char* what) {
   int rounds = 0;
@@ -353,6 +664,34 @@ int run_rounds(const afp_context* ctx, int m, DevBuf<int>& counter, F launch, co
   }
 }
 
+// Launches a wave kernel as one cluster, of 16 blocks where the device can
+// place one that large, else of the portable 8.
+template <class... K, class... Args>
+void launch_wave(const afp_context* ctx, const char* what, size_t smem, void (*kernel)(K...), Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.dynamicSmemBytes = smem;
+  AFP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cfg.blockDim = kWaveThreads;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  AFP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (unsigned size : {16u, 8u}) {
+    at[0].val.clusterDim = {size, 1, 1};
+    cfg.gridDim = size;
+    int fit = 0;
+    if (size > 8 && (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess || fit < 1)) {
+      cudaGetLastError();
+      continue;
+    }
+    AFP_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    break;
+  }
+  check_launch(ctx, what);
+}
+
 }  // namespace
 
 int gpu_project(const afp_context* ctx, int64_t m64, const int* rp, const int* ci, const double* va, double alpha,
@@ -364,23 +703,34 @@ int gpu_project(const afp_context* ctx, int64_t m64, const int* rp, const int* c
   sync(ctx);
   const unsigned warp_grid = grid_for((int64_t)m * 32, 256);
   DevBuf<double> beta(ctx, m);
-  DevBuf<uint8_t> in_edge(ctx, nnz > 0 ? nnz : 1);
-  DevBuf<int8_t> st1(ctx, m), s2(ctx, m);
-  DevBuf<int> counter(ctx, 1);
+  DevBuf<int> st1(ctx, m), s2(ctx, m), cnt(ctx, m), list(ctx, 2 * (size_t)m);
+  DevBuf<int> waves(ctx, 9);  // list counts of both passes, steps of both, candidates left
   k_cf_beta<<<warp_grid, 256, 0, s>>>(m, rp, va, alpha, beta.get());
-  k_cf_in_edges<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), in_edge.get());
   st1.zero();
-  out.rounds1 = run_rounds(
-      ctx, m, counter,
-      [&](int* cnt) { k_cf_pass1<<<grid_for(m, 256), 256, 0, s>>>(m, rp, ci, in_edge.get(), st1.get(), cnt); },
-      "C/F pass 1");
+  cnt.zero();
+  waves.zero();
+  k_cf_count_in<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), cnt.get());
+  const double len = (double)nnz / (double)m;  // mean row
+  launch_wave(ctx, "C/F pass 1", 0, len <= 24.0 ? k_cf_pass1_wave<8> : k_cf_pass1_wave<32>, m, rp, ci, va,
+              (const double*)beta.get(), st1.get(), cnt.get(), list.get(), waves.get(), waves.get() + 6);
   k_cf_pass2_candidates<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), st1.get(), s2.get());
-  out.rounds2 = run_rounds(
-      ctx, m, counter,
-      [&](int* cnt) {
-        k_cf_pass2_round<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), st1.get(), s2.get(), cnt);
-      },
-      "C/F pass 2");
+  k_cf_pass2_count<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), s2.get(), cnt.get());
+  launch_wave(ctx, "C/F pass 2", kWaveThreads / 32 * kSet * sizeof(int), k_cf_pass2_wave, m, rp, ci, va, (const double*)beta.get(), (const int*)st1.get(),
+              s2.get(), cnt.get(), list.get(), waves.get() + 3, waves.get() + 7, waves.get() + 8, len > 64.0 ? 96 : 0);
+  int hw[3] = {0, 0, 0};
+  copy(ctx, hw, waves.get() + 6, sizeof(hw));
+  sync(ctx);
+  out.rounds1 = hw[0];
+  out.rounds2 = hw[1];
+  if (hw[2] != 0) {
+    DevBuf<int> counter(ctx, 1);
+    out.rounds2 += run_rounds(
+        ctx, m, counter,
+        [&](int* left) {
+          k_cf_pass2_round<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), st1.get(), s2.get(), left);
+        },
+        "C/F pass 2 (nonsymmetric pattern)");
+  }
   DevBuf<int> is_c(ctx, m), core_at(ctx, m + 1);
   k_cf_flags<<<grid_for(m, 256), 256, 0, s>>>(m, st1.get(), s2.get(), is_c.get());
   const int nc = (int)exclusive_scan(ctx, is_c.get(), core_at.get(), m);
@@ -415,8 +765,13 @@ int gpu_project(const afp_context* ctx, int64_t m64, const int* rp, const int* c
   k_cf_a_lc<<<grid_for(m, 128), 128, 0, s>>>(m, rp, ci, va, T.rp.get(), T.ci.get(), core_point.get(), a_lc.get());
   T.va.alloc(ctx, T.nnz);
   T.va.zero();
-  k_cf_weights<<<grid_for(m, 128), 128, 0, s>>>(m, rp, ci, va, beta.get(), is_c.get(), core_at.get(), T.rp.get(),
-                                                T.ci.get(), a_lc.get(), T.va.get());
+  if ((double)nnz > kWarpWeightsLen * (double)m)
+    k_cf_weights_warp<<<grid_for((int64_t)m * 32, 128), 128, 0, s>>>(m, rp, ci, va, beta.get(), is_c.get(),
+                                                                     core_at.get(), T.rp.get(), T.ci.get(),
+                                                                     a_lc.get(), T.va.get());
+  else
+    k_cf_weights<<<grid_for(m, 128), 128, 0, s>>>(m, rp, ci, va, beta.get(), is_c.get(), core_at.get(), T.rp.get(),
+                                                  T.ci.get(), a_lc.get(), T.va.get());
   P.va.alloc(ctx, P.nnz);
   k_cf_p_vals<<<grid_for(nc, 128), 128, 0, s>>>(nc, P.rp.get(), P.ci.get(), T.rp.get(), T.ci.get(), T.va.get(),
                                                 P.va.get());
