@@ -11,8 +11,7 @@
 // by binary searches on the sorted rows, which return the same entries.
 #include <algorithm>
 #include <cmath>
-#include <queue>
-#include <tuple>
+#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 
@@ -24,14 +23,14 @@ namespace afp {
 namespace {
 
 // value of (i, j) in a [diag, ascending others] row, 0 when absent
-inline double entry(const HostCSR& M, int i, int j) {
+inline double entry(const CSRRef& M, int i, int j) {
   const int b = M.rowptr[i], e = M.rowptr[i + 1];
   if (b == e) return 0.0;
   if (M.cols[b] == j) return M.vals[b];
-  const int* lo = M.cols.data() + b + 1;
-  const int* hi = M.cols.data() + e;
+  const int* lo = M.cols + b + 1;
+  const int* hi = M.cols + e;
   const int* p = std::lower_bound(lo, hi, j);
-  return (p != hi && *p == j) ? M.vals[p - M.cols.data()] : 0.0;
+  return (p != hi && *p == j) ? M.vals[p - M.cols] : 0.0;
 }
 
 }  // namespace
@@ -284,18 +283,23 @@ namespace {
 
 // Greedy colouring in row order: row i takes the smallest colour that none of
 // its coupled, already coloured rows has (max_colors: the overflow class).
-int greedy_color(const HostCSR& A, int max_colors, std::vector<int>& color) {
+// A row that has met every colour is decided: the long rows of coarse levels
+// are left after a few entries.
+int greedy_color(const CSRRef& A, int max_colors, std::vector<int>& color) {
   const int m = (int)A.m;
   color.assign(m, -1);
   std::vector<int> mark(max_colors + 1, -1);
   int used = 0;
   bool overflow = false;
   for (int i = 0; i < m; ++i) {
+    int met = 0;
     for (int q = A.rowptr[i] + 1; q < A.rowptr[i + 1]; ++q) {
       const int k = A.cols[q];
-      if (color[k] < 0) continue;
+      const int ck = color[k];
+      if (ck < 0 || mark[ck] == i) continue;
       if (A.vals[q] == 0.0 && entry(A, k, i) == 0.0) continue;  // no coupling either way
-      mark[color[k]] = i;
+      mark[ck] = i;
+      if (ck < max_colors && ++met == max_colors) break;
     }
     int c = 0;
     while (c < max_colors && mark[c] == i) ++c;
@@ -306,18 +310,60 @@ int greedy_color(const HostCSR& A, int max_colors, std::vector<int>& color) {
   return overflow ? max_colors + 1 : used;
 }
 
+// A set of numbers in [0, n): a bitmap with 64-ary summary levels.
+class RankSet {
+ public:
+  explicit RankSet(int n) {
+    int64_t w = n;
+    do {
+      w = (w + 63) / 64;
+      level_.emplace_back((size_t)w, 0);
+    } while (w > 1);
+  }
+  void insert(int i) {
+    for (auto& l : level_) {
+      uint64_t& w = l[(size_t)(i >> 6)];
+      const bool had = w != 0;
+      w |= uint64_t(1) << (i & 63);
+      if (had) return;
+      i >>= 6;
+    }
+  }
+  void erase(int i) {
+    for (auto& l : level_) {
+      uint64_t& w = l[(size_t)(i >> 6)];
+      w &= ~(uint64_t(1) << (i & 63));
+      if (w != 0) return;
+      i >>= 6;
+    }
+  }
+  bool empty() const { return level_.back()[0] == 0; }
+  int first() const {
+    int64_t i = 0;
+    for (size_t l = level_.size(); l-- > 0;) i = i * 64 + __builtin_ctzll(level_[l][(size_t)i]);
+    return (int)i;
+  }
+
+ private:
+  std::vector<std::vector<uint64_t>> level_;
+};
+
 // DSATUR (Brelaz): repeatedly colours the uncoloured row whose coupled rows
 // already show the most distinct colours (ties: more couplings, then the
 // lower row), with the smallest colour they leave free.  On mesh graphs it
 // finds colourings close to the fewest classes where row-order greedy
 // colouring needs about twice as many (the 3D Kuhn-split lattice: 4 against
-// 8).  Returns the colours used, or max_colors + 1 if some row found no free
-// colour below max_colors (it is then left in the overflow class).
-int dsatur_color(const HostCSR& A, int max_colors, std::vector<int>& color) {
+// 8).  Returns the colours used; gives up, returning `bound`, once it needs
+// that many.  Couplings and row order are fixed, so rows are ranked by them
+// once and each saturation keeps the set of its rows' ranks: a step is a few
+// word operations (a queue of keys with stale entries took 19 ms on 19,683
+// rows of 27 entries, this takes 5).
+int dsatur_color(const CSRRef& A, int bound, std::vector<int>& color) {
   const int m = (int)A.m;
   // coupled neighbours (a nonzero entry either way), as adjacency lists
   std::vector<int> off(m + 1, 0), adj;
-  adj.reserve(A.nnz());
+  adj.reserve((size_t)A.rowptr[m]);
+  int most = 0;
   for (int i = 0; i < m; ++i) {
     for (int q = A.rowptr[i] + 1; q < A.rowptr[i + 1]; ++q) {
       const int k = A.cols[q];
@@ -325,42 +371,48 @@ int dsatur_color(const HostCSR& A, int max_colors, std::vector<int>& color) {
       adj.push_back(k);
     }
     off[i + 1] = (int)adj.size();
+    most = std::max(most, off[i + 1] - off[i]);
+  }
+  // rank: more couplings first, then the lower row (counting sort)
+  std::vector<int> at(most + 2, 0), rank(m), row_of(m);
+  for (int i = 0; i < m; ++i) at[most - (off[i + 1] - off[i]) + 1]++;
+  for (int d = 0; d <= most; ++d) at[d + 1] += at[d];
+  for (int i = 0; i < m; ++i) {
+    const int r = at[most - (off[i + 1] - off[i])]++;
+    rank[i] = r;
+    row_of[r] = i;
   }
   color.assign(m, -1);
-  std::vector<uint64_t> seen(m, 0);  // colours present among coupled rows (max_colors <= 63)
-  std::vector<int> sat(m, 0);
-  using Key = std::tuple<int, int, int>;  // (saturation, couplings, -row)
-  std::priority_queue<Key> pq;
-  for (int i = 0; i < m; ++i) pq.push(Key(0, off[i + 1] - off[i], -i));
-  int used = 0;
-  bool overflow = false;
-  while (!pq.empty()) {
-    const Key top = pq.top();
-    pq.pop();
-    const int i = -std::get<2>(top);
-    if (color[i] >= 0 || std::get<0>(top) != sat[i]) continue;  // stale entry
-    int c = 0;
-    while (c < max_colors && ((seen[i] >> c) & 1u)) ++c;
+  std::vector<uint64_t> seen(m, 0);  // colours present among coupled rows (bound <= 63)
+  std::vector<uint8_t> sat(m, 0);
+  std::vector<RankSet> by_sat(1, RankSet(m));
+  for (int r = 0; r < m; ++r) by_sat[0].insert(r);
+  int used = 0, top = 0;
+  for (int left = m; left > 0; --left) {
+    while (by_sat[top].empty()) --top;
+    const int r = by_sat[top].first(), i = row_of[r];
+    by_sat[top].erase(r);
+    const int c = __builtin_ctzll(~seen[i]);
+    if (c + 1 >= bound) return bound;
     color[i] = c;
-    if (c == max_colors) {
-      overflow = true;
-      continue;
-    }
     used = std::max(used, c + 1);
     for (int q = off[i]; q < off[i + 1]; ++q) {
       const int k = adj[q];
       if (color[k] >= 0 || ((seen[k] >> c) & 1u)) continue;
       seen[k] |= uint64_t(1) << c;
-      ++sat[k];
-      pq.push(Key(sat[k], off[k + 1] - off[k], -k));
+      by_sat[sat[k]].erase(rank[k]);
+      const int t = ++sat[k];
+      if (t == (int)by_sat.size()) by_sat.emplace_back(m);
+      by_sat[t].insert(rank[k]);
+      top = std::max(top, t);
     }
   }
-  return overflow ? max_colors + 1 : used;
+  return used;
 }
 
 }  // namespace
 
-int host_color(const HostCSR& A, int max_colors, std::vector<int>& color) {
+int host_color(const CSRRef& A, int max_colors, std::vector<int>& color) {
   const int greedy = greedy_color(A, max_colors, color);
   // A level that needs the overflow class keeps the row-order classes (each
   // a maximal independent set of the rows left, which keeps the l1-Jacobi
@@ -368,7 +420,7 @@ int host_color(const HostCSR& A, int max_colors, std::vector<int>& color) {
   // dependent steps per Gauss-Seidel sweep.
   if (greedy > max_colors || greedy <= 2 || max_colors > 63) return greedy;
   std::vector<int> ds;
-  const int k = dsatur_color(A, max_colors, ds);
+  const int k = dsatur_color(A, greedy, ds);
   if (k < greedy) {
     color.swap(ds);
     return k;

@@ -44,6 +44,15 @@ struct HostCSR {
   int64_t nnz() const { return rowptr.empty() ? 0 : rowptr[m]; }
 };
 
+// The arrays of a HostCSR, which stay where they are when it is moved.
+struct CSRRef {
+  int64_t m = 0;
+  const int* rowptr = nullptr;
+  const int* cols = nullptr;
+  const double* vals = nullptr;
+  CSRRef(const HostCSR& H) : m(H.m), rowptr(H.rowptr.data()), cols(H.cols.data()), vals(H.vals.data()) {}
+};
+
 // A device CSR (AFEPack layout for square levels, ascending rows for P, P^T).
 struct DevCSR {
   int64_t m = 0, n = 0, nnz = 0;
@@ -72,6 +81,6 @@ void host_lazy_project(const HostCSR& M, HostCSR& P, HostCSR& Pt);
 // Greedy colouring of a square matrix's graph (nonzero off-diagonal entries
 // couple rows): colour[i] < max_colors, or max_colors for rows that found no
 // free colour (the overflow class).  Returns the number of classes used.
-int host_color(const HostCSR& A, int max_colors, std::vector<int>& color);
+int host_color(const CSRRef& A, int max_colors, std::vector<int>& color);
 
 }  // namespace afp
