@@ -709,7 +709,7 @@ void build_pattern_nd(const afp_space* sp, Pattern& pat) {
   while (wpb > 1 && (size_t)wpb * cap * sizeof(int) > 96 * 1024) wpb >>= 1;
   size_t smem = (size_t)wpb * cap * sizeof(int);
   AFP_REQUIRE(smem <= 200 * 1024, AFP_ERR_UNSUPPORTED, "a DOF touches too many cells for the pattern kernel");
-  AFP_CUDA(cudaFuncSetAttribute(k_pattern<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(k_pattern<ND>);
   unsigned grid = (unsigned)std::min<int64_t>((sp->n_dof + wpb - 1) / wpb, (int64_t)ctx->sm_count * 32);
   DevBuf<int> row_len(ctx, sp->n_dof);
   k_pattern<ND><<<grid, wpb * 32, smem, ctx->stream>>>(sp->n_dof, sp->inc_ptr.get(), sp->inc.get(), sp->elem_dof.get(),
@@ -738,7 +738,7 @@ void gather_values_nd(const afp_space* sp, const Pattern& pat, const double* eK,
   const int wpb = 4;
   size_t smem = (size_t)wpb * rcap * (2 * sizeof(double) + sizeof(int));
   AFP_REQUIRE(smem <= 200 * 1024, AFP_ERR_UNSUPPORTED, "matrix row too long for the scatter kernel");
-  AFP_CUDA(cudaFuncSetAttribute(k_gather_values<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(k_gather_values<ND>);
   unsigned grid = (unsigned)std::min<int64_t>((pat.m + wpb - 1) / wpb, (int64_t)ctx->sm_count * 32);
   k_gather_values<ND><<<grid, wpb * 32, smem, ctx->stream>>>(pat.m, sp->inc_ptr.get(), sp->inc.get(),
                                                              sp->elem_dof.get(), pat.rowptr.get(), pat.cols.get(), eK,

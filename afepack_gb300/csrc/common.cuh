@@ -156,6 +156,18 @@ class DevBuf {
   const afp_context* ctx_ = nullptr;
 };
 
+// Dynamic shared memory a block may ask for with allow_smem (of 227 KB).
+constexpr int kMaxDynamicSmem = 200 * 1024;
+
+// Lets `kernel` be launched with up to kMaxDynamicSmem of dynamic shared
+// memory.  The limit belongs to the function, not to the launch: it is always
+// set to the same value, since a thread that lowered it to its own size could
+// do so between another thread's setting and launch, which would then fail.
+template <class K>
+void allow_smem(K kernel) {
+  AFP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem));
+}
+
 // Host <-> device copy of any pointer pair (unified addressing).
 void copy(const afp_context* ctx, void* dst, const void* src, size_t bytes);
 void sync(const afp_context* ctx);

