@@ -766,7 +766,7 @@ void copy2d(const afp_context* ctx, int64_t rows, int64_t cols, const double* sr
 
 // Dense inverse of the coarsest level of the hierarchy.  A symmetric positive
 // definite matrix, which every SPD system's hierarchy ends in, takes
-// spd_inverse() (6,744 rows: 49 ms; the sweep below: 706 ms).  Any other (a
+// spd_inverse() (6,744 rows: 35 ms; the sweep below: 706 ms).  Any other (a
 // nonsymmetric or indefinite system) needs pivots and is swept in FP64: up to kPanel rows by Gauss-Jordan with partial
 // pivoting, larger ones in place on the output, kPanel pivots at a time --
 // with the block pivot P, the panel rows R, the panel columns C and the rest S,

@@ -27,16 +27,17 @@
 // FP64 products: 2.2e-15, 8e-14 and 2e-11 of its norm on either side; with
 // 8 digits the small entries of the last two were 40 and more times worse.
 //
-// Measured (GB300, whole inverse): 6,744 rows 49 ms against 706 ms with the
+// Measured (GB300, whole inverse): 6,744 rows 35 ms against 706 ms with the
 // pivoted FP64 sweep of solve.cu (two launches per pivot, FP64 products);
-// 2,196 rows 4.5 against 68 ms.  At 6,744 rows the trailing updates take 36
-// of the 49 ms, the panels' own inverses 8.
+// 2,048 rows 3.6 ms, 256 rows 0.39 ms.  At 6,744 rows the trailing updates
+// take 24 of the 35 ms, the panels' own inverses 7.
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <cstdint>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "solve.cuh"
 
 namespace afp {
@@ -86,51 +87,82 @@ __global__ void k_spd_pivot_block(int64_t n, int64_t k0, int pb, const double* _
   P[t] = v;
 }
 
+// 1/p for a normal p by Newton-Raphson from the hardware's approximation
+__device__ __forceinline__ double newton_reciprocal(double p) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
+#pragma unroll
+  for (int i = 0; i < 2; ++i) y = fma(y, fma(-p, y, 1.0), y);
+  return y;
+}
+
 // One step of the block Gauss-Jordan inverse of P: kSub pivots, from `in` to
-// `out`.  A block owns 32 rows x kSub columns and inverts the kSub x kSub
-// pivot itself: 2 us of FP64 latency in every block instead of one more
-// launch in the chain.
+// `out`.  A block owns 32 rows x kSub columns; its first warp inverts the
+// kSub x kSub pivot itself, in registers (lane l: row l / 2, eight columns),
+// instead of one more launch in the chain.  The 256 pivots of a panel follow
+// one another, each a reciprocal and a rank-1 update whose FP64 instructions
+// take 16 clocks apiece, so every entry is updated by one multiply-add, the
+// pivot row and column included: 15 us a step, against 19 by four warps with
+// a division and two barriers per pivot.
 __global__ void __launch_bounds__(128) k_spd_sweep(int kk, const double* __restrict__ in, double* __restrict__ out,
                                                    int* __restrict__ flag) {
   __shared__ double D[kSub][kSub + 1], R[kSub][kSub + 1], T[kSub][kSub + 1], Cc[32][kSub + 1];
   const int tid = threadIdx.x;
   const int jb = blockIdx.x, ib = blockIdx.y;
   const int p0 = kk * kSub, c0 = jb * kSub, r0 = ib * 32;
-  for (int t = tid; t < kSub * kSub; t += 128) {
-    const int r = t / kSub, c = t % kSub;
-    D[r][c] = in[(p0 + r) * kB + p0 + c];
-    R[r][c] = in[(p0 + r) * kB + c0 + c];
+  pdl_wait();
+  if (tid < 32) {
+    const int row = tid >> 1, half = tid & 1;
+    double d[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) d[e] = in[(p0 + row) * kB + p0 + half * 8 + e];
+    bool bad = false;
+#pragma unroll
+    for (int q = 0; q < kSub; ++q) {
+      const int h = q >> 3, qc = q & 7;
+      const double p = __shfl_sync(0xffffffffu, d[qc], 2 * q + h);
+      const double f = __shfl_sync(0xffffffffu, d[qc], (tid & ~1) + h);
+      bad |= !(p > 0.0);
+      const double y = newton_reciprocal(p);
+      const double g = row == q ? -y : f * y;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        double r = __shfl_sync(0xffffffffu, d[e], 2 * q + half);
+        const bool pc = half == h && e == qc;  // the pivot's column
+        if (pc) r = 1.0;
+        d[e] = fma(-g, r, (pc || row == q) ? 0.0 : d[e]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) D[row][half * 8 + e] = d[e];
+    if (bad && tid == 0) atomicOr(flag, 1);
+  } else {
+    for (int t = tid - 32; t < kSub * kSub; t += 96) R[t / kSub][t % kSub] = in[(p0 + t / kSub) * kB + c0 + t % kSub];
+    for (int t = tid - 32; t < 32 * kSub; t += 96) Cc[t / kSub][t % kSub] = in[(r0 + t / kSub) * kB + p0 + t % kSub];
   }
-  for (int t = tid; t < 32 * kSub; t += 128) Cc[t / kSub][t % kSub] = in[(r0 + t / kSub) * kB + p0 + t % kSub];
-  __syncthreads();
-  // in-place inverse: thread t holds entries (r, c) and (r + 8, c)
   const int r = tid / kSub, c = tid % kSub;
-  for (int q = 0; q < kSub; ++q) {
-    const double p = D[q][q];
-    const double ip = 1.0 / p;
-    if (!(p > 0.0) && tid == 0) atomicOr(flag, 1);
-    const double rowv = (c == q ? 1.0 : D[q][c]) * ip;
-    const double f0 = D[r][q], f1 = D[r + 8][q];
-    const double a0 = c == q ? 0.0 : D[r][c], a1 = c == q ? 0.0 : D[r + 8][c];
-    __syncthreads();
-    D[r][c] = r == q ? rowv : a0 - f0 * rowv;
-    D[r + 8][c] = r + 8 == q ? rowv : a1 - f1 * rowv;
-    __syncthreads();
-  }
+  double old[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) old[h] = in[(r0 + r + 8 * h) * kB + c0 + c];
+  __syncthreads();
   // T = Q R_j, or Q itself in the pivot's own columns
+#pragma unroll
   for (int h = 0; h < 2; ++h) {
     double s = 0;
+#pragma unroll
     for (int q = 0; q < kSub; ++q) s += D[r + 8 * h][q] * R[q][c];
     T[r + 8 * h][c] = jb == kk ? D[r + 8 * h][c] : s;
   }
   __syncthreads();
+#pragma unroll
   for (int h = 0; h < 4; ++h) {
     const int rr = r + 8 * h, row = r0 + rr;
     double v;
     if (row >= p0 && row < p0 + kSub) {
       v = T[row - p0][c];
     } else {
-      v = jb == kk ? 0.0 : in[row * kB + c0 + c];
+      v = jb == kk ? 0.0 : old[h];
+#pragma unroll
       for (int q = 0; q < kSub; ++q) v -= Cc[rr][q] * T[q][c];
     }
     out[row * kB + c0 + c] = v;
@@ -324,6 +356,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// an integer below 2^51 as a double: placed in the fraction of 3 * 2^51, which is then taken off
+__device__ __forceinline__ double exact_double(long long v) {
+  return __longlong_as_double(0x4338000000000000LL + v) - 0x1.8p52;
+}
+
 constexpr uint32_t kABytes = kTM * kKC * 2, kBBytes = kTN * kKC * 2;  // one digit's tile of a stage
 constexpr uint32_t kStageBytes = kS * (kABytes + kBBytes);
 constexpr int kStages = 2;
@@ -335,10 +372,13 @@ constexpr int kProdThreads = 192;
 // to the tiles of the lower triangle of `out` (row stride ld) that the panel
 // [k0, k0 + kB) does not own; otherwise stored to `out`.  One tile per block:
 // warp 4 streams the digits, warp 5 issues the products, warps 0-3 put the
-// sums together.  A tile is 720 products of 128 x 64 x 16 (23K clocks) and
-// 8,192 entries of five FP64-rate operations (20K clocks), which bounds it.
+// sums together.  A tile is 720 products of 128 x 64 x 16, which read 6 KB of
+// shared memory each (48 clocks, 35K in all), and then 8,192 entries of six
+// FP64 operations (25K clocks); the accumulators fill tensor memory, so the
+// two do not overlap: 46 us a tile.  (73 us with integer conversions in place
+// of the fraction trick and the entries to update read after the products.)
 template <bool UPDATE>
-__global__ void __launch_bounds__(kProdThreads) k_spd_product(const __nv_bfloat16* __restrict__ A, int64_t groups_a,
+__global__ void __launch_bounds__(kProdThreads, 1) k_spd_product(const __nv_bfloat16* __restrict__ A, int64_t groups_a,
                                                               const double* __restrict__ sa,
                                                               const __nv_bfloat16* __restrict__ B, int64_t groups_b,
                                                               const double* __restrict__ sb, int64_t rows,
@@ -412,15 +452,27 @@ __global__ void __launch_bounds__(kProdThreads) k_spd_product(const __nv_bfloat1
     }
     mma_commit(&done);
   } else if (warp < 4) {
+    // the entries to update, read while the products run: lane l holds columns l and 32 + l of its warp's 32 rows
+    const int64_t ja = j0 + lane, jb = j0 + 32 + lane, iw = i0 + warp * 32;
+    double old[32][2];
+    if (UPDATE) {
+#pragma unroll
+      for (int r = 0; r < 32; ++r) {
+        const int64_t i = iw + r;
+        old[r][0] = i < rows && ja <= i ? out[i * ld + ja] : 0.0;
+        old[r][1] = i < rows && jb <= i ? out[i * ld + jb] : 0.0;
+      }
+    }
+    const double rs = sa[iw + lane] * (UPDATE && i0 >= k0 ? -0x1p-68 : 0x1p-68);  // 2^-12 of the digits' scale, 2^-56 of lo's units
+    const double ca = sb[ja], cb = sb[jb];
     const bool ok = bar_wait(&done, 0);
     if (!ok) {
       if (lane == 0) atomicOr(error, 2);
     } else {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // the stages are free: warp w keeps its 32 rows of the tile there
-      double* tile = reinterpret_cast<double*>(prod_raw + (base - smem_u32(prod_raw))) + warp * 32 * (kTN + 1);
-      const int64_t row = i0 + warp * 32 + lane;
-      const double rs = sa[row] * 0x1p-68;  // 2^-12 of the digits' scale, 2^-56 of the units of `lo`
+      // the stages are free: warp w puts its rows' (hi, lo) there
+      double2* tile = reinterpret_cast<double2*>(prod_raw + (base - smem_u32(prod_raw))) + warp * 32 * (kTN + 1);
+#pragma unroll 1
       for (int c = 0; c < kTN; c += 8) {
         float v[kAcc][8];
 #pragma unroll
@@ -428,31 +480,27 @@ __global__ void __launch_bounds__(kProdThreads) k_spd_product(const __nv_bfloat1
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          long long hi = 0, lo = 0;
+          int w[kAcc];
 #pragma unroll
-          for (int s = 0; s < 4; ++s) hi = hi * 128 + __float2int_rn(v[s][e] * __int_as_float((127 + 7 * s) << 23));
-#pragma unroll
-          for (int s = 4; s < 7; ++s) lo = lo * 128 + __float2int_rn(v[s][e] * __int_as_float((127 + 7 * s) << 23));
-          lo = lo * 16384 + __float2int_rn(v[7][e] * 0x1p56f);
-          tile[lane * (kTN + 1) + c + e] = fma((double)hi, 0x1p35, (double)lo) * rs;
+          for (int s = 0; s < 7; ++s) w[s] = __float2int_rn(v[s][e] * __int_as_float((127 + 7 * s) << 23));
+          w[7] = __float2int_rn(v[7][e] * 0x1p56f);
+          // hi = the weights 0..3 in units of weight 3, lo = the rest in units of weight 8: |hi| < 2^43, |lo| < 2^51
+          const long long hi = (long long)(w[0] * 128 + w[1]) * 16384 + (w[2] * 128 + w[3]);
+          const long long lo = (long long)(w[4] * 128 + w[5]) * 2097152 + ((long long)w[6] * 16384 + w[7]);
+          tile[lane * (kTN + 1) + c + e] = make_double2(exact_double(hi), exact_double(lo));
         }
       }
       __syncwarp();
-      const double c0 = sb[j0 + lane], c1 = sb[j0 + 32 + lane];
-      const int64_t ja = j0 + lane, jb = j0 + 32 + lane;
+#pragma unroll
       for (int r = 0; r < 32; ++r) {
-        const int64_t i = i0 + warp * 32 + r;
-        if (i >= rows) break;
-        double* o = out + i * ld;
-        const double ta = tile[r * (kTN + 1) + lane] * c0, tb = tile[r * (kTN + 1) + 32 + lane] * c1;
-        if (UPDATE) {
-          const double sg = i0 >= k0 ? -1.0 : 1.0;
-          if (ja <= i) o[ja] += sg * ta;
-          if (jb <= i) o[jb] += sg * tb;
-        } else {
-          if (ja < cols) o[ja] = ta;
-          if (jb < cols) o[jb] = tb;
-        }
+        const int64_t i = iw + r;
+        const double s = __shfl_sync(0xffffffffu, rs, r);
+        const double2 ta = tile[r * (kTN + 1) + lane], tb = tile[r * (kTN + 1) + 32 + lane];
+        const double sca = s * ca, scb = s * cb;
+        const double va = fma(ta.y, sca, fma(ta.x, sca * 0x1p35, UPDATE ? old[r][0] : 0.0));
+        const double vb = fma(tb.y, scb, fma(tb.x, scb * 0x1p35, UPDATE ? old[r][1] : 0.0));
+        if (i < rows && (UPDATE ? ja <= i : ja < cols)) out[i * ld + ja] = va;
+        if (i < rows && (UPDATE ? jb <= i : jb < cols)) out[i * ld + jb] = vb;
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -498,7 +546,7 @@ bool spd_inverse(const afp_context* ctx, int64_t n, double* M) {
     check_launch(ctx, "spd pivot block");
     double *in = P0.get(), *out = P1.get();
     for (int kk = 0; kk * kSub < pb; ++kk) {
-      k_spd_sweep<<<dim3(kB / kSub, kB / 32), 128, 0, ctx->stream>>>(kk, in, out, flag.get());
+      launch_pdl(ctx->stream, dim3(kB / kSub, kB / 32), 128, 0, k_spd_sweep, kk, (const double*)in, out, flag.get());
       check_launch(ctx, "spd panel sweep");
       std::swap(in, out);
     }
