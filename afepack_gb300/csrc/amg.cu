@@ -144,8 +144,10 @@ const float* l1<float>(const Level& L) {
   return L.l1d32.get();
 }
 
+// smooth_step sweeps; from_zero: forward, from an iterate of zeros that is
+// not read (the first sweep writes every row)
 template <class X>
-void smooth(afp_amg* h, int l, X* x, const X* r, bool backward) {
+void smooth(afp_amg* h, int l, X* x, const X* r, bool backward, bool from_zero) {
   const Level& L = h->lv[l];
   CSRView<X> A = L.A<X>();
   const int K = (int)L.cls.size() - 1;
@@ -153,25 +155,27 @@ void smooth(afp_amg* h, int l, X* x, const X* r, bool backward) {
     for (int q = 0; q < K; ++q) {
       const int c = backward ? K - 1 - q : q;
       const int64_t r0 = L.cls[c], r1 = L.cls[c + 1];
+      const bool first = from_zero && s == 0;
       if (L.overflow && c == K - 1)
-        jacobi_l1_class<X>(h->ctx, A, r0, r1, x, r, l1<X>(L), lvt<X>(h, l));
+        jacobi_l1_class<X>(h->ctx, A, r0, r1, x, r, l1<X>(L), lvt<X>(h, l), first);
       else
-        gs_class<X>(h->ctx, A, r0, r1, x, r);
+        gs_class<X>(h->ctx, A, r0, r1, x, r, first);
     }
   }
 }
 
-// One V-cycle on x0 (level-0 solve order) for right-hand side r0.
+// One V-cycle from zero for right-hand side r0; x0 takes the result (level-0
+// solve order).
 template <class X, class PV>
-void vcycle(afp_amg* h, X* x0, const X* r0, bool zero_init) {
+void vcycle(afp_amg* h, X* x0, const X* r0) {
   const afp_context* ctx = h->ctx;
   const int t = h->t;
   for (int l = 0; l < t; ++l) {
     Level& L = h->lv[l];
     X* x = l == 0 ? x0 : lvx<X>(h, l);
     const X* r = l == 0 ? r0 : lvr<X>(h, l);
-    if (l > 0 || zero_init) fill_zero<X>(ctx, L.n, x);
-    smooth<X>(h, l, x, r, false);
+    if (h->opts.smooth_step == 0) fill_zero<X>(ctx, L.n, x);
+    smooth<X>(h, l, x, r, false, true);
     residual<X>(ctx, L.A<X>(), x, r, lvt<X>(h, l));
     CSRView<PV> P{h->lv[l + 1].n, L.prp.get(), L.pci.get(), p_vals<PV>(L), L.pvec};
     spmv<PV, X>(ctx, P, lvt<X>(h, l), lvr<X>(h, l + 1), false);
@@ -190,31 +194,36 @@ void vcycle(afp_amg* h, X* x0, const X* r0, bool zero_init) {
     const X* r = l == 0 ? r0 : lvr<X>(h, l);
     CSRView<PV> T{L.n, L.trp.get(), L.tci.get(), pt_vals<PV>(L), L.tvec};
     spmv<PV, X>(ctx, T, lvx<X>(h, l + 1), x, true);
-    smooth<X>(h, l, x, r, h->opts.symmetric != 0);
+    smooth<X>(h, l, x, r, h->opts.symmetric != 0, false);
   }
 }
 
 // Mixed-precision V-cycle as the launch chain: FP32 levels, P / P^T in BF16
 // or FP32 (opts.interp_bf16).
 void vcycle_mixed(afp_amg* h, float* x0, const float* r0) {
-  if (h->opts.interp_bf16) vcycle<float, __nv_bfloat16>(h, x0, r0, true);
-  else vcycle<float, float>(h, x0, r0, true);
+  if (h->opts.interp_bf16) vcycle<float, __nv_bfloat16>(h, x0, r0);
+  else vcycle<float, float>(h, x0, r0);
 }
 
-// z = V(r) on the solver's level-0 buffers (FP64 in and out): the streamed
-// kernel when its plan exists (it converts r and z itself), else the chain.
+// Whether the V-cycle leaves its result in z32 and takes r from r32 (the
+// mixed-precision chain), rather than in z and from r (FP64, and the streamed
+// kernel, which converts both itself).
+bool fp32_level0(const afp_amg* h) { return h->opts.precision == AFP_PRECISION_MIXED && !h->fused; }
+
+// z = V(r) on the solver's level-0 buffers as fp32_level0 says.
 void vcycle_level0(afp_amg* h) {
-  afp_context* ctx = h->ctx;
+  if (h->opts.precision != AFP_PRECISION_MIXED) vcycle<double, double>(h, h->z.get(), h->r.get());
+  else if (h->fused) fused_vcycle(h, h->r.get(), h->z.get());
+  else vcycle_mixed(h, h->z32.get(), h->r32.get());
+}
+
+// The same, FP64 in (r) and out (z) in any case.
+void vcycle_level0_fp64(afp_amg* h) {
   const int64_t n = h->lv[0].n;
-  if (h->opts.precision != AFP_PRECISION_MIXED) {
-    vcycle<double, double>(h, h->z.get(), h->r.get(), true);
-  } else if (h->fused) {
-    fused_vcycle(h, h->r.get(), h->z.get());
-  } else {
-    convert<double, float>(ctx, n, h->r.get(), h->r32.get());
-    vcycle_mixed(h, h->z32.get(), h->r32.get());
-    convert<float, double>(ctx, n, h->z32.get(), h->z.get());
-  }
+  const bool conv = fp32_level0(h);
+  if (conv) convert<double, float>(h->ctx, n, h->r.get(), h->r32.get());
+  vcycle_level0(h);
+  if (conv) convert<float, double>(h->ctx, n, h->z32.get(), h->z.get());
 }
 
 // Runs a graph build; if it fails while the streamed V-cycle is in use (a
@@ -257,7 +266,7 @@ void precondition(afp_amg* h) {
       const int64_t before = ctx->launches.n;
       AFP_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
       try {
-        vcycle_level0(h);
+        vcycle_level0_fp64(h);
       } catch (...) {
         cudaStreamEndCapture(ctx->stream, &g);
         if (g) cudaGraphDestroy(g);
@@ -660,34 +669,19 @@ void check_finite(double v, const char* what) {
 
 // ------------------------------------------------------------------------
 // CG as one CUDA graph: the first iteration, then a conditional WHILE node
-// whose body is a whole iteration (V-cycle included); a one-thread kernel at
-// the end of each iteration sets the loop condition from r.r, so the host
-// synchronises once per solve instead of once per iteration.
+// whose body is a whole iteration (V-cycle included); its last kernel sets the
+// loop condition from r.r, so the host synchronises once per solve instead of
+// once per iteration.
 // Device scalars: s[0] rz, s[1] p.q, s[2] r.r, s[3] rz', s[4] b.b,
-// s[6] tol^2 b.b; loopvars = [iterations done, limit].
-__global__ void k_pcg_check(const double* __restrict__ s, int* __restrict__ it, cudaGraphConditionalHandle handle) {
-  pdl_wait();
-  const int k = ++it[0];
-  const double rr = s[2];
-  const bool cont = (rr > s[6]) && (k < it[1]) && isfinite(rr);
-  cudaGraphSetConditional(handle, cont ? 1u : 0u);
-}
-
-__global__ void k_copy_scalar(double* s, int from, int to) {
-  pdl_wait();
-  s[to] = s[from];
-}
-
-// z = M r on the solver's level-0 buffers, launched into the current capture
-void precondition_inline(afp_amg* h) { vcycle_level0(h); }
-
-void pcg_iteration_tail(afp_amg* h, double* s, cudaGraphConditionalHandle handle) {
+// s[6] tol^2 b.b; loopvars = [iterations done, limit].  Each iteration ends in
+// cg_update_xr, which sets the loop condition and writes the next V-cycle's
+// FP32 right-hand side; the V-cycle's FP32 result is used as it is.
+void pcg_iteration_tail(afp_amg* h, double* s, int num, cudaGraphConditionalHandle handle) {
   afp_context* ctx = h->ctx;
   const Level& L0 = h->lv[0];
   spmv_dot(ctx, L0.A<double>(), h->p.get(), h->q.get(), s + 1);
-  cg_update_xr(ctx, L0.n, s, 0, 1, h->x.get(), h->r.get(), h->p.get(), h->q.get(), s + 2);
-  launch_pdl(ctx->stream, 1, 1, 0, k_pcg_check, (const double*)s, h->loopvars.get(), handle);
-  check_launch(ctx, "cg check");
+  cg_update_xr(ctx, L0.n, s, num, h->x.get(), h->r.get(), h->p.get(), h->q.get(),
+               fp32_level0(h) ? h->r32.get() : nullptr, h->loopvars.get(), handle);
 }
 
 cudaGraphExec_t& loop_graph(afp_amg* h) {
@@ -696,6 +690,7 @@ cudaGraphExec_t& loop_graph(afp_amg* h) {
   cudaGraphExec_t& exec = pi ? h->loop32 : h->loop64;
   if (exec != nullptr) return exec;
   const int64_t n = h->lv[0].n;
+  const bool fp32 = fp32_level0(h);
   double* s = ctx->d_scalars;
   if (h->loopvars.size() == 0) h->loopvars.alloc(ctx, 2);
   cudaGraph_t g;
@@ -706,10 +701,17 @@ cudaGraphExec_t& loop_graph(afp_amg* h) {
   AFP_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
   try {
-    precondition_inline(h);
-    dot(ctx, n, h->r.get(), h->z.get(), s + 0);
-    AFP_CUDA(cudaMemcpyAsync(h->p.get(), h->z.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-    pcg_iteration_tail(h, s, handle);
+    if (fp32) {
+      convert<double, float>(ctx, n, h->r.get(), h->r32.get());
+      vcycle_level0(h);
+      dot(ctx, n, h->r.get(), h->z32.get(), s + 0);
+      convert<float, double>(ctx, n, h->z32.get(), h->p.get());
+    } else {
+      vcycle_level0(h);
+      dot(ctx, n, h->r.get(), h->z.get(), s + 0);
+      AFP_CUDA(cudaMemcpyAsync(h->p.get(), h->z.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
+    }
+    pcg_iteration_tail(h, s, 0, handle);
     cudaStreamCaptureStatus st;
     cudaGraph_t cg;
     const cudaGraphNode_t* deps = nullptr;
@@ -731,12 +733,15 @@ cudaGraphExec_t& loop_graph(afp_amg* h) {
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   AFP_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   try {
-    precondition_inline(h);
-    dot(ctx, n, h->r.get(), h->z.get(), s + 3);
-    cg_update_p(ctx, n, s, 3, 0, h->z.get(), h->p.get());
-    launch_pdl(ctx->stream, 1, 1, 0, k_copy_scalar, s, 3, 0);
-    check_launch(ctx, "copy scalar");
-    pcg_iteration_tail(h, s, handle);
+    vcycle_level0(h);
+    if (fp32) {
+      dot(ctx, n, h->r.get(), h->z32.get(), s + 3);
+      cg_update_p(ctx, n, s, 3, 0, h->z32.get(), h->p.get());
+    } else {
+      dot(ctx, n, h->r.get(), h->z.get(), s + 3);
+      cg_update_p(ctx, n, s, 3, 0, h->z.get(), h->p.get());
+    }
+    pcg_iteration_tail(h, s, 3, handle);
   } catch (...) {
     cudaStreamEndCapture(ctx->stream, &body);
     cudaGraphDestroy(g);
@@ -805,7 +810,7 @@ void pcg(afp_amg* h, double* x_user, const double* b_user, double tol, int maxit
     int cur = 0, nxt = 3;
     for (it = 1; it <= maxit; ++it) {
       spmv_dot(ctx, A, h->p.get(), h->q.get(), s + 1);
-      cg_update_xr(ctx, n, s, cur, 1, h->x.get(), h->r.get(), h->p.get(), h->q.get(), s + 2);
+      cg_update_xr(ctx, n, s, cur, h->x.get(), h->r.get(), h->p.get(), h->q.get(), nullptr, nullptr, 0);
       double rr;
       copy(ctx, &rr, s + 2, sizeof(double));
       sync(ctx);
@@ -1038,7 +1043,7 @@ afp_status afp_amg_time_kernel(afp_amg* h, int kind, int level, int reps, double
           if (kind == 0) {
             afp_amg_opts keep = h->opts;
             h->opts.smooth_step = 1;
-            smooth<float>(h, level, x, r, false);
+            smooth<float>(h, level, x, r, false, false);
             h->opts = keep;
           } else {
             residual<float>(ctx, L.A<float>(), x, r, L.tmp32.get());
@@ -1049,7 +1054,7 @@ afp_status afp_amg_time_kernel(afp_amg* h, int kind, int level, int reps, double
           if (kind == 0) {
             afp_amg_opts keep = h->opts;
             h->opts.smooth_step = 1;
-            smooth<double>(h, level, x, r, false);
+            smooth<double>(h, level, x, r, false, false);
             h->opts = keep;
           } else {
             residual<double>(ctx, L.A<double>(), x, r, L.tmp.get());
@@ -1058,7 +1063,7 @@ afp_status afp_amg_time_kernel(afp_amg* h, int kind, int level, int reps, double
       } else if (kind == 2) {
         if (mixed && h->fused) fused_vcycle(h, h->r.get(), h->z.get());
         else if (mixed) vcycle_mixed(h, h->z32.get(), h->r32.get());
-        else vcycle<double, double>(h, h->z.get(), h->r.get(), true);
+        else vcycle<double, double>(h, h->z.get(), h->r.get());
       } else {
         spmv<double, double>(ctx, h->lv[0].A<double>(), h->p.get(), h->q.get(), false);
       }

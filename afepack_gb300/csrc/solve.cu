@@ -9,8 +9,6 @@
 //
 // Reductions are deterministic: each block writes a partial sum and the last
 // block to finish adds the partials in block order.
-#include <cstdlib>
-
 #include "df32.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
@@ -18,19 +16,15 @@
 
 namespace afp {
 
-// Lanes per row: the smallest power of two in [4, 32] with at most
-// `entries per lane` of the level's mean row length on each lane.  Four per
-// lane (AFP_ENTRIES_PER_LANE overrides it for tuning) measured fastest on the
-// 64^3 P1 level 0 (15 entries per row, 4 lanes): its FP32 Gauss-Seidel sweep
-// 20 us against 32 us with one entry per lane, the residual 7 us against 19.
+// Lanes per row: the smallest power of two in [4, 32] with at most four
+// entries of the level's mean row on each lane, but 32 only above six on each
+// of 16: rows of 74 entries (the second level of a 3D P1 hierarchy) take 16.
+// CG on the 48^3 P1 hierarchy (rows of 15, 74 and 273 entries) with limits of
+// 4, 6 and this: FP64 22.9, 19.8 and 19.2 ms, mixed 10.0, 9.3 and 9.4; on the
+// P2 100^2 one (11, 21, 54) 30.7, 32.1 and 30.7 ms in FP64.
 int pick_vec(double avg) {
-  static const double epl = [] {
-    const char* e = std::getenv("AFP_ENTRIES_PER_LANE");
-    const double v = e ? std::atof(e) : 0.0;
-    return v > 0.0 ? v : 4.0;
-  }();
   int vec = 4;
-  while (vec < 32 && vec * epl < avg) vec *= 2;
+  while (vec < 32 && vec * (vec < 16 ? 4.0 : 6.0) < avg) vec *= 2;
   return vec;
 }
 
@@ -79,13 +73,13 @@ __device__ __forceinline__ T group_sum(T s) {
 // this overlaps two of the three dependent memory round trips of a row with
 // the predecessor's drain.  The products are summed in the same order as a
 // plain k = begin + lane, begin + lane + VEC, ... loop.
-// Pairs loaded ahead per lane.  FP64 keeps it short: each guarded product
-// of the unrolled loop costs an FP64 instruction slot whether or not the
-// entry exists, and FP64 instruction throughput is what bounds the FP64
-// kernels on this GPU.
+// Pairs loaded ahead per lane: all of a row at pick_vec's lanes, so that after
+// the wait a row is one round of gathers.  (FP64 with one pair ahead left the
+// other entries two dependent loads behind the wait: 2D P1 256^2 15.5 ms a
+// solve against 14.4, P2 100^2 34.5 against 30.7.)
 template <int VEC, class V>
 constexpr int prefetch_depth() {
-  return sizeof(V) == 8 ? (VEC >= 32 ? 2 : 1) : (VEC >= 32 ? 8 : 4);
+  return VEC >= 32 ? 8 : 4;
 }
 
 template <int VEC, class V>
@@ -104,14 +98,16 @@ struct RowAhead {
       v[q] = kk < e ? va[kk] : V(0);
     }
   }
-  template <class A, class X>
-  __device__ __forceinline__ A dot(const int* __restrict__ ci, const V* __restrict__ va,
-                                   const X* __restrict__ x) const {
+  // sum of the row's entries times x, with LIM only of those in columns below lim
+  template <class A, bool LIM, class X>
+  __device__ __forceinline__ A dot(const int* __restrict__ ci, const V* __restrict__ va, const X* __restrict__ x,
+                                   int lim) const {
     A s = 0;
 #pragma unroll
     for (int q = 0; q < PF; ++q)
-      if (k + q * VEC < e) s += val_as<A>(v[q]) * (A)x[c[q]];
-    for (int kk = k + PF * VEC; kk < e; kk += VEC) s += val_as<A>(va[kk]) * (A)x[ci[kk]];
+      if (k + q * VEC < e && (!LIM || c[q] < lim)) s += val_as<A>(v[q]) * (A)x[c[q]];
+    for (int kk = k + PF * VEC; kk < e; kk += VEC)
+      if (!LIM || ci[kk] < lim) s += val_as<A>(va[kk]) * (A)x[ci[kk]];
     return s;
   }
 };
@@ -125,7 +121,7 @@ __global__ void k_spmv(int64_t m, const int* __restrict__ rp, const int* __restr
   RowAhead<VEC, V> row;
   row.load(ci, va, g < m ? rp[g] + lane : 0, g < m ? rp[g + 1] : 0);
   pdl_wait();
-  A s = row.template dot<A>(ci, va, x);
+  A s = row.template dot<A, false>(ci, va, x, 0);
   s = group_sum<VEC>(s);
   if (g < m && lane == 0) y[g] = ADD ? (X)((A)y[g] + s) : (X)s;
 }
@@ -139,12 +135,12 @@ __global__ void k_residual(int64_t m, const int* __restrict__ rp, const int* __r
   RowAhead<VEC, X> row;
   row.load(ci, va, g < m ? rp[g] + lane : 0, g < m ? rp[g + 1] : 0);
   pdl_wait();
-  A s = row.template dot<A>(ci, va, x);
+  A s = row.template dot<A, false>(ci, va, x, 0);
   s = group_sum<VEC>(s);
   if (g < m && lane == 0) out[g] = (X)((A)r[g] - s);
 }
 
-template <int VEC, class X>
+template <int VEC, class X, bool FIRST>
 __global__ void k_gs_class(int64_t r0, int64_t r1, const int* __restrict__ rp, const int* __restrict__ ci,
                            const X* __restrict__ va, X* __restrict__ x, const X* __restrict__ r) {
   using A = typename Acc<X>::type;
@@ -156,12 +152,12 @@ __global__ void k_gs_class(int64_t r0, int64_t r1, const int* __restrict__ rp, c
   RowAhead<VEC, X> ahead;
   ahead.load(ci, va, d + 1 + lane, on ? rp[row + 1] : 0);
   pdl_wait();
-  A s = ahead.template dot<A>(ci, va, (const X*)x);
+  A s = ahead.template dot<A, FIRST>(ci, va, (const X*)x, (int)r0);
   s = group_sum<VEC>(s);
   if (on && lane == 0) x[row] = (X)(((A)r[row] - s) / (A)diag);
 }
 
-template <int VEC, class X>
+template <int VEC, class X, bool FIRST>
 __global__ void k_jacobi_l1(int64_t r0, int64_t r1, const int* __restrict__ rp, const int* __restrict__ ci,
                             const X* __restrict__ va, const X* __restrict__ x, const X* __restrict__ r,
                             const X* __restrict__ d, X* __restrict__ tmp) {
@@ -172,9 +168,12 @@ __global__ void k_jacobi_l1(int64_t r0, int64_t r1, const int* __restrict__ rp, 
   RowAhead<VEC, X> ahead;
   ahead.load(ci, va, on ? rp[row] + lane : 0, on ? rp[row + 1] : 0);
   pdl_wait();
-  A s = ahead.template dot<A>(ci, va, x);
+  A s = ahead.template dot<A, FIRST>(ci, va, x, (int)r0);
   s = group_sum<VEC>(s);
-  if (on && lane == 0) tmp[row - r0] = (X)((A)x[row] + ((A)r[row] - s) / (A)d[row - r0]);
+  if (on && lane == 0) {
+    const A old = FIRST ? A(0) : (A)x[row];
+    tmp[row - r0] = (X)(old + ((A)r[row] - s) / (A)d[row - r0]);
+  }
 }
 
 template <class X>
@@ -184,16 +183,40 @@ __global__ void k_copy_range(int64_t n, const X* __restrict__ src, X* __restrict
   if (i < n) dst[i] = src[i];
 }
 
+// One warp per row; eight products of a lane in flight, the first eight
+// entries loaded ahead of the wait.  FP64: n^2 multiply-adds at 2 a clock and
+// SM (3,725 rows: 23 us) against n^2 * 8 bytes (17 us), so it is bound by the
+// FP64 pipe; two sums per lane keep it fed.
 template <class X>
 __global__ void k_dense_gemv(int64_t n, const X* __restrict__ M, const X* __restrict__ r, X* __restrict__ x) {
-  pdl_wait();
   using A = typename Acc<X>::type;
+  constexpr int U = 8;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x & 31;
-  A s = 0;
-  if (row < n)
-    for (int64_t j = lane; j < n; j += 32) s += (A)M[row * n + j] * (A)r[j];
-  s = group_sum<32>(s);
+  const X* m = M + (row < n ? row * n : 0);
+  X v[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) v[u] = row < n && lane + 32 * u < n ? m[lane + 32 * u] : X(0);
+  pdl_wait();
+  A s0 = 0, s1 = 0;
+  if (row < n) {
+    for (int64_t j = lane; j < n; j += 32 * U) {
+      X w[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) w[u] = j + 32 * u < n ? r[j + 32 * u] : X(0);
+      X next[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) next[u] = j + 32 * (U + u) < n ? m[j + 32 * (U + u)] : X(0);
+#pragma unroll
+      for (int u = 0; u < U; u += 2) {
+        s0 += (A)v[u] * (A)w[u];
+        s1 += (A)v[u + 1] * (A)w[u + 1];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = next[u];
+    }
+  }
+  const A s = group_sum<32>(s0 + s1);
   if (row < n && lane == 0) x[row] = (X)s;
 }
 
@@ -316,8 +339,9 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;  // valid in thread 0
 }
 
-// Partial of this block -> scratch; the last block sums them in order.
-__device__ __forceinline__ void finish_reduction(double partial, double* dst, RedScratch rs) {
+// Partial of this block -> scratch; the last block sums them in order.  True
+// in the last block, whose thread 0 has written *dst.
+__device__ __forceinline__ bool finish_reduction(double partial, double* dst, RedScratch rs) {
   __shared__ bool last;
   if (threadIdx.x == 0) {
     rs.partials[blockIdx.x] = partial;
@@ -332,13 +356,16 @@ __device__ __forceinline__ void finish_reduction(double partial, double* dst, Re
     s = block_sum(s);
     if (threadIdx.x == 0) *dst = s;
   }
+  return last;
 }
 
-__global__ void k_dot(int64_t n, const double* __restrict__ a, const double* __restrict__ b, double* dst,
+template <class Z>
+__global__ void k_dot(int64_t n, const double* __restrict__ a, const Z* __restrict__ b, double* dst,
                       RedScratch rs) {
   pdl_wait();
   double s = 0;
-  for (int64_t i = (int64_t)blockIdx.x * BLK + threadIdx.x; i < n; i += (int64_t)gridDim.x * BLK) s += a[i] * b[i];
+  for (int64_t i = (int64_t)blockIdx.x * BLK + threadIdx.x; i < n; i += (int64_t)gridDim.x * BLK)
+    s += a[i] * (double)b[i];
   s = block_sum(s);
   finish_reduction(s, dst, rs);
 }
@@ -368,28 +395,38 @@ __global__ void k_spmv_dot(int64_t m, const int* __restrict__ rp, const int* __r
   finish_reduction(part, dst, rs);
 }
 
-__global__ void k_cg_update_xr(int64_t n, const double* __restrict__ sc, int num, int den, double* __restrict__ x,
-                               double* __restrict__ r, const double* __restrict__ p, const double* __restrict__ q,
-                               double* dst, RedScratch rs) {
+// See cg_update_xr: the last block to finish also ends the CG iteration, in
+// place of two one-thread kernels.
+__global__ void k_cg_update_xr(int64_t n, double* sc, int num, double* __restrict__ x, double* __restrict__ r,
+                               const double* __restrict__ p, const double* __restrict__ q, float* __restrict__ r32,
+                               RedScratch rs, int* it, cudaGraphConditionalHandle loop) {
   pdl_wait();
-  const double alpha = sc[num] / sc[den];
+  const double rz = sc[num], alpha = rz / sc[1];
   double s = 0;
   for (int64_t i = (int64_t)blockIdx.x * BLK + threadIdx.x; i < n; i += (int64_t)gridDim.x * BLK) {
     x[i] += alpha * p[i];
     const double ri = r[i] - alpha * q[i];
     r[i] = ri;
+    if (r32 != nullptr) r32[i] = (float)ri;
     s += ri * ri;
   }
   s = block_sum(s);
-  finish_reduction(s, dst, rs);
+  if (finish_reduction(s, sc + 2, rs) && it != nullptr && threadIdx.x == 0) {
+    // every block has read sc[num] and sc[1] before it finished
+    sc[0] = rz;
+    const int k = ++it[0];
+    const double rr = sc[2];
+    cudaGraphSetConditional(loop, rr > sc[6] && k < it[1] && isfinite(rr) ? 1u : 0u);
+  }
 }
 
-__global__ void k_cg_update_p(int64_t n, const double* __restrict__ sc, int num, int den, const double* __restrict__ z,
+template <class Z>
+__global__ void k_cg_update_p(int64_t n, const double* __restrict__ sc, int num, int den, const Z* __restrict__ z,
                               double* __restrict__ p) {
   pdl_wait();
   const double beta = sc[num] / sc[den];
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = z[i] + beta * p[i];
+  if (i < n) p[i] = (double)z[i] + beta * p[i];
 }
 
 // ----------------------------------------------------------- setup kernels
@@ -565,6 +602,17 @@ void launch_vec(int vec, F&& f) {
   }
 }
 
+// A row kernel of the chain.  PDL pays while a kernel does not fill the GPU
+// (2D P1 60^2 FP64: 0.99 ms a solve with, 1.04 without); FP64 kernels of more
+// than a block per SM are better off without it, as their successors' loads
+// ahead take slots and issue cycles from them: 256^2 13.6 against 14.3 ms,
+// 3D P1 48^3 17.9 against 19.1.
+template <class X, class K, class... Args>
+void launch_row(const afp_context* ctx, unsigned grid, K kernel, Args... args) {
+  const bool pdl = sizeof(X) == 4 || grid <= (unsigned)ctx->sm_count;
+  launch_pdl_if(pdl, ctx->stream, grid, BLK, 0, kernel, args...);
+}
+
 unsigned red_grid(const afp_context* ctx, int64_t n) {
   int64_t g = (n + BLK - 1) / BLK;
   int64_t cap = std::min<int64_t>(RED_BLOCKS, (int64_t)ctx->sm_count * 2);
@@ -578,8 +626,8 @@ void spmv(const afp_context* ctx, const CSRView<V>& A, const X* x, X* y, bool ad
   launch_vec(A.vec, [&](auto VEC) {
     constexpr int W = decltype(VEC)::value;
     unsigned grid = grid_for(A.m * W, BLK);
-    if (add) launch_pdl(ctx->stream, grid, BLK, 0, k_spmv<W, V, X, true>, A.m, A.rowptr, A.cols, A.vals, x, y);
-    else launch_pdl(ctx->stream, grid, BLK, 0, k_spmv<W, V, X, false>, A.m, A.rowptr, A.cols, A.vals, x, y);
+    if (add) launch_row<X>(ctx, grid, k_spmv<W, V, X, true>, A.m, A.rowptr, A.cols, A.vals, x, y);
+    else launch_row<X>(ctx, grid, k_spmv<W, V, X, false>, A.m, A.rowptr, A.cols, A.vals, x, y);
   });
   check_launch(ctx, "spmv");
 }
@@ -588,31 +636,31 @@ template <class X>
 void residual(const afp_context* ctx, const CSRView<X>& A, const X* x, const X* r, X* out) {
   launch_vec(A.vec, [&](auto VEC) {
     constexpr int W = decltype(VEC)::value;
-    launch_pdl(ctx->stream, grid_for(A.m * W, BLK), BLK, 0, k_residual<W, X>, A.m, A.rowptr, A.cols, A.vals, x, r,
+    launch_row<X>(ctx, grid_for(A.m * W, BLK), k_residual<W, X>, A.m, A.rowptr, A.cols, A.vals, x, r,
                out);
   });
   check_launch(ctx, "residual");
 }
 
 template <class X>
-void gs_class(const afp_context* ctx, const CSRView<X>& A, int64_t r0, int64_t r1, X* x, const X* r) {
+void gs_class(const afp_context* ctx, const CSRView<X>& A, int64_t r0, int64_t r1, X* x, const X* r, bool first) {
   if (r1 <= r0) return;
   launch_vec(A.vec, [&](auto VEC) {
     constexpr int W = decltype(VEC)::value;
-    launch_pdl(ctx->stream, grid_for((r1 - r0) * W, BLK), BLK, 0, k_gs_class<W, X>, r0, r1, A.rowptr, A.cols, A.vals,
-               x, r);
+    launch_row<X>(ctx, grid_for((r1 - r0) * W, BLK), first ? k_gs_class<W, X, true> : k_gs_class<W, X, false>, r0, r1,
+                  A.rowptr, A.cols, A.vals, x, r);
   });
   check_launch(ctx, "gauss-seidel class");
 }
 
 template <class X>
 void jacobi_l1_class(const afp_context* ctx, const CSRView<X>& A, int64_t r0, int64_t r1, X* x, const X* r,
-                     const X* l1diag, X* tmp) {
+                     const X* l1diag, X* tmp, bool first) {
   if (r1 <= r0) return;
   launch_vec(A.vec, [&](auto VEC) {
     constexpr int W = decltype(VEC)::value;
-    launch_pdl(ctx->stream, grid_for((r1 - r0) * W, BLK), BLK, 0, k_jacobi_l1<W, X>, r0, r1, A.rowptr, A.cols,
-               A.vals, (const X*)x, r, l1diag, tmp);
+    launch_row<X>(ctx, grid_for((r1 - r0) * W, BLK), first ? k_jacobi_l1<W, X, true> : k_jacobi_l1<W, X, false>, r0,
+                  r1, A.rowptr, A.cols, A.vals, (const X*)x, r, l1diag, tmp);
   });
   check_launch(ctx, "l1-jacobi class");
   launch_pdl(ctx->stream, grid_for(r1 - r0, BLK), BLK, 0, k_copy_range<X>, r1 - r0, (const X*)tmp, x + r0);
@@ -676,8 +724,10 @@ void fill_zero(const afp_context* ctx, int64_t n, X* x) {
   check_launch(ctx, "zero");
 }
 
-void dot(const afp_context* ctx, int64_t n, const double* a, const double* b, double* dst) {
-  launch_pdl(ctx->stream, red_grid(ctx, n), BLK, 0, k_dot, n, a, b, dst, RedScratch{ctx->d_partials, ctx->d_retire});
+template <class Z>
+void dot(const afp_context* ctx, int64_t n, const double* a, const Z* b, double* dst) {
+  launch_pdl(ctx->stream, red_grid(ctx, n), BLK, 0, k_dot<Z>, n, a, b, dst,
+             RedScratch{ctx->d_partials, ctx->d_retire});
   check_launch(ctx, "dot");
 }
 
@@ -690,15 +740,16 @@ void spmv_dot(const afp_context* ctx, const CSRView<double>& A, const double* p,
   check_launch(ctx, "spmv+dot");
 }
 
-void cg_update_xr(const afp_context* ctx, int64_t n, const double* s, int num, int den, double* x, double* r,
-                  const double* p, const double* q, double* dst) {
-  launch_pdl(ctx->stream, red_grid(ctx, n), BLK, 0, k_cg_update_xr, n, s, num, den, x, r, p, q, dst,
-             RedScratch{ctx->d_partials, ctx->d_retire});
+void cg_update_xr(const afp_context* ctx, int64_t n, double* s, int num, double* x, double* r, const double* p,
+                  const double* q, float* r32, int* it, cudaGraphConditionalHandle loop) {
+  launch_pdl(ctx->stream, red_grid(ctx, n), BLK, 0, k_cg_update_xr, n, s, num, x, r, p, q, r32,
+             RedScratch{ctx->d_partials, ctx->d_retire}, it, loop);
   check_launch(ctx, "cg update x r");
 }
 
-void cg_update_p(const afp_context* ctx, int64_t n, const double* s, int num, int den, const double* z, double* p) {
-  launch_pdl(ctx->stream, grid_for(n, BLK), BLK, 0, k_cg_update_p, n, s, num, den, z, p);
+template <class Z>
+void cg_update_p(const afp_context* ctx, int64_t n, const double* s, int num, int den, const Z* z, double* p) {
+  launch_pdl(ctx->stream, grid_for(n, BLK), BLK, 0, k_cg_update_p<Z>, n, s, num, den, z, p);
   check_launch(ctx, "cg update p");
 }
 
@@ -826,14 +877,18 @@ template void spmv<double, double>(const afp_context*, const CSRView<double>&, c
 template void spmv<float, float>(const afp_context*, const CSRView<float>&, const float*, float*, bool);
 template void spmv<__nv_bfloat16, float>(const afp_context*, const CSRView<__nv_bfloat16>&, const float*, float*,
                                          bool);
-template void residual<double>(const afp_context*, const CSRView<double>&, const double*, const double*, double*);
-template void residual<float>(const afp_context*, const CSRView<float>&, const float*, const float*, float*);
-template void gs_class<double>(const afp_context*, const CSRView<double>&, int64_t, int64_t, double*, const double*);
-template void gs_class<float>(const afp_context*, const CSRView<float>&, int64_t, int64_t, float*, const float*);
-template void jacobi_l1_class<double>(const afp_context*, const CSRView<double>&, int64_t, int64_t, double*,
-                                      const double*, const double*, double*);
-template void jacobi_l1_class<float>(const afp_context*, const CSRView<float>&, int64_t, int64_t, float*,
-                                     const float*, const float*, float*);
+#define AFP_LEVEL_OPS(X)                                                                                           \
+  template void residual<X>(const afp_context*, const CSRView<X>&, const X*, const X*, X*);                        \
+  template void gs_class<X>(const afp_context*, const CSRView<X>&, int64_t, int64_t, X*, const X*, bool);          \
+  template void jacobi_l1_class<X>(const afp_context*, const CSRView<X>&, int64_t, int64_t, X*, const X*,          \
+                                   const X*, X*, bool);
+AFP_LEVEL_OPS(double)
+AFP_LEVEL_OPS(float)
+#undef AFP_LEVEL_OPS
+template void dot<double>(const afp_context*, int64_t, const double*, const double*, double*);
+template void dot<float>(const afp_context*, int64_t, const double*, const float*, double*);
+template void cg_update_p<double>(const afp_context*, int64_t, const double*, int, int, const double*, double*);
+template void cg_update_p<float>(const afp_context*, int64_t, const double*, int, int, const float*, double*);
 template void dense_gemv<double>(const afp_context*, int64_t, const double*, const double*, double*);
 template void dense_gemv<float>(const afp_context*, int64_t, const float*, const float*, float*);
 template void diag_solve<double>(const afp_context*, const CSRView<double>&, const double*, double*);

@@ -3,6 +3,8 @@
 
 #include <cuda_bf16.h>
 
+#include <climits>
+
 #include "common.cuh"
 
 namespace afp {
@@ -29,14 +31,16 @@ void residual(const afp_context* ctx, const CSRView<X>& A, const X* x, const X* 
 
 // One Gauss-Seidel colour class: rows [r0, r1) are mutually uncoupled,
 // x_j = (r_j - sum_{k != j} a_jk x_k) / a_jj with the diagonal stored first.
+// With `first` the iterate is zero from row r0 on (the first forward sweep
+// from zero), and nothing there is read.
 template <class X>
-void gs_class(const afp_context* ctx, const CSRView<X>& A, int64_t r0, int64_t r1, X* x, const X* r);
+void gs_class(const afp_context* ctx, const CSRView<X>& A, int64_t r0, int64_t r1, X* x, const X* r, bool first);
 
 // l1-Jacobi on the overflow class [r0, r1): x_j += (r_j - (A x)_j) / d_j,
 // d_j = a_jj + sum of |a_jk| over the class's other rows; tmp holds r1-r0 values.
 template <class X>
 void jacobi_l1_class(const afp_context* ctx, const CSRView<X>& A, int64_t r0, int64_t r1, X* x, const X* r,
-                     const X* l1diag, X* tmp);
+                     const X* l1diag, X* tmp, bool first);
 
 // x = Ainv r for a dense n x n row-major inverse.
 template <class X>
@@ -68,15 +72,20 @@ void strided_copy(const afp_context* ctx, int64_t n, const double* src, int64_t 
 template <class X>
 void fill_zero(const afp_context* ctx, int64_t n, X* x);
 
-// Deterministic FP64 reductions into dst (device scalar).
-void dot(const afp_context* ctx, int64_t n, const double* a, const double* b, double* dst);
+// Deterministic FP64 reductions into dst (device scalar); Z is double or float.
+template <class Z>
+void dot(const afp_context* ctx, int64_t n, const double* a, const Z* b, double* dst);
 // y = A p and dst = p . y in one pass
 void spmv_dot(const afp_context* ctx, const CSRView<double>& A, const double* p, double* y, double* dst);
-// x += alpha p, r -= alpha q, alpha = s[num] / s[den]; dst = r . r
-void cg_update_xr(const afp_context* ctx, int64_t n, const double* s, int num, int den, double* x, double* r,
-                  const double* p, const double* q, double* dst);
-// p = z + beta p, beta = s[num] / s[den]
-void cg_update_p(const afp_context* ctx, int64_t n, const double* s, int num, int den, const double* z, double* p);
+// x += alpha p, r -= alpha q, alpha = s[num] / s[1]; s[2] = r . r.  With r32,
+// r also goes there in FP32 (the next V-cycle's right-hand side).  With `it`,
+// also the end of a CG iteration in a graph: s[0] = s[num], ++it[0], and the
+// loop goes on while r.r > s[6], it[0] < it[1] and r.r is finite.
+void cg_update_xr(const afp_context* ctx, int64_t n, double* s, int num, double* x, double* r, const double* p,
+                  const double* q, float* r32, int* it, cudaGraphConditionalHandle loop);
+// p = z + beta p, beta = s[num] / s[den]; Z is double or float
+template <class Z>
+void cg_update_p(const afp_context* ctx, int64_t n, const double* s, int num, int den, const Z* z, double* p);
 
 // --------------------------------------------------------- setup helpers
 // Builds B with rows B[i] = A[rperm[i]] and columns mapped through cmap
