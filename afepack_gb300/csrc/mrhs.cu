@@ -89,13 +89,22 @@ __global__ void k_dense_gemm(int64_t n, const X* __restrict__ M, const X* __rest
 // columns, KPL per lane: with VEC, lane l owns the contiguous columns
 // l*KPL .. l*KPL+KPL-1 (k == W*KPL) and gathers them with one vector load;
 // otherwise lane l owns columns l, l + W, ... (W >= k up to 32, scalar
-// loads).  SPL groups share one row, group p taking the row's entries in chunks
-// p, p + SPL, ... of W (long coarse-level rows: enough groups in flight to
+// loads).  spl groups share one row, group p taking the row's entries in chunks
+// p, p + spl, ... of W (long coarse-level rows: enough groups in flight to
 // cover the gather latency).  A chunk's (column, value) pairs are loaded one
-// per lane and broadcast with shuffles; the gathers of the x rows of U = 8
+// per lane and broadcast with shuffles; the gathers of the x rows of U = 4
 // entries are issued before any of their products is summed.  The groups'
 // partial sums meet in shared memory and are added in group order, so the
 // result does not depend on timing.
+//
+// Bound by the latency of the gathers (a 256-byte row of x per entry at
+// k = 64, mostly from L2): at 43% of the warps and a quarter of L2's rate it
+// wants warps, not longer bursts.  Six blocks of 256 threads an SM (at most 42
+// registers) with 4 entries in flight against four blocks (62 registers)
+// with 8: one V-cycle of a 64^3 P1 hierarchy with 64 columns 6.05 against 7.76
+// ms, of a 200^2 one 0.68 against 0.78.  With the fewer groups per row of
+// rows_m, whole fours of entries without bounds and the first sweep's
+// unwritten rows left out: 5.65 ms.
 enum RowOp { RO_SPMM = 0, RO_SPMM_ADD, RO_RES, RO_GS, RO_JAC };
 
 constexpr int ROWS_BLK = 256;
@@ -115,16 +124,20 @@ __device__ __forceinline__ void load_vec(const X* p, X (&v)[KPL]) {
   }
 }
 
-template <int W, int KPL, int SPL, class V, class X, int OP, bool VEC>
-__global__ void __launch_bounds__(ROWS_BLK) k_rows_m(int64_t r0, int64_t r1, const int* __restrict__ rp,
-                                                     const int* __restrict__ ci, const V* __restrict__ va, const X* x,
-                                                     X* y, const X* __restrict__ r, const X* __restrict__ d, int k) {
+// With FIRST (the first sweep from an iterate of zeros) only entries in
+// columns below r0 count: the rows from r0 on have not been written yet.
+template <int W, int KPL, class V, class X, int OP, bool VEC, bool FIRST>
+__global__ void __launch_bounds__(ROWS_BLK, 6) k_rows_m(int64_t r0, int64_t r1, const int* __restrict__ rp,
+                                                        const int* __restrict__ ci, const V* __restrict__ va,
+                                                        const X* x, X* y, const X* __restrict__ r,
+                                                        const X* __restrict__ d, int k, int log_spl) {
   using A = typename AccT<X>::type;
   constexpr int GPB = ROWS_BLK / W;  // groups per block
-  __shared__ A part[SPL > 1 ? GPB : 1][SPL > 1 ? W : 1][KPL];
+  __shared__ A part[GPB][W][KPL];
+  const int spl = 1 << log_spl;
   const int grp = threadIdx.x / W, lane = threadIdx.x & (W - 1);
-  const int64_t row = r0 + (int64_t)blockIdx.x * (GPB / SPL) + grp / SPL;
-  const int pidx = grp % SPL;
+  const int64_t row = r0 + (int64_t)blockIdx.x * (GPB >> log_spl) + (grp >> log_spl);
+  const int pidx = grp & (spl - 1);
   const bool on = row < r1;
   const unsigned mask = W >= 32 ? 0xffffffffu : (((1u << W) - 1u) << ((threadIdx.x & 31) & ~(W - 1)));
   A acc[KPL];
@@ -138,14 +151,14 @@ __global__ void __launch_bounds__(ROWS_BLK) k_rows_m(int64_t r0, int64_t r1, con
       diag = as<A>(va[b]);
       ++b;
     }
-    constexpr int U = 8;
+    constexpr int U = 4;
     if (W == 1) {
-      for (int j0 = b + pidx * U; j0 < e; j0 += SPL * U) {
+      for (int j0 = b + pidx * U; j0 < e; j0 += spl * U) {
         A vals[U];
         X xv[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const bool in = j0 + u < e;
+          const bool in = j0 + u < e && (!FIRST || ci[j0 + u] < r0);
           vals[u] = in ? as<A>(va[j0 + u]) : A(0);
           xv[u] = in ? x[(int64_t)ci[j0 + u] * k] : X(0);
         }
@@ -153,43 +166,49 @@ __global__ void __launch_bounds__(ROWS_BLK) k_rows_m(int64_t r0, int64_t r1, con
         for (int u = 0; u < U; ++u) acc[0] += vals[u] * (A)xv[u];
       }
     } else {
-      for (int base = b + pidx * W; base < e; base += SPL * W) {
+      // U entries from the chunk's position jj on; ALL: all of them exist
+      auto take = [&](int cc, A vv, int jj, int cnt, auto ALLc) {
+        constexpr bool ALL = decltype(ALLc)::value;
+        A vals[U];
+        X xv[U][KPL];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const bool got = ALL || jj + u < cnt;  // the same for the whole group
+          const int col = __shfl_sync(mask, cc, got ? jj + u : 0, W);
+          const A val = __shfl_sync(mask, vv, got ? jj + u : 0, W);
+          const bool in = got && (!FIRST || col < r0);
+          vals[u] = in ? val : A(0);
+          const X* xr = x + (int64_t)col * k;
+          if constexpr (VEC) {
+            if (in) load_vec<KPL>(xr + lane * KPL, xv[u]);
+            else
+#pragma unroll
+              for (int q = 0; q < KPL; ++q) xv[u][q] = X(0);
+          } else {
+#pragma unroll
+            for (int q = 0; q < KPL; ++q) {
+              const int c = lane + W * q;
+              xv[u][q] = (in && c < k) ? xr[c] : X(0);
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int q = 0; q < KPL; ++q) acc[q] += vals[u] * (A)xv[u][q];
+      };
+      for (int base = b + pidx * W; base < e; base += spl * W) {
         const int my = base + lane;
         const int cc = my < e ? ci[my] : 0;
         const A vv = my < e ? as<A>(va[my]) : A(0);
         const int cnt = min(W, e - base);
-        for (int jj = 0; jj < cnt; jj += U) {
-          A vals[U];
-          X xv[U][KPL];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const bool in = jj + u < cnt;  // the same for the whole group
-            const int col = __shfl_sync(mask, cc, in ? jj + u : 0, W);
-            const A val = __shfl_sync(mask, vv, in ? jj + u : 0, W);
-            vals[u] = in ? val : A(0);
-            const X* xr = x + (int64_t)col * k;
-            if constexpr (VEC) {
-              if (in) load_vec<KPL>(xr + lane * KPL, xv[u]);
-              else
-#pragma unroll
-                for (int q = 0; q < KPL; ++q) xv[u][q] = X(0);
-            } else {
-#pragma unroll
-              for (int q = 0; q < KPL; ++q) {
-                const int c = lane + W * q;
-                xv[u][q] = (in && c < k) ? xr[c] : X(0);
-              }
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int q = 0; q < KPL; ++q) acc[q] += vals[u] * (A)xv[u][q];
-        }
+        int jj = 0;
+        for (; jj + U <= cnt; jj += U) take(cc, vv, jj, cnt, std::true_type());
+        if (jj < cnt) take(cc, vv, jj, cnt, std::false_type());
       }
     }
   }
-  if (SPL > 1) {
+  if (spl > 1) {
 #pragma unroll
     for (int q = 0; q < KPL; ++q) part[grp][lane][q] = acc[q];
     __syncthreads();
@@ -197,7 +216,7 @@ __global__ void __launch_bounds__(ROWS_BLK) k_rows_m(int64_t r0, int64_t r1, con
 #pragma unroll
     for (int q = 0; q < KPL; ++q) {
       A s = part[grp][lane][q];
-      for (int p = 1; p < SPL; ++p) s += part[grp + p][lane][q];
+      for (int p = 1; p < spl; ++p) s += part[grp + p][lane][q];
       acc[q] = s;
     }
   }
@@ -211,42 +230,42 @@ __global__ void __launch_bounds__(ROWS_BLK) k_rows_m(int64_t r0, int64_t r1, con
     else if (OP == RO_SPMM_ADD) y[o] = (X)((A)y[o] + acc[q]);
     else if (OP == RO_RES) y[o] = (X)((A)r[o] - acc[q]);
     else if (OP == RO_GS) y[o] = (X)(((A)r[o] - acc[q]) / diag);
-    else y[(row - r0) * k + c] = (X)((A)x[o] + ((A)r[o] - acc[q]) / (A)d[row - r0]);  // RO_JAC into tmp
+    else y[(row - r0) * k + c] = (X)((FIRST ? A(0) : (A)x[o]) + ((A)r[o] - acc[q]) / (A)d[row - r0]);  // RO_JAC into tmp
   }
 }
 
 // Launches k_rows_m with 16-byte vector gathers (KPL = 16 bytes of columns
 // per lane, W = k / KPL lanes) when k allows them and x is aligned, else
 // with W = the smallest power of two >= k (at most 32) and KPL = columns per
-// lane; SPL groups per row for rows of about `row_len` entries (about 48
-// entries per group).
+// lane; a power of two of groups per row for rows of about `row_len` entries.
+// `first`: see k_rows_m's FIRST.
 template <class V, class X, int OP>
 void rows_m(const afp_context* ctx, int64_t r0, int64_t r1, const int* rp, const int* ci, const V* va, const X* x,
-            X* y, const X* r, const X* d, int k, double row_len, const char* what) {
+            X* y, const X* r, const X* d, int k, double row_len, const char* what, bool first = false) {
   if (r1 <= r0) return;
   auto go = [&](auto Wc, auto Kc, auto Vc) {
     constexpr int W = decltype(Wc)::value, KPL = decltype(Kc)::value;
     constexpr bool VEC = decltype(Vc)::value;
-    // groups per row: enough for the row's gathers to overlap (about 48
-    // entries per group), and for short row ranges (small colour classes of
-    // coarse levels) enough lanes to fill about half the GPU
-    int spl = 1;
-    while (spl < 8 && spl * 48 < row_len) spl *= 2;
-    while (spl < 16 && spl * W < row_len && (double)(r1 - r0) * W * spl < 1024.0 * ctx->sm_count) spl *= 2;
-    spl = std::min(spl, ROWS_BLK / W);
-    auto launch = [&](auto Sc) {
-      constexpr int SPL = decltype(Sc)::value;
-      if constexpr (ROWS_BLK / W >= SPL) {  // a block holds whole rows
-        constexpr int rows_per_blk = ROWS_BLK / W / SPL;
-        const unsigned grid = (unsigned)((r1 - r0 + rows_per_blk - 1) / rows_per_blk);
-        k_rows_m<W, KPL, SPL, V, X, OP, VEC><<<grid, ROWS_BLK, 0, ctx->stream>>>(r0, r1, rp, ci, va, x, y, r, d, k);
+    // groups per row: about 96 entries per group (fewer groups spend less on
+    // adding their sums up: 64^3 level 1, 75 entries a row, 246 us a sweep
+    // with one, 275 with two), and for short row ranges (small colour
+    // classes of coarse levels) enough lanes to fill a quarter of the GPU
+    int log_spl = 0;
+    while (log_spl < 3 && (96 << log_spl) < row_len) ++log_spl;
+    while (log_spl < 4 && (W << log_spl) < row_len && (double)(r1 - r0) * (W << log_spl) < 512.0 * ctx->sm_count)
+      ++log_spl;
+    while ((1 << log_spl) > ROWS_BLK / W) --log_spl;  // a block holds whole rows
+    const int rows_per_blk = (ROWS_BLK / W) >> log_spl;
+    const unsigned grid = (unsigned)((r1 - r0 + rows_per_blk - 1) / rows_per_blk);
+    if constexpr (OP == RO_GS || OP == RO_JAC) {
+      if (first) {
+        k_rows_m<W, KPL, V, X, OP, VEC, true><<<grid, ROWS_BLK, 0, ctx->stream>>>(r0, r1, rp, ci, va, x, y, r, d, k,
+                                                                                  log_spl);
+        return;
       }
-    };
-    if (spl == 1) launch(std::integral_constant<int, 1>());
-    else if (spl == 2) launch(std::integral_constant<int, 2>());
-    else if (spl == 4) launch(std::integral_constant<int, 4>());
-    else if (spl == 8) launch(std::integral_constant<int, 8>());
-    else launch(std::integral_constant<int, 16>());
+    }
+    k_rows_m<W, KPL, V, X, OP, VEC, false><<<grid, ROWS_BLK, 0, ctx->stream>>>(r0, r1, rp, ci, va, x, y, r, d, k,
+                                                                               log_spl);
   };
   using I1 = std::integral_constant<int, 1>;
   using I2 = std::integral_constant<int, 2>;
@@ -629,7 +648,7 @@ template <class X, class PV>
 void vcycle_m(afp_amg* h, MultiState& S) {
   const afp_context* ctx = h->ctx;
   const int k = S.k, t = h->t;
-  auto smooth = [&](int l, X* x, const X* r, bool backward) {
+  auto smooth = [&](int l, X* x, const X* r, bool backward, bool from_zero) {
     const Level& L = h->lv[l];
     CSRView<X> A = L.A<X>();
     const double len = (double)L.nnz / (double)L.n;
@@ -644,12 +663,13 @@ void vcycle_m(afp_amg* h, MultiState& S) {
           if constexpr (std::is_same<X, double>::value) d = L.l1d.get();
           else d = L.l1d32.get();
           X* tmp = blk<X>(S, 2, l);
-          rows_m<X, X, RO_JAC>(ctx, r0, r1, A.rowptr, A.cols, A.vals, x, tmp, r, d, k, len, "mrhs l1-jacobi");
+          rows_m<X, X, RO_JAC>(ctx, r0, r1, A.rowptr, A.cols, A.vals, x, tmp, r, d, k, len, "mrhs l1-jacobi",
+                               from_zero && s == 0);
           k_copy<X><<<grid_for((r1 - r0) * k, BLK), BLK, 0, ctx->stream>>>((r1 - r0) * k, tmp, x + r0 * k);
           check_launch(ctx, "mrhs copy");
         } else {
           rows_m<X, X, RO_GS>(ctx, r0, r1, A.rowptr, A.cols, A.vals, x, x, r, nullptr, k, len,
-                              "mrhs gauss-seidel class");
+                              "mrhs gauss-seidel class", from_zero && s == 0);
         }
       }
   };
@@ -657,9 +677,11 @@ void vcycle_m(afp_amg* h, MultiState& S) {
     Level& L = h->lv[l];
     X* x = blk<X>(S, 0, l);
     const X* r = blk<X>(S, 1, l);
-    k_zero_m<X><<<grid_for(L.n * k, BLK), BLK, 0, ctx->stream>>>(L.n * k, x);
-    check_launch(ctx, "mrhs zero");
-    smooth(l, x, r, false);
+    if (h->opts.smooth_step == 0) {
+      k_zero_m<X><<<grid_for(L.n * k, BLK), BLK, 0, ctx->stream>>>(L.n * k, x);
+      check_launch(ctx, "mrhs zero");
+    }
+    smooth(l, x, r, false, true);
     CSRView<X> A = L.A<X>();
     rows_m<X, X, RO_RES>(ctx, 0, L.n, A.rowptr, A.cols, A.vals, x, blk<X>(S, 2, l), r, nullptr, k,
                          (double)L.nnz / L.n, "mrhs residual");
@@ -699,7 +721,7 @@ void vcycle_m(afp_amg* h, MultiState& S) {
     Level& L = h->lv[l];
     rows_m<PV, X, RO_SPMM_ADD>(ctx, 0, L.n, L.trp.get(), L.tci.get(), pt_vals<PV>(L), blk<X>(S, 0, l + 1),
                                blk<X>(S, 0, l), nullptr, nullptr, k, (double)L.pnnz / L.n, "mrhs prolongation");
-    smooth(l, blk<X>(S, 0, l), blk<X>(S, 1, l), h->opts.symmetric != 0);
+    smooth(l, blk<X>(S, 0, l), blk<X>(S, 1, l), h->opts.symmetric != 0, false);
   }
 }
 
