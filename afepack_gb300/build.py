@@ -28,6 +28,7 @@ SOURCES = [
     ("coarsen.cu", ["-fmad=false"]),
     ("solve.cu", []),
     ("spd_inverse.cu", []),
+    ("tail_product.cu", []),
     ("amg.cu", []),
     ("mrhs.cu", []),
     ("vcycle_stream.cu", []),
@@ -35,7 +36,8 @@ SOURCES = [
     ("coarsen_host.cpp", []),
     ("server.cpp", []),
 ]
-HEADERS = ["common.cuh", "kernels.cuh", "solve.cuh", "amg_internal.cuh", "launch.cuh", "quadrature_tables.h"]
+HEADERS = ["common.cuh", "kernels.cuh", "solve.cuh", "amg_internal.cuh", "launch.cuh", "df32.cuh", "digits.cuh",
+           "tail_product.cuh", "quadrature_tables.h"]
 
 
 def _nvcc() -> str:

@@ -659,6 +659,7 @@ void lazy_reinit(afp_amg* h, afp_matrix* A) {
   if (h->loop32) cudaGraphExecDestroy(h->loop32);
   h->graph64 = h->graph32 = h->loop64 = h->loop32 = nullptr;
   h->multi.reset();
+  h->tail_digits.reset();
   h->lv.clear();
   build_solve_layout(h, built, A);
 }

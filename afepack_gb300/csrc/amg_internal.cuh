@@ -5,6 +5,7 @@
 
 #include "kernels.cuh"
 #include "solve.cuh"
+#include "tail_product.cuh"
 
 namespace afp {
 
@@ -68,10 +69,9 @@ struct MultiState {
   std::vector<DevBuf<double>> X, R, T;      // per level, n_l x k (FP64 V-cycle)
   std::vector<DevBuf<float>> X32, R32, T32; // per level, n_l x k (FP32 V-cycle)
   DevBuf<double> B, Xs, Rs, Z, P, Q, Tmp;   // level-0 CG blocks, n x k
-  DevBuf<double> scal;                      // column scalars, 8 x k
+  DevBuf<double> scal;                      // column scalars, 8 x k (row 5: error word of the tail product)
   DevBuf<int> active;                       // k flags
-  DevBuf<float2> tail_part;                 // split-inner-dimension partial pairs of the dense tail
-  int tail_split = 1;
+  std::unique_ptr<TailWork> tail;           // set when the dense tail is a digit product
   cudaGraphExec_t graph = nullptr;
   int64_t graph_nodes = 0;
   ~MultiState() {
@@ -175,6 +175,7 @@ struct afp_amg {
   afp::DevBuf<double> tail_inv;           // FP64 dense inverse (FP64 precision)
   afp::DevBuf<float> tail_hi, tail_lo;    // the same as an FP32 pair hi + lo (mixed precision)
   int64_t tail_ld = 0;                    // row stride of hi / lo (a multiple of 4 floats)
+  std::unique_ptr<afp::TailDigits> tail_digits;  // the inverse's digits, made by the first batched solve
   // solver vectors (level-0 solve order)
   afp::DevBuf<double> b, x, r, z, p, q, tmp;
   afp::DevBuf<float> r32, z32;

@@ -12,20 +12,12 @@
 //
 // FP64 arithmetic runs at 2 multiply-adds a clock and SM here, so the n^3
 // part of a 6,744-row inverse is at least 0.25 s in FP64 even with symmetry.
-// The two products of a panel are therefore formed from exact pieces on the
-// tensor cores (Ozaki, Ogita, Oishi, Rump, Numer. Algorithms 59, 2012): every
-// row is scaled by a power of two and cut into kS = 9 signed digits of 7 bits
-// (|d| <= 64; the cut rounds at 2^-63 of the row's scale), digit i stored
-// times 2^-7i in BF16, which holds it exactly.  In units of their weight a
-// product of two digits is at most 2^12 and a sum over kB = 256 inner indices
-// and up to 8 digit pairs of one weight at most 2^23, so the FP32
-// accumulators of the weights 0..7 are exact.  Weight 8 shares the last
-// accumulator (its rounding is 2^-24 of weight 7); the pairs below are left
-// out.  An entry's eight sums are put together in 64-bit integers and FP64.
-// On grid matrices of 576 rows with coefficients of contrast 1, 1e4 and 1e8
-// the inverse is as far from an extended-precision one as the same sweep with
-// FP64 products: 2.2e-15, 8e-14 and 2e-11 of its norm on either side; with
-// 8 digits the small entries of the last two were 40 and more times worse.
+// The two products of a panel are therefore formed from kS = 9 digits of 7
+// bits (digits.cuh).  On grid matrices of 576 rows with coefficients of
+// contrast 1, 1e4 and 1e8 the inverse is as far from an extended-precision one
+// as the same sweep with FP64 products: 2.2e-15, 8e-14 and 2e-11 of its norm
+// on either side; with 8 digits the small entries of the last two were 40 and
+// more times worse.
 //
 // Measured (GB300, whole inverse): 6,744 rows 35 ms against 706 ms with the
 // pivoted FP64 sweep of solve.cu (two launches per pivot, FP64 products);
@@ -37,6 +29,7 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "digits.cuh"
 #include "launch.cuh"
 #include "solve.cuh"
 
@@ -46,7 +39,6 @@ namespace {
 constexpr int kB = 256;         // panel width
 constexpr int kS = 9;           // digits per number
 constexpr int kAcc = 8;         // accumulators of an output tile
-constexpr int kKC = 32;         // inner indices per pipeline stage
 constexpr int kNK = kB / kKC;   // stages of one product
 constexpr int kTM = 128, kTN = 64;  // output tile of a block: kAcc accumulators of kTN columns fill tensor memory
 constexpr int kSub = 16;        // pivots per step of the panel's own inverse
@@ -170,47 +162,6 @@ __global__ void __launch_bounds__(128) k_spd_sweep(int kk, const double* __restr
 }
 
 // --------------------------------------------------------------- the digits
-// Digit arrays: [stage kc][digit][8-row group][octet of kKC][8 rows][8
-// inner], BF16: any run of row groups of one stage and digit is contiguous in
-// the core-matrix order the tensor cores read (8 rows x 16 bytes, next octet
-// 128 bytes on, next row group 512 bytes on), so a tile is one bulk copy.
-__device__ __forceinline__ size_t digit_offset(int64_t groups, int kc, int s, int64_t row, int octet) {
-  return ((((size_t)kc * kS + s) * groups + row / 8) * (kKC / 8) + octet) * 64 + (row % 8) * 8;
-}
-
-// One warp cuts one row: lane l holds inner indices 8 l .. 8 l + 7.
-__device__ __forceinline__ void cut_row(const double (&v)[8], int lane, int64_t groups, int64_t row,
-                                        __nv_bfloat16* __restrict__ dig, double* __restrict__ scale) {
-  double mx = 0.0;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) mx = fmax(mx, fabs(v[e]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  // 2^ex > mx, from the exponent bits; a row below 2^-900 counts as zeros
-  const int ex = min(900, max(-900, (int)((__double2hiint(mx) >> 20) & 0x7ff) - 1022));
-  const double up = __hiloint2double((1023 + 7 * kS - 1 - ex) << 20, 0);
-  long long w[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) w[e] = __double2ll_rn(v[e] * up);
-#pragma unroll
-  for (int s = kS - 1; s >= 0; --s) {
-    __align__(16) __nv_bfloat16 d[8];
-    const float unit = __int_as_float((127 - 7 * s) << 23);  // 2^-7s
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      long long g = w[e];
-      if (s > 0) {
-        g = ((w[e] + 64) & 127) - 64;
-        w[e] = (w[e] - g) >> 7;
-      }
-      d[e] = __float2bfloat16_rn((float)(int)g * unit);
-    }
-    *reinterpret_cast<uint4*>(dig + digit_offset(groups, lane / 4, s, row, lane % 4)) =
-        *reinterpret_cast<const uint4*>(d);
-  }
-  if (lane == 0) *scale = __hiloint2double((1023 + ex) << 20, 0);
-}
-
 // C of the panel [k0, k0 + pb) cut into digits; a block takes one 8-row group.
 // Rows below the panel read their own columns, rows above it the panel's rows
 // transposed, the panel's rows and the padding are zeros.
@@ -221,7 +172,7 @@ __global__ void __launch_bounds__(256) k_spd_cut_panel(int64_t n, int64_t k0, in
   const int64_t i0 = (int64_t)blockIdx.x * 8;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t row = i0 + w;
-  double v[8];
+  double v[1][8];
   if (i0 < k0) {  // k0 is a multiple of 8: the whole group is above the panel
     const int j = threadIdx.x;
     if (j < pb) {
@@ -233,16 +184,16 @@ __global__ void __launch_bounds__(256) k_spd_cut_panel(int64_t n, int64_t k0, in
     }
     __syncthreads();
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = tile[w][8 * lane + e];
+    for (int e = 0; e < 8; ++e) v[0][e] = tile[w][8 * lane + e];
   } else {
     const bool on = row >= k0 + pb && row < n;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int j = 8 * lane + e;
-      v[e] = (on && j < pb) ? M[row * n + k0 + j] : 0.0;
+      v[0][e] = (on && j < pb) ? M[row * n + k0 + j] : 0.0;
     }
   }
-  cut_row(v, lane, groups, row, dig, scale + row);
+  cut_row<kS>(v, lane, groups, row, 0, dig, scale + row);
 }
 
 // A dense `rows` x kB array cut into digits; with M, its rows also go back
@@ -255,13 +206,13 @@ __global__ void __launch_bounds__(256) k_spd_cut_dense(int64_t n, int64_t k0, in
   const int64_t i0 = (int64_t)blockIdx.x * 8;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t row = i0 + w;
-  double v[8];
+  double v[1][8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) v[e] = Z[row * kB + 8 * lane + e];
-  cut_row(v, lane, groups, row, dig, scale + row);
+  for (int e = 0; e < 8; ++e) v[0][e] = Z[row * kB + 8 * lane + e];
+  cut_row<kS>(v, lane, groups, row, 0, dig, scale + row);
   if (M == nullptr) return;
 #pragma unroll
-  for (int e = 0; e < 8; ++e) tile[w][8 * lane + e] = v[e];
+  for (int e = 0; e < 8; ++e) tile[w][8 * lane + e] = v[0][e];
   __syncthreads();
   const int j = threadIdx.x;
   if (i0 < k0) {
@@ -299,68 +250,6 @@ __global__ void k_spd_mirror(int64_t n, double* __restrict__ M) {
 }
 
 // -------------------------------------------------------- the digit product
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void bar_init(uint64_t* b, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
-}
-// false when the phase does not complete within the bound (seconds at most)
-__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t phase) {
-  for (int it = 0; it < (1 << 22); ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(b)), "r"(phase)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* b) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(smem_u32(b))
-               : "memory");
-}
-// Shared-memory matrix descriptor: no swizzle, K-major, next octet 128 bytes
-// on (leading offset), next 8-row group 512 bytes on (stride offset).
-__device__ __forceinline__ uint64_t mat_desc(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
-         ((uint64_t)1 << 46);
-}
-// FP32 accumulators, both operands BF16 and K-major, kTM x kTN
-constexpr uint32_t kInstr = (1u << 4) | (1u << 7) | (1u << 10) | ((kTN / 8) << 17) | ((kTM / 16) << 24);
-
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-      "l"(a), "l"(b), "r"(kInstr), "r"((uint32_t)accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t* b) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
-  uint32_t r[8];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(addr));
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// an integer below 2^51 as a double: placed in the fraction of 3 * 2^51, which is then taken off
-__device__ __forceinline__ double exact_double(long long v) {
-  return __longlong_as_double(0x4338000000000000LL + v) - 0x1.8p52;
-}
-
 constexpr uint32_t kABytes = kTM * kKC * 2, kBBytes = kTN * kKC * 2;  // one digit's tile of a stage
 constexpr uint32_t kStageBytes = kS * (kABytes + kBBytes);
 constexpr int kStages = 2;
@@ -447,7 +336,7 @@ __global__ void __launch_bounds__(kProdThreads, 1) k_spd_product(const __nv_bflo
 #pragma unroll
           for (int q = 0; q < kKC / 16; ++q)
             mma(tmem + min(i + j, kAcc - 1) * kTN, mat_desc(ab + i * kABytes + q * 256), mat_desc(bb + j * kBBytes + q * 256),
-                kc > 0 || i > 0 || q > 0);
+                instr_desc(kTM, kTN), kc > 0 || i > 0 || q > 0);
       mma_commit(&empty[st]);
     }
     mma_commit(&done);
