@@ -206,16 +206,40 @@ struct Elem {
   static constexpr int ND = DIM == 2 ? 3 * DEG : (DEG == 1 ? 4 : 10);
 };
 
-// Quadrature point l of a triangle: its global point p and the basis values
-// of triangle.{1,2}.bas_fun.c there (lam: barycentric coordinates, P2 only).
+// The quadrature points' template coordinates (the barycentric ones of the
+// template element, from the basis plugins' arithmetic) are the same for every
+// cell: a block computes them once, into shared memory.  Per cell they were a
+// fifth of the quadratic tetrahedra's FP64 operations, eight divisions a point.
+template <int DIM>
+__device__ __forceinline__ void template_coords(const QuadRule& q, double (*tl)[4]) {
+  for (int l = threadIdx.x; l < q.n; l += blockDim.x) {
+    if constexpr (DIM == 2) {
+      const double R[3][2] = {{0.0, 0.0}, {1.0, 0.0}, {0.0, 1.0}};
+      const double larea = area2(R[0], R[1], R[2]);
+      const double lp[2] = {q.p[l][0], q.p[l][1]};
+      tl[l][0] = area2(lp, R[1], R[2]) / larea;
+      tl[l][1] = area2(lp, R[2], R[0]) / larea;
+      tl[l][2] = area2(lp, R[0], R[1]) / larea;
+    } else {
+      const double R[4][3] = {{0.0, 0.0, 0.0}, {1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
+      const double lvol = det6(R[0], R[1], R[2], R[3]) / 6.;
+      const double lp[3] = {q.p[l][0], q.p[l][1], q.p[l][2]};
+      tl[l][0] = det6(lp, R[1], R[2], R[3]) / 6. / lvol;
+      tl[l][1] = det6(R[0], lp, R[2], R[3]) / 6. / lvol;
+      tl[l][2] = det6(R[0], R[1], lp, R[3]) / 6. / lvol;
+      tl[l][3] = det6(R[0], R[1], R[2], lp) / 6. / lvol;
+    }
+  }
+  __syncthreads();
+}
+
+// A quadrature point of a triangle from its template coordinates t: the global
+// point p and the basis values of triangle.{1,2}.bas_fun.c there (lam:
+// barycentric coordinates, P2 only).
 template <int DEG>
-__device__ __forceinline__ void tri_values(const double (&gv)[3][2], double area, const double (&R)[3][2],
-                                           double larea, const QuadRule& q, int l, double (&p)[2], double (&lam)[3],
-                                           double* val) {
-  const double lp[2] = {q.p[l][0], q.p[l][1]};
-  const double l0 = area2(lp, R[1], R[2]) / larea;
-  const double l1 = area2(lp, R[2], R[0]) / larea;
-  const double l2 = area2(lp, R[0], R[1]) / larea;
+__device__ __forceinline__ void tri_values(const double (&gv)[3][2], double area, const double* t, double (&p)[2],
+                                           double (&lam)[3], double* val) {
+  const double l0 = t[0], l1 = t[1], l2 = t[2];
   p[0] = l0 * gv[0][0] + l1 * gv[1][0] + l2 * gv[2][0];
   p[1] = l0 * gv[0][1] + l1 * gv[1][1] + l2 * gv[2][1];
   if constexpr (DEG == 1) {
@@ -236,14 +260,9 @@ __device__ __forceinline__ void tri_values(const double (&gv)[3][2], double area
 
 // the same for a tetrahedron (tetrahedron.{1,2}.bas_fun.c); vol = det6 of the cell
 template <int DEG>
-__device__ __forceinline__ void tet_values(const double (&v)[4][3], double vol, const double (&R)[4][3], double lvol,
-                                           const QuadRule& q, int l, double (&p)[3], double (&lam)[4],
-                                           double* val) {
-  const double lp[3] = {q.p[l][0], q.p[l][1], q.p[l][2]};
-  const double l0 = det6(lp, R[1], R[2], R[3]) / 6. / lvol;
-  const double l1 = det6(R[0], lp, R[2], R[3]) / 6. / lvol;
-  const double l2 = det6(R[0], R[1], lp, R[3]) / 6. / lvol;
-  const double l3 = det6(R[0], R[1], R[2], lp) / 6. / lvol;
+__device__ __forceinline__ void tet_values(const double (&v)[4][3], double vol, const double* t, double (&p)[3],
+                                           double (&lam)[4], double* val) {
+  const double l0 = t[0], l1 = t[1], l2 = t[2], l3 = t[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) p[d] = l0 * v[0][d] + l1 * v[1][d] + l2 * v[2][d] + l3 * v[3][d];
   lam[0] = det6(p, v[1], v[2], v[3]) / vol;
@@ -266,12 +285,22 @@ __device__ __forceinline__ void tet_values(const double (&v)[4][3], double vol, 
   }
 }
 
-// Element matrix of one cell, reference arithmetic (see file comment).
+// Element matrix of one cell, reference arithmetic (see file comment).  Bound
+// by FP64 operations (2 a clock and SM, multiplications and additions apart
+// since nothing may be contracted).  The stiffness matrix is symmetric bit for
+// bit -- products commute and every entry sums in the same order -- so its
+// upper triangle is computed and both halves are written; a mass entry,
+// (Jxw val_j) val_k, is not.
+// Quadratic tetrahedra, 55,566 cells: stiffness 0.80 ms (1.05 with all 100
+// entries and the template coordinates per cell), mass 0.49 ms (0.61).
 template <int DIM, int DEG, bool MASS>
 __global__ void __launch_bounds__(128) k_element_matrix(const double* __restrict__ coords, const int* __restrict__ cells,
                                                         int64_t n_cell, QuadRule q, const double* __restrict__ coef,
                                                         double* __restrict__ out) {
   constexpr int NV = Elem<DIM, DEG>::NV, ND = Elem<DIM, DEG>::ND;
+  constexpr int NK = MASS ? ND * ND : ND * (ND + 1) / 2;
+  __shared__ double tl[64][4];
+  template_coords<DIM>(q, tl);
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_cell) return;
   double v[4][3] = {{0}};
@@ -281,9 +310,29 @@ __global__ void __launch_bounds__(128) k_element_matrix(const double* __restrict
 #pragma unroll
     for (int d = 0; d < DIM; ++d) v[a][d] = coords[(int64_t)vi * DIM + d];
   }
-  double K[ND * ND];
+  double K[NK];
 #pragma unroll
-  for (int t = 0; t < ND * ND; ++t) K[t] = 0.0;
+  for (int t = 0; t < NK; ++t) K[t] = 0.0;
+  // adds this point's terms
+  auto add = [&](double Jxw, const double* val, const double (*g)[DIM]) {
+    if constexpr (MASS) {
+#pragma unroll
+      for (int j = 0; j < ND; ++j)
+#pragma unroll
+        for (int k = 0; k < ND; ++k) K[j * ND + k] += Jxw * val[j] * val[k];
+    } else {
+      int t = 0;
+#pragma unroll
+      for (int j = 0; j < ND; ++j)
+#pragma unroll
+        for (int k = j; k < ND; ++k, ++t) {
+          double ip = g[j][0] * g[k][0];  // (the reference starts from 0, which changes no sum)
+#pragma unroll
+          for (int d = 1; d < DIM; ++d) ip += g[j][d] * g[k][d];
+          K[t] += Jxw * ip;
+        }
+    }
+  };
 
   if constexpr (DIM == 2) {
     const double R[3][2] = {{0.0, 0.0}, {1.0, 0.0}, {0.0, 1.0}};
@@ -299,7 +348,7 @@ __global__ void __launch_bounds__(128) k_element_matrix(const double* __restrict
     dx[2] = (gv[0][1] - gv[1][1]) / area; dy[2] = (gv[1][0] - gv[0][0]) / area;
     for (int l = 0; l < q.n; ++l) {
       double p[2], lam[3], val[ND], g[ND][2];
-      tri_values<DEG>(gv, area, R, larea, q, l, p, lam, val);
+      tri_values<DEG>(gv, area, tl[l], p, lam, val);
       const double Jxw = q.p[l][2] * jac * tmpl_volume;
       if constexpr (DEG == 1) {
 #pragma unroll
@@ -314,19 +363,7 @@ __global__ void __launch_bounds__(128) k_element_matrix(const double* __restrict
         g[4][0] = 4.0 * (lam[0] * dx[2] + lam[2] * dx[0]); g[4][1] = 4.0 * (lam[0] * dy[2] + lam[2] * dy[0]);
         g[5][0] = 4.0 * (lam[1] * dx[0] + lam[0] * dx[1]); g[5][1] = 4.0 * (lam[1] * dy[0] + lam[0] * dy[1]);
       }
-#pragma unroll
-      for (int j = 0; j < ND; ++j)
-#pragma unroll
-        for (int k = 0; k < ND; ++k) {
-          if constexpr (MASS) {
-            K[j * ND + k] += Jxw * val[j] * val[k];
-          } else {
-            double ip = 0;
-            ip += g[j][0] * g[k][0];
-            ip += g[j][1] * g[k][1];
-            K[j * ND + k] += Jxw * ip;
-          }
-        }
+      add(Jxw, val, g);
     }
   } else {
     const double R[4][3] = {{0.0, 0.0, 0.0}, {1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
@@ -341,7 +378,7 @@ __global__ void __launch_bounds__(128) k_element_matrix(const double* __restrict
       for (int n = 0; n < 3; ++n) gl[m][n] = co_det(v, m, n) / vol;
     for (int l = 0; l < q.n; ++l) {
       double p[3], lam[4], val[ND], g[ND][3];
-      tet_values<DEG>(v, vol, R, lvol, q, l, p, lam, val);
+      tet_values<DEG>(v, vol, tl[l], p, lam, val);
       const double Jxw = q.p[l][3] * jac * tmpl_volume;
       if constexpr (DEG == 1) {
 #pragma unroll
@@ -365,30 +402,27 @@ __global__ void __launch_bounds__(128) k_element_matrix(const double* __restrict
 #pragma unroll
           for (int n = 0; n < 3; ++n) g[4 + t][n] = 4 * (gl[first[t]][n] * lam[la[t]] + gl[second[t]][n] * lam[lb[t]]);
       }
-#pragma unroll
-      for (int j = 0; j < ND; ++j)
-#pragma unroll
-        for (int k = 0; k < ND; ++k) {
-          if constexpr (MASS) {
-            K[j * ND + k] += Jxw * val[j] * val[k];
-          } else {
-            double ip = 0;
-            ip += g[j][0] * g[k][0];
-            ip += g[j][1] * g[k][1];
-            ip += g[j][2] * g[k][2];
-            K[j * ND + k] += Jxw * ip;
-          }
-        }
+      add(Jxw, val, g);
     }
   }
   if (!MASS && coef != nullptr) {
     const double a = coef[e];
 #pragma unroll
-    for (int t = 0; t < ND * ND; ++t) K[t] *= a;
+    for (int t = 0; t < NK; ++t) K[t] *= a;
   }
   double* o = out + e * (ND * ND);
+  if constexpr (MASS) {
 #pragma unroll
-  for (int t = 0; t < ND * ND; ++t) o[t] = K[t];
+    for (int t = 0; t < ND * ND; ++t) o[t] = K[t];
+  } else {
+#pragma unroll
+    for (int j = 0; j < ND; ++j)
+#pragma unroll
+      for (int k = 0; k < ND; ++k) {
+        const int a = j < k ? j : k, b = j < k ? k : j;
+        o[j * ND + k] = K[a * ND - a * (a - 1) / 2 + b - a];
+      }
+  }
 }
 
 // ---------------------------------------------------- L2Discretize
@@ -405,6 +439,8 @@ __global__ void __launch_bounds__(128) k_element_rhs(const double* __restrict__ 
                                                      QuadRule q, const double* __restrict__ data, int n_gauss,
                                                      double* __restrict__ terms, double* __restrict__ points) {
   constexpr int NV = Elem<DIM, DEG>::NV, ND = Elem<DIM, DEG>::ND;
+  __shared__ double tl[64][4];
+  template_coords<DIM>(q, tl);
   const int64_t e = c0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= c1) return;
   double v[4][3] = {{0}};
@@ -423,7 +459,7 @@ __global__ void __launch_bounds__(128) k_element_rhs(const double* __restrict__ 
       const double gv[3][2] = {{v[0][0], v[0][1]}, {v[1][0], v[1][1]}, {v[2][0], v[2][1]}};
       const double garea = area2(gv[0], gv[1], gv[2]);
       double lam[3];
-      tri_values<DEG>(gv, garea, R, larea, q, l, p, lam, val);
+      tri_values<DEG>(gv, garea, tl[l], p, lam, val);
       Jxw = q.p[l][2] * (garea / larea) * tmpl_volume;
     } else {
       const double R[4][3] = {{0.0, 0.0, 0.0}, {1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
@@ -431,7 +467,7 @@ __global__ void __launch_bounds__(128) k_element_rhs(const double* __restrict__ 
       const double tmpl_volume = det6(R[0], R[1], R[2], R[3]) / 6.;
       const double jac = (det6(v[0], v[1], v[2], v[3]) / 6.) / lvol;
       double lam[4];
-      tet_values<DEG>(v, det6(v[0], v[1], v[2], v[3]), R, lvol, q, l, p, lam, val);
+      tet_values<DEG>(v, det6(v[0], v[1], v[2], v[3]), tl[l], p, lam, val);
       Jxw = q.p[l][3] * jac * tmpl_volume;
     }
     const int64_t ql = (e - c0) * q.n + l;
@@ -505,12 +541,15 @@ __device__ __forceinline__ void warp_bitonic_sort(int* buf, int P, int lane) {
 }
 
 // One warp per row: gather the DOFs of the cells around DOF `row`, sort,
-// de-duplicate.  count pass: row_len[row] = #unique; fill pass: write the
-// row as [row, ascending others].
+// de-duplicate, and write [row, ascending others] to `lists` at
+// inc_ptr[row] * ND, where the row's cells leave room for it; row_len[row] =
+// its length.  k_pattern_pack moves the rows to their places once those are
+// known, so that they are sorted once (quadratic tetrahedra, 21^3 cubes: 165
+// us a time).
 template <int ND>
 __global__ void k_pattern(int64_t n_dof, const int* __restrict__ inc_ptr, const int* __restrict__ inc,
                           const int* __restrict__ elem_dof, int cap, int* __restrict__ row_len,
-                          const int* __restrict__ rowptr, int* __restrict__ cols) {
+                          int* __restrict__ lists) {
   extern __shared__ int sm_pat[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   int* buf = sm_pat + warp * cap;
@@ -528,25 +567,32 @@ __global__ void k_pattern(int64_t n_dof, const int* __restrict__ inc_ptr, const 
     }
     __syncwarp();
     warp_bitonic_sort(buf, P, lane);
-    if (rowptr == nullptr) {
-      int cnt = 0;
-      for (int t = lane; t < S; t += 32) cnt += (t == 0 || buf[t] != buf[t - 1]);
-      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-      if (lane == 0) row_len[row] = cnt;
-    } else {
-      int* out = cols + rowptr[row];
-      if (lane == 0) out[0] = (int)row;
-      int base = 1;
-      for (int t0 = 0; t0 < S; t0 += 32) {
-        int t = t0 + lane;
-        bool keep = t < S && (t == 0 || buf[t] != buf[t - 1]) && buf[t] != (int)row;
-        unsigned mask = __ballot_sync(0xffffffffu, keep);
-        if (keep) out[base + __popc(mask & ((1u << lane) - 1u))] = buf[t];
-        base += __popc(mask);
-      }
+    int* out = lists + (int64_t)b * ND;
+    int base = 1;
+    for (int t0 = 0; t0 < S; t0 += 32) {
+      int t = t0 + lane;
+      bool keep = t < S && (t == 0 || buf[t] != buf[t - 1]) && buf[t] != (int)row;
+      unsigned mask = __ballot_sync(0xffffffffu, keep);
+      if (keep) out[base + __popc(mask & ((1u << lane) - 1u))] = buf[t];
+      base += __popc(mask);
+    }
+    if (lane == 0) {
+      if (S > 0) out[0] = (int)row;
+      row_len[row] = S > 0 ? base : 0;
     }
     __syncwarp();
   }
+}
+
+// cols[rowptr[i] ...] = row i's list; 8 lanes a row
+template <int ND>
+__global__ void k_pattern_pack(int64_t n_dof, const int* __restrict__ inc_ptr, const int* __restrict__ lists,
+                               const int* __restrict__ rowptr, int* __restrict__ cols) {
+  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 8;
+  if (row >= n_dof) return;
+  const int* in = lists + (int64_t)inc_ptr[row] * ND;
+  const int b = rowptr[row], len = rowptr[row + 1] - b;
+  for (int t = threadIdx.x & 7; t < len; t += 8) cols[b + t] = in[t];
 }
 
 // One warp per row: add the element matrices' rows into the CSR row in
@@ -711,16 +757,16 @@ void build_pattern_nd(const afp_space* sp, Pattern& pat) {
   AFP_REQUIRE(smem <= 200 * 1024, AFP_ERR_UNSUPPORTED, "a DOF touches too many cells for the pattern kernel");
   allow_smem(k_pattern<ND>);
   unsigned grid = (unsigned)std::min<int64_t>((sp->n_dof + wpb - 1) / wpb, (int64_t)ctx->sm_count * 32);
-  DevBuf<int> row_len(ctx, sp->n_dof);
+  DevBuf<int> row_len(ctx, sp->n_dof), lists(ctx, (size_t)sp->n_cell * ND * ND);
   k_pattern<ND><<<grid, wpb * 32, smem, ctx->stream>>>(sp->n_dof, sp->inc_ptr.get(), sp->inc.get(), sp->elem_dof.get(),
-                                                       cap, row_len.get(), nullptr, nullptr);
-  check_launch(ctx, "pattern count");
+                                                       cap, row_len.get(), lists.get());
+  check_launch(ctx, "pattern rows");
   pat.m = pat.n = sp->n_dof;
   pat.rowptr.alloc(ctx, sp->n_dof + 1);
   pat.nnz = exclusive_scan(ctx, row_len.get(), pat.rowptr.get(), sp->n_dof);
   pat.cols.alloc(ctx, pat.nnz);
-  k_pattern<ND><<<grid, wpb * 32, smem, ctx->stream>>>(sp->n_dof, sp->inc_ptr.get(), sp->inc.get(), sp->elem_dof.get(),
-                                                       cap, nullptr, pat.rowptr.get(), pat.cols.get());
+  k_pattern_pack<ND><<<grid_for(sp->n_dof * 8, BLOCK), BLOCK, 0, ctx->stream>>>(
+      sp->n_dof, sp->inc_ptr.get(), lists.get(), pat.rowptr.get(), pat.cols.get());
   check_launch(ctx, "pattern fill");
 }
 
@@ -992,14 +1038,15 @@ afp_status afp_assemble(afp_space* sp, const afp_assemble_opts* opts, afp_matrix
       coef.alloc(ctx, sp->n_cell);
       coef.upload(opts->coef, sp->n_cell);
     }
+    // the pattern first: its row lists are gone before the element matrices come
+    auto pat = std::make_shared<Pattern>();
+    build_pattern(sp, *pat);
     DevBuf<double> eK(ctx, esz), eM;
     element_matrices(sp, opts->acc_stiff, opts->coef ? coef.get() : nullptr, false, eK.get());
     if (mass) {
       eM.alloc(ctx, esz);
       element_matrices(sp, opts->acc_mass, nullptr, true, eM.get());
     }
-    auto pat = std::make_shared<Pattern>();
-    build_pattern(sp, *pat);
     auto K = std::make_unique<afp_matrix>();
     K->ctx = ctx;
     K->pat = pat;
