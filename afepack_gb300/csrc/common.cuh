@@ -171,6 +171,8 @@ void allow_smem(K kernel) {
 // Host <-> device copy of any pointer pair (unified addressing).
 void copy(const afp_context* ctx, void* dst, const void* src, size_t bytes);
 void sync(const afp_context* ctx);
+// Whether a kernel can read and write the caller's array in place.
+bool device_array(const afp_context* ctx, const void* p, size_t bytes);
 // Raises AFP_ERR_CUDA if a kernel launch failed.
 void check_launch(const afp_context* ctx, const char* what);
 

@@ -126,6 +126,35 @@ int64_t exclusive_scan(const afp_context* ctx, const int* counts, int* out, int6
   return total;
 }
 
+// ------------------------------------------------------- callers' arrays
+// Whether [p, p + bytes) can be used by a kernel where it is: an 8-byte
+// aligned range inside one device allocation of the context's GPU, which is
+// what a copy would check.  (The range query is a driver call, looked up once.)
+bool device_array(const afp_context* ctx, const void* p, size_t bytes) {
+  if (reinterpret_cast<uintptr_t>(p) % sizeof(double) != 0) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != ctx->device) return false;
+  using RangeFn = int (*)(unsigned long long*, size_t*, unsigned long long);
+  static const RangeFn range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult got;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &got) != cudaSuccess ||
+        got != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<RangeFn>(f);
+  }();
+  unsigned long long base = 0;
+  size_t size = 0;
+  const unsigned long long q = reinterpret_cast<unsigned long long>(p);
+  return range != nullptr && range(&base, &size, q) == 0 && q >= base && q + bytes <= base + size;
+}
+
 }  // namespace afp
 
 using namespace afp;
@@ -279,10 +308,20 @@ afp_status afp_matrix_vmult(afp_matrix* a, const double* x, double* y) {
     AFP_REQUIRE(a && x && y, AFP_ERR_INVALID, "null argument");
     afp_context* ctx = a->ctx;
     bind(ctx);
-    DevBuf<double> dx(ctx, a->pat->n), dy(ctx, a->pat->m);
-    dx.upload(x, a->pat->n);
-    csr_spmv(ctx, a->pat->m, a->pat->rowptr.get(), a->pat->cols.get(), a->vals.get(), dx.get(), dy.get());
-    dy.download(y, a->pat->m);
+    const int64_t n = a->pat->n, m = a->pat->m;
+    // device arrays are used where they are: two allocations and two copies less
+    // (625 rows: 30 us a call against 40); in-place and overlapping calls are
+    // staged, as the product must not be seen by its own gathers
+    const bool apart = (const char*)(x + n) <= (const char*)y || (const char*)(y + m) <= (const char*)x;
+    if (apart && device_array(ctx, x, sizeof(double) * n) && device_array(ctx, y, sizeof(double) * m)) {
+      csr_spmv(ctx, m, a->pat->rowptr.get(), a->pat->cols.get(), a->vals.get(), x, y);
+      sync(ctx);
+      return;
+    }
+    DevBuf<double> dx(ctx, n), dy(ctx, m);
+    dx.upload(x, n);
+    csr_spmv(ctx, m, a->pat->rowptr.get(), a->pat->cols.get(), a->vals.get(), dx.get(), dy.get());
+    dy.download(y, m);
     sync(ctx);
   });
 }
