@@ -16,14 +16,16 @@
 
 namespace afp {
 
-// Lanes per row: the smallest power of two in [4, 32] with at most four
+// Lanes per row: the smallest power of two in [2, 32] with at most four
 // entries of the level's mean row on each lane, but 32 only above six on each
 // of 16: rows of 74 entries (the second level of a 3D P1 hierarchy) take 16.
 // CG on the 48^3 P1 hierarchy (rows of 15, 74 and 273 entries) with limits of
 // 4, 6 and this: FP64 22.9, 19.8 and 19.2 ms, mixed 10.0, 9.3 and 9.4; on the
-// P2 100^2 one (11, 21, 54) 30.7, 32.1 and 30.7 ms in FP64.
+// P2 100^2 one (11, 21, 54) 30.7, 32.1 and 30.7 ms in FP64.  Two lanes for the
+// rows of 7 of a 2D P1 level instead of four: 256^2 FP64 12.8 against 13.7 ms,
+// mixed 9.9 against 10.6; one lane gains nothing more.
 int pick_vec(double avg) {
-  int vec = 4;
+  int vec = 2;
   while (vec < 32 && vec * (vec < 16 ? 4.0 : 6.0) < avg) vec *= 2;
   return vec;
 }
@@ -595,6 +597,7 @@ __global__ void k_zero_cols(int64_t rows, int64_t cols, double* __restrict__ M, 
 template <class F>
 void launch_vec(int vec, F&& f) {
   switch (vec) {
+    case 2: f(std::integral_constant<int, 2>()); break;
     case 4: f(std::integral_constant<int, 4>()); break;
     case 8: f(std::integral_constant<int, 8>()); break;
     case 16: f(std::integral_constant<int, 16>()); break;
