@@ -75,13 +75,16 @@ __device__ __forceinline__ T group_sum(T s) {
 // this overlaps two of the three dependent memory round trips of a row with
 // the predecessor's drain.  The products are summed in the same order as a
 // plain k = begin + lane, begin + lane + VEC, ... loop.
-// Pairs loaded ahead per lane: all of a row at pick_vec's lanes, so that after
-// the wait a row is one round of gathers.  (FP64 with one pair ahead left the
-// other entries two dependent loads behind the wait: 2D P1 256^2 15.5 ms a
-// solve against 14.4, P2 100^2 34.5 against 30.7.)
+// Pairs loaded ahead per lane: most rows whole at pick_vec's lanes, so that
+// after the wait a row is one round of gathers.  (FP64 with one pair ahead left
+// the other entries two dependent loads behind the wait: 2D P1 256^2 15.5 ms a
+// solve against 14.4, P2 100^2 34.5 against 30.7.)  FP32 takes one or two more
+// for the rows above the mean, P2 100^2 mixed 18.6 ms against 20.3, 3D P1 32^3
+// 2.98 against 3.26; in FP64 their registers cost what they gain.
 template <int VEC, class V>
 constexpr int prefetch_depth() {
-  return VEC >= 32 ? 8 : 4;
+  if (sizeof(V) == 8) return VEC >= 32 ? 8 : 4;
+  return VEC >= 32 ? 10 : VEC >= 16 ? 6 : VEC >= 4 ? 5 : 4;
 }
 
 template <int VEC, class V>
@@ -233,36 +236,64 @@ __global__ void k_split_df(int64_t n, int64_t ld, const double* __restrict__ in,
   lo[t] = __double2float_rn(d - (double)h);
 }
 
-// One warp per row; each lane walks the row with stride 32 (coalesced loads of
-// hi and lo), accumulating a double-float pair; the pairs are merged across
-// the warp with TwoSum.
+// One warp per row, four consecutive columns of hi, lo and r per lane and load
+// (rows of the pair are padded to a multiple of 4 and 16-byte aligned; its
+// padding is zeros), four such loads in flight and the next four ahead, so
+// that the row streams while the double-float sums run; the lanes' pairs are
+// merged across the warp with TwoSum.  r is read by entries: it is small, and
+// not padded.  Bound by the pair's bytes (3,115 rows: 77 MB).  CG on the 48^3
+// P1 hierarchy 8.8 ms; with four 4-byte loads of each in flight 9.3, on the
+// 256^2 one 8.7 against 9.9.
+struct PairAhead {
+  float4 h[4], l[4];
+  __device__ __forceinline__ void load(const float* __restrict__ hi, const float* __restrict__ lo, int64_t j,
+                                       int64_t ld) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t c = j + 128 * u;
+      const bool on = c < ld;
+      h[u] = on ? *reinterpret_cast<const float4*>(hi + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      l[u] = on ? *reinterpret_cast<const float4*>(lo + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+};
+
 __global__ void k_dense_gemv_df(int64_t n, int64_t ld, const float* __restrict__ hi, const float* __restrict__ lo,
                                 const float* __restrict__ r, float* __restrict__ x) {
-  pdl_wait();
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x & 31;
+  const float* h = hi + (row < n ? row * ld : 0);
+  const float* l = lo + (row < n ? row * ld : 0);
+  PairAhead cur;
+  cur.load(h, l, 4 * lane, ld);
+  pdl_wait();
   if (row >= n) return;  // whole warps leave together
-  const float* h = hi + row * ld;
-  const float* l = lo + row * ld;
-  float sh = 0.f, sl = 0.f;
-  int64_t j = lane;
-  for (; j + 96 < n; j += 128) {
-    const float h0 = h[j], h1 = h[j + 32], h2 = h[j + 64], h3 = h[j + 96];
-    const float l0 = l[j], l1 = l[j + 32], l2 = l[j + 64], l3 = l[j + 96];
-    const float v0 = r[j], v1 = r[j + 32], v2 = r[j + 64], v3 = r[j + 96];
-    df_add_prod(sh, sl, h0, l0, v0);
-    df_add_prod(sh, sl, h1, l1, v1);
-    df_add_prod(sh, sl, h2, l2, v2);
-    df_add_prod(sh, sl, h3, l3, v3);
+  float sh[2] = {0.f, 0.f}, sl[2] = {0.f, 0.f};
+  for (int64_t j = 4 * lane; j < ld; j += 512) {
+    float v[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[u][e] = j + 128 * u + e < n ? r[j + 128 * u + e] : 0.f;
+    PairAhead next;
+    next.load(h, l, j + 512, ld);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float hh[4] = {cur.h[u].x, cur.h[u].y, cur.h[u].z, cur.h[u].w};
+      const float ll[4] = {cur.l[u].x, cur.l[u].y, cur.l[u].z, cur.l[u].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) df_add_prod(sh[u & 1], sl[u & 1], hh[e], ll[e], v[u][e]);
+    }
+    cur = next;
   }
-  for (; j < n; j += 32) df_add_prod(sh, sl, h[j], l[j], r[j]);
+  df_add(sh[0], sl[0], sh[1], sl[1]);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
-    const float oh = __shfl_xor_sync(0xffffffffu, sh, off);
-    const float ol = __shfl_xor_sync(0xffffffffu, sl, off);
-    df_add(sh, sl, oh, ol);
+    const float oh = __shfl_xor_sync(0xffffffffu, sh[0], off);
+    const float ol = __shfl_xor_sync(0xffffffffu, sl[0], off);
+    df_add(sh[0], sl[0], oh, ol);
   }
-  if (lane == 0) x[row] = __fadd_rn(sh, sl);
+  if (lane == 0) x[row] = __fadd_rn(sh[0], sl[0]);
 }
 
 template <class X>
@@ -318,7 +349,7 @@ __global__ void k_zero(int64_t n, X* __restrict__ x) {
 }
 
 // ------------------------------------------------------------ reductions
-constexpr int RED_BLOCKS = 512;
+constexpr int RED_BLOCKS = 1024;
 
 // the context's partials array (RED_BLOCKS entries) and retire counter
 struct RedScratch {
@@ -616,9 +647,12 @@ void launch_row(const afp_context* ctx, unsigned grid, K kernel, Args... args) {
   launch_pdl_if(pdl, ctx->stream, grid, BLK, 0, kernel, args...);
 }
 
-unsigned red_grid(const afp_context* ctx, int64_t n) {
+// Blocks of a reduction over n threads' worth of work: per_sm per SM at most.
+// Two for vector sums; six for the A p product, which then goes through the
+// rows of a 48^3 mesh in two rounds of dependent loads instead of six.
+unsigned red_grid(const afp_context* ctx, int64_t n, int per_sm = 2) {
   int64_t g = (n + BLK - 1) / BLK;
-  int64_t cap = std::min<int64_t>(RED_BLOCKS, (int64_t)ctx->sm_count * 2);
+  int64_t cap = std::min<int64_t>(RED_BLOCKS, (int64_t)ctx->sm_count * per_sm);
   return (unsigned)std::max<int64_t>(1, std::min(g, cap));
 }
 
@@ -737,7 +771,7 @@ void dot(const afp_context* ctx, int64_t n, const double* a, const Z* b, double*
 void spmv_dot(const afp_context* ctx, const CSRView<double>& A, const double* p, double* y, double* dst) {
   launch_vec(A.vec, [&](auto VEC) {
     constexpr int W = decltype(VEC)::value;
-    launch_pdl(ctx->stream, red_grid(ctx, A.m * W), BLK, 0, k_spmv_dot<W>, A.m, A.rowptr, A.cols, A.vals, p, y, dst,
+    launch_pdl(ctx->stream, red_grid(ctx, A.m * W, 6), BLK, 0, k_spmv_dot<W>, A.m, A.rowptr, A.cols, A.vals, p, y, dst,
                RedScratch{ctx->d_partials, ctx->d_retire});
   });
   check_launch(ctx, "spmv+dot");
