@@ -596,7 +596,11 @@ __global__ void k_pattern_pack(int64_t n_dof, const int* __restrict__ inc_ptr, c
 }
 
 // One warp per row: add the element matrices' rows into the CSR row in
-// ascending cell order (one cell at a time, one lane per element column).
+// ascending cell order, one lane per element column.  The warp takes 32 / ND
+// cells at a time: their entries are loaded and their places found together
+// (a dependent chain of five loads and a binary search), and only the
+// additions go cell by cell.  Quadratic tetrahedra, 21^3 cubes: 91 us, one cell
+// at a time 137.
 template <int ND>
 __global__ void k_gather_values(int64_t n_dof, const int* __restrict__ inc_ptr, const int* __restrict__ inc,
                                 const int* __restrict__ elem_dof, const int* __restrict__ rowptr,
@@ -604,7 +608,9 @@ __global__ void k_gather_values(int64_t n_dof, const int* __restrict__ inc_ptr, 
                                 const double* __restrict__ eM, double* __restrict__ vK, double* __restrict__ vM,
                                 int rcap) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
+  constexpr int CELLS = 32 / ND;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  const int mine = lane / ND, col = lane % ND;  // the lane's cell of a batch and column in it
   double* accK = reinterpret_cast<double*>(sm_raw) + (size_t)warp * 2 * rcap;
   double* accM = accK + rcap;
   int* ucol = reinterpret_cast<int*>(reinterpret_cast<double*>(sm_raw) + (size_t)wpb * 2 * rcap) + warp * rcap;
@@ -617,13 +623,18 @@ __global__ void k_gather_values(int64_t n_dof, const int* __restrict__ inc_ptr, 
     }
     __syncwarp();
     const int b = inc_ptr[row], e = inc_ptr[row + 1];
-    for (int p = b; p < e; ++p) {
-      const int qd = inc[p];
-      const int64_t c = qd / ND;
-      const int li = qd % ND;
-      if (lane < ND) {
-        const int dof = elem_dof[c * ND + lane];
-        int slot = 0;
+    for (int p = b; p < e; p += CELLS) {
+      int slot = -1;
+      double k = 0.0, m = 0.0;
+      if (mine < CELLS && p + mine < e) {
+        const int qd = inc[p + mine];
+        const int64_t c = qd / ND;
+        const int li = qd % ND;
+        const int64_t src = (c * ND + li) * ND + col;
+        k = eK[src];
+        if (eM != nullptr) m = eM[src];
+        const int dof = elem_dof[c * ND + col];
+        slot = 0;
         if (dof != (int)row) {
           int lo = 1, hi = R;  // first position >= dof in the sorted part
           while (lo < hi) {
@@ -632,11 +643,15 @@ __global__ void k_gather_values(int64_t n_dof, const int* __restrict__ inc_ptr, 
           }
           slot = lo;
         }
-        const int64_t src = (c * ND + li) * ND + lane;
-        accK[slot] += eK[src];
-        if (eM != nullptr) accM[slot] += eM[src];
       }
-      __syncwarp();
+      const int n = min(CELLS, e - p);
+      for (int q = 0; q < n; ++q) {
+        if (mine == q && slot >= 0) {
+          accK[slot] += k;
+          if (eM != nullptr) accM[slot] += m;
+        }
+        __syncwarp();
+      }
     }
     for (int t = lane; t < R; t += 32) {
       vK[r0 + t] = accK[t];
