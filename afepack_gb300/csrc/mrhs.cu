@@ -31,7 +31,7 @@ namespace {
 constexpr int BLK = 256;
 constexpr int WPB = BLK / 32;
 constexpr int MAXK = 64;
-constexpr int RED_GRID = 304;
+constexpr int RED_GRID = 912;  // blocks of a column reduction: six per SM
 
 template <class X>
 struct AccT {
@@ -393,10 +393,40 @@ __global__ void k_rows_scatter(int64_t n, int k, const int* __restrict__ perm, c
 
 // ------------------------------------------------------ column reductions
 // Per-column sums of a.b over n x k blocks; deterministic (block partials,
-// last block adds them in block order).
+// last block adds them in a fixed order).  Lane l owns the columns l and
+// l + 32, or with VEC (an even k above 32) 2 l and 2 l + 1, which it reads as
+// one 16-byte load.
+template <int KPL, bool VEC>
+__device__ __forceinline__ int lane_col(int lane, int q) {
+  return VEC ? lane * KPL + q : lane + 32 * q;
+}
+
+// a row's values of the lane's columns (zeros beyond k)
+template <int KPL, bool VEC>
+__device__ __forceinline__ void row_load(const double* __restrict__ p, int lane, int k, double (&v)[KPL]) {
+  if constexpr (VEC) {
+    const double2 t = 2 * lane < k ? *reinterpret_cast<const double2*>(p + 2 * lane) : make_double2(0.0, 0.0);
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+#pragma unroll
+    for (int q = 0; q < KPL; ++q) v[q] = lane + 32 * q < k ? p[lane + 32 * q] : 0.0;
+  }
+}
+template <int KPL, bool VEC>
+__device__ __forceinline__ void row_store(double* __restrict__ p, int lane, int k, const double (&v)[KPL]) {
+  if constexpr (VEC) {
+    if (2 * lane < k) *reinterpret_cast<double2*>(p + 2 * lane) = make_double2(v[0], v[1]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < KPL; ++q)
+      if (lane + 32 * q < k) p[lane + 32 * q] = v[q];
+  }
+}
+
 // partials: the batch's [RED_GRID x MAXK] scratch, followed in memory by the
 // batch's retire counter (an unsigned in the next double slot)
-template <int KPL>
+template <int KPL, bool VEC>
 __device__ void col_finish(double (&part)[KPL], int k, double* partials, double* dst) {
   unsigned* retire = reinterpret_cast<unsigned*>(partials + (int64_t)RED_GRID * MAXK);
   __shared__ double sm[WPB][MAXK];
@@ -404,7 +434,7 @@ __device__ void col_finish(double (&part)[KPL], int k, double* partials, double*
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < KPL; ++q) {
-    const int c = lane + 32 * q;
+    const int c = lane_col<KPL, VEC>(lane, q);
     if (c < MAXK) sm[w][c] = part[q];
   }
   __syncthreads();
@@ -418,15 +448,22 @@ __device__ void col_finish(double (&part)[KPL], int k, double* partials, double*
   if (threadIdx.x == 0) last = (atomicInc(retire, gridDim.x - 1) == gridDim.x - 1);
   __syncthreads();
   if (last) {
-    for (int c = threadIdx.x; c < k; c += blockDim.x) {
-      double s = 0;
-      for (unsigned b = 0; b < gridDim.x; ++b) s += ((volatile double*)partials)[(int64_t)b * MAXK + c];
+    // four threads a column, each every fourth block; their sums in order
+    constexpr int PARTS = BLK / MAXK;
+    const int c = threadIdx.x % MAXK, h = threadIdx.x / MAXK;
+    double s = 0;
+    if (c < k)
+      for (unsigned b = h; b < gridDim.x; b += PARTS) s += __ldcg(partials + (int64_t)b * MAXK + c);
+    sm[h][c] = s;
+    __syncthreads();
+    if (h == 0 && c < k) {
+      for (int q = 1; q < PARTS; ++q) s += sm[q][c];
       dst[c] = s;
     }
   }
 }
 
-template <int KPL>
+template <int KPL, bool VEC>
 __global__ void k_col_dot(int64_t n, const double* __restrict__ a, const double* __restrict__ b, int k,
                           double* partials, double* dst) {
   const int lane = threadIdx.x & 31;
@@ -434,19 +471,23 @@ __global__ void k_col_dot(int64_t n, const double* __restrict__ a, const double*
 #pragma unroll
   for (int q = 0; q < KPL; ++q) part[q] = 0;
   for (int64_t row = warp_id(); row < n; row += n_warps()) {
+    double va[KPL], vb[KPL];
+    row_load<KPL, VEC>(a + row * k, lane, k, va);
+    row_load<KPL, VEC>(b + row * k, lane, k, vb);
 #pragma unroll
-    for (int q = 0; q < KPL; ++q) {
-      const int c = lane + 32 * q;
-      if (c < k) part[q] += a[row * k + c] * b[row * k + c];
-    }
+    for (int q = 0; q < KPL; ++q) part[q] += va[q] * vb[q];
   }
-  col_finish<KPL>(part, k, partials, dst);
+  col_finish<KPL, VEC>(part, k, partials, dst);
 }
 
-template <int KPL>
-__global__ void k_spmm_dot(int64_t m, const int* __restrict__ rp, const int* __restrict__ ci,
-                           const double* __restrict__ va, const double* __restrict__ p, double* __restrict__ q_out,
-                           int k, double* partials, double* dst) {
+// q = A p and p.q per column, a warp per row.  At 64 columns of a 64^3 mesh
+// 257M multiply-adds, 0.44 ms at the FP64 rate, and 4M gathered rows of 512
+// bytes.
+template <int KPL, bool VEC>
+__global__ void __launch_bounds__(BLK, 4) k_spmm_dot(int64_t m, const int* __restrict__ rp,
+                                                     const int* __restrict__ ci, const double* __restrict__ va,
+                                                     const double* __restrict__ p, double* __restrict__ q_out, int k,
+                                                     double* partials, double* dst) {
   const int lane = threadIdx.x & 31;
   double part[KPL];
 #pragma unroll
@@ -464,7 +505,7 @@ __global__ void k_spmm_dot(int64_t m, const int* __restrict__ rp, const int* __r
       const int cc = my < e ? ci[my] : 0;
       const double vv = my < e ? va[my] : 0.0;
       const int cnt = min(32, e - base);
-      constexpr int U = 8;
+      constexpr int U = 4;
       for (int jj = 0; jj < cnt; jj += U) {
         double vals[U], pv[U][KPL];
 #pragma unroll
@@ -472,36 +513,32 @@ __global__ void k_spmm_dot(int64_t m, const int* __restrict__ rp, const int* __r
           const bool in = jj + u < cnt;  // the same for the whole warp
           const int col = __shfl_sync(0xffffffffu, cc, in ? jj + u : 0);
           vals[u] = __shfl_sync(0xffffffffu, vv, in ? jj + u : 0);
-          const double* pr = p + (int64_t)col * k;
+          if (in) {
+            row_load<KPL, VEC>(p + (int64_t)col * k, lane, k, pv[u]);
+          } else {
 #pragma unroll
-          for (int q = 0; q < KPL; ++q) {
-            const int c = lane + 32 * q;
-            pv[u][q] = (in && c < k) ? pr[c] : 0.0;
+            for (int q = 0; q < KPL; ++q) pv[u][q] = 0.0;
           }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           if (jj + u >= cnt) break;
 #pragma unroll
-          for (int q = 0; q < KPL; ++q)
-            if (lane + 32 * q < k) acc[q] += vals[u] * pv[u][q];
+          for (int q = 0; q < KPL; ++q) acc[q] += vals[u] * pv[u][q];
         }
       }
     }
+    double own[KPL];
+    row_load<KPL, VEC>(p + row * k, lane, k, own);
+    row_store<KPL, VEC>(q_out + row * k, lane, k, acc);
 #pragma unroll
-    for (int q = 0; q < KPL; ++q) {
-      const int c = lane + 32 * q;
-      if (c < k) {
-        q_out[row * k + c] = acc[q];
-        part[q] += acc[q] * p[row * k + c];
-      }
-    }
+    for (int q = 0; q < KPL; ++q) part[q] += acc[q] * own[q];
   }
-  col_finish<KPL>(part, k, partials, dst);
+  col_finish<KPL, VEC>(part, k, partials, dst);
 }
 
 // x += alpha_c p, r -= alpha_c q for active columns; rr_c = r.r
-template <int KPL>
+template <int KPL, bool VEC>
 __global__ void k_update_xr(int64_t n, int k, const double* __restrict__ num, const double* __restrict__ den,
                             const int* __restrict__ active, double* __restrict__ x, double* __restrict__ r,
                             const double* __restrict__ p, const double* __restrict__ q, double* partials,
@@ -510,27 +547,29 @@ __global__ void k_update_xr(int64_t n, int k, const double* __restrict__ num, co
   double alpha[KPL], part[KPL];
 #pragma unroll
   for (int t = 0; t < KPL; ++t) {
-    const int c = lane + 32 * t;
+    const int c = lane_col<KPL, VEC>(lane, t);
     alpha[t] = (c < k && active[c]) ? num[c] / den[c] : 0.0;
     part[t] = 0;
   }
   for (int64_t row = warp_id(); row < n; row += n_warps()) {
+    double vx[KPL], vr[KPL], vp[KPL], vq[KPL];
+    row_load<KPL, VEC>(x + row * k, lane, k, vx);
+    row_load<KPL, VEC>(r + row * k, lane, k, vr);
+    row_load<KPL, VEC>(p + row * k, lane, k, vp);
+    row_load<KPL, VEC>(q + row * k, lane, k, vq);
 #pragma unroll
     for (int t = 0; t < KPL; ++t) {
-      const int c = lane + 32 * t;
-      if (c < k) {
-        const int64_t o = row * k + c;
-        x[o] += alpha[t] * p[o];
-        const double rv = r[o] - alpha[t] * q[o];
-        r[o] = rv;
-        part[t] += rv * rv;
-      }
+      vx[t] += alpha[t] * vp[t];
+      vr[t] -= alpha[t] * vq[t];
+      part[t] += vr[t] * vr[t];
     }
+    row_store<KPL, VEC>(x + row * k, lane, k, vx);
+    row_store<KPL, VEC>(r + row * k, lane, k, vr);
   }
-  col_finish<KPL>(part, k, partials, dst);
+  col_finish<KPL, VEC>(part, k, partials, dst);
 }
 
-template <int KPL>
+template <int KPL, bool VEC>
 __global__ void k_update_p(int64_t n, int k, const double* __restrict__ num, const double* __restrict__ den,
                            const int* __restrict__ active, const double* __restrict__ z, double* __restrict__ p) {
   const int lane = threadIdx.x & 31;
@@ -538,16 +577,18 @@ __global__ void k_update_p(int64_t n, int k, const double* __restrict__ num, con
   bool act[KPL];
 #pragma unroll
   for (int t = 0; t < KPL; ++t) {
-    const int c = lane + 32 * t;
+    const int c = lane_col<KPL, VEC>(lane, t);
     act[t] = c < k && active[c];
     beta[t] = act[t] ? num[c] / den[c] : 0.0;
   }
   for (int64_t row = warp_id(); row < n; row += n_warps()) {
+    double vz[KPL], vp[KPL];
+    row_load<KPL, VEC>(z + row * k, lane, k, vz);
+    row_load<KPL, VEC>(p + row * k, lane, k, vp);
 #pragma unroll
-    for (int t = 0; t < KPL; ++t) {
-      const int c = lane + 32 * t;
-      if (c < k && act[t]) p[row * k + c] = z[row * k + c] + beta[t] * p[row * k + c];
-    }
+    for (int t = 0; t < KPL; ++t)
+      if (act[t]) vp[t] = vz[t] + beta[t] * vp[t];
+    row_store<KPL, VEC>(p + row * k, lane, k, vp);
   }
 }
 
@@ -556,10 +597,12 @@ unsigned rows_grid(const afp_context* ctx, int64_t rows) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * 16));
 }
 
+// f(columns per lane, whether as one 16-byte load)
 template <class F>
 void with_kpl(int k, F&& f) {
-  if (k <= 32) f(std::integral_constant<int, 1>());
-  else f(std::integral_constant<int, 2>());
+  if (k <= 32) f(std::integral_constant<int, 1>(), std::false_type());
+  else if (k % 2 == 0) f(std::integral_constant<int, 2>(), std::true_type());
+  else f(std::integral_constant<int, 2>(), std::false_type());
 }
 
 // ---------------------------------------------------------------- V-cycle
@@ -630,7 +673,7 @@ void vcycle_m(afp_amg* h, MultiState& S) {
     if (S.tail) {
       tail_product<X>(ctx, *h->tail_digits, *S.tail, blk<X>(S, 1, t), blk<X>(S, 0, t), k, tail_error(S));
     } else if constexpr (std::is_same<X, double>::value) {
-      with_kpl(k, [&](auto KPLc) {
+      with_kpl(k, [&](auto KPLc, auto) {
         constexpr int KPL = decltype(KPLc)::value;
         k_dense_gemm<KPL, X><<<rows_grid(ctx, T.n), BLK, 0, ctx->stream>>>(T.n, h->tail_inv.get(), blk<X>(S, 1, t),
                                                                           blk<X>(S, 0, t), k);
@@ -787,11 +830,12 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
   const unsigned rg = std::min<unsigned>(RED_GRID, rows_grid(ctx, n));
   rows_m<double, double, RO_RES>(ctx, 0, n, A.rowptr, A.cols, A.vals, S.Xs.get(), S.Rs.get(), S.B.get(), nullptr, k,
                                  (double)L0.nnz / n, "mrhs residual");
-  with_kpl(k, [&](auto KPLc) {
+  with_kpl(k, [&](auto KPLc, auto VECc) {
     constexpr int KPL = decltype(KPLc)::value;
-    k_col_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, S.B.get(), S.B.get(), k, partials, sc + 4 * MAXK);
+    constexpr bool VEC = decltype(VECc)::value;
+    k_col_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, S.B.get(), S.B.get(), k, partials, sc + 4 * MAXK);
     check_launch(ctx, "mrhs dot");
-    k_col_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Rs.get(), k, partials, sc + 2 * MAXK);
+    k_col_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Rs.get(), k, partials, sc + 2 * MAXK);
     check_launch(ctx, "mrhs dot");
   });
   std::vector<double> hb(k), hr(k), init(k), rel(k);
@@ -813,19 +857,21 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
   if (n_active > 0) {
     precondition_m(h);
     int cur = 0, nxt = 3;
-    with_kpl(k, [&](auto KPLc) {
+    with_kpl(k, [&](auto KPLc, auto VECc) {
       constexpr int KPL = decltype(KPLc)::value;
-      k_col_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Z.get(), k, partials, sc + cur * MAXK);
+      constexpr bool VEC = decltype(VECc)::value;
+      k_col_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Z.get(), k, partials, sc + cur * MAXK);
       check_launch(ctx, "mrhs dot");
     });
     AFP_CUDA(cudaMemcpyAsync(S.P.get(), S.Z.get(), sizeof(double) * nk, cudaMemcpyDeviceToDevice, ctx->stream));
     for (it = 1; it <= maxit; ++it) {
-      with_kpl(k, [&](auto KPLc) {
+      with_kpl(k, [&](auto KPLc, auto VECc) {
         constexpr int KPL = decltype(KPLc)::value;
-        k_spmm_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, A.rowptr, A.cols, A.vals, S.P.get(), S.Q.get(), k, partials,
+        constexpr bool VEC = decltype(VECc)::value;
+        k_spmm_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, A.rowptr, A.cols, A.vals, S.P.get(), S.Q.get(), k, partials,
                                                      sc + 1 * MAXK);
         check_launch(ctx, "mrhs spmm+dot");
-        k_update_xr<KPL><<<rg, BLK, 0, ctx->stream>>>(n, k, sc + cur * MAXK, sc + 1 * MAXK, S.active.get(),
+        k_update_xr<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, k, sc + cur * MAXK, sc + 1 * MAXK, S.active.get(),
                                                       S.Xs.get(), S.Rs.get(), S.P.get(), S.Q.get(), partials,
                                                       sc + 2 * MAXK);
         check_launch(ctx, "mrhs update x r");
@@ -844,11 +890,12 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
       if (n_active == 0) break;
       S.active.upload(act.data(), k);
       precondition_m(h);
-      with_kpl(k, [&](auto KPLc) {
+      with_kpl(k, [&](auto KPLc, auto VECc) {
         constexpr int KPL = decltype(KPLc)::value;
-        k_col_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Z.get(), k, partials, sc + nxt * MAXK);
+        constexpr bool VEC = decltype(VECc)::value;
+        k_col_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Z.get(), k, partials, sc + nxt * MAXK);
         check_launch(ctx, "mrhs dot");
-        k_update_p<KPL><<<rows_grid(ctx, n), BLK, 0, ctx->stream>>>(n, k, sc + nxt * MAXK, sc + cur * MAXK,
+        k_update_p<KPL, VEC><<<rows_grid(ctx, n), BLK, 0, ctx->stream>>>(n, k, sc + nxt * MAXK, sc + cur * MAXK,
                                                                      S.active.get(), S.Z.get(), S.P.get());
         check_launch(ctx, "mrhs update p");
       });
@@ -1069,25 +1116,27 @@ void batch_driver(afp_batch_server* s) {
           act[c] = 1;
         }
         S.active.upload(act.data(), k);
-        with_kpl(k, [&](auto KPLc) {
+        with_kpl(k, [&](auto KPLc, auto VECc) {
           constexpr int KPL = decltype(KPLc)::value;
-          k_col_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, S.B.get(), S.B.get(), k, partials, sc + 4 * MAXK);
+          constexpr bool VEC = decltype(VECc)::value;
+          k_col_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, S.B.get(), S.B.get(), k, partials, sc + 4 * MAXK);
           check_launch(ctx, "batch b.b");
         });
       }
       // ---- one CG iteration over every column (free ones are masked)
       precondition_m(h);  // Z = V(R)
-      with_kpl(k, [&](auto KPLc) {
+      with_kpl(k, [&](auto KPLc, auto VECc) {
         constexpr int KPL = decltype(KPLc)::value;
-        k_col_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Z.get(), k, partials, sc + 3 * MAXK);
+        constexpr bool VEC = decltype(VECc)::value;
+        k_col_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Z.get(), k, partials, sc + 3 * MAXK);
         check_launch(ctx, "batch r.z");
-        k_update_p<KPL><<<rows_grid(ctx, n), BLK, 0, ctx->stream>>>(n, k, sc + 3 * MAXK, sc, S.active.get(),
+        k_update_p<KPL, VEC><<<rows_grid(ctx, n), BLK, 0, ctx->stream>>>(n, k, sc + 3 * MAXK, sc, S.active.get(),
                                                                      S.Z.get(), S.P.get());
         check_launch(ctx, "batch p");
-        k_spmm_dot<KPL><<<rg, BLK, 0, ctx->stream>>>(n, A.rowptr, A.cols, A.vals, S.P.get(), S.Q.get(), k, partials,
+        k_spmm_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, A.rowptr, A.cols, A.vals, S.P.get(), S.Q.get(), k, partials,
                                                      sc + 1 * MAXK);
         check_launch(ctx, "batch A p");
-        k_update_xr<KPL><<<rg, BLK, 0, ctx->stream>>>(n, k, sc + 3 * MAXK, sc + 1 * MAXK, S.active.get(), S.Xs.get(),
+        k_update_xr<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, k, sc + 3 * MAXK, sc + 1 * MAXK, S.active.get(), S.Xs.get(),
                                                       S.Rs.get(), S.P.get(), S.Q.get(), partials, sc + 2 * MAXK);
         check_launch(ctx, "batch x r");
       });
