@@ -99,12 +99,12 @@ __global__ void k_dense_gemm(int64_t n, const X* __restrict__ M, const X* __rest
 //
 // Bound by the latency of the gathers (a 256-byte row of x per entry at
 // k = 64, mostly from L2): at 43% of the warps and a quarter of L2's rate it
-// wants warps, not longer bursts.  Six blocks of 256 threads an SM (at most 42
-// registers) with 4 entries in flight against four blocks (62 registers)
-// with 8: one V-cycle of a 64^3 P1 hierarchy with 64 columns 6.05 against 7.76
-// ms, of a 200^2 one 0.68 against 0.78.  With the fewer groups per row of
-// rows_m, whole fours of entries without bounds and the first sweep's
-// unwritten rows left out: 5.65 ms.
+// wanted more chunks under way, not longer bursts.  One V-cycle of a 64^3 P1
+// hierarchy with 64 columns took 7.76 ms with 8 entries in flight and nothing
+// ahead, 6.05 with 4 entries and six blocks an SM, 5.65 with fewer groups per
+// row (rows_m); the tail aside, loading the next chunk ahead at four blocks (64
+// registers) is another 0.15 ms less than six blocks without.  The l1-Jacobi
+// class of a 48^3 second level now runs at 76% of L1's throughput.
 enum RowOp { RO_SPMM = 0, RO_SPMM_ADD, RO_RES, RO_GS, RO_JAC };
 
 constexpr int ROWS_BLK = 256;
@@ -127,7 +127,7 @@ __device__ __forceinline__ void load_vec(const X* p, X (&v)[KPL]) {
 // With FIRST (the first sweep from an iterate of zeros) only entries in
 // columns below r0 count: the rows from r0 on have not been written yet.
 template <int W, int KPL, class V, class X, int OP, bool VEC, bool FIRST>
-__global__ void __launch_bounds__(ROWS_BLK, 6) k_rows_m(int64_t r0, int64_t r1, const int* __restrict__ rp,
+__global__ void __launch_bounds__(ROWS_BLK, 4) k_rows_m(int64_t r0, int64_t r1, const int* __restrict__ rp,
                                                         const int* __restrict__ ci, const V* __restrict__ va,
                                                         const X* x, X* y, const X* __restrict__ r,
                                                         const X* __restrict__ d, int k, int log_spl) {
@@ -166,17 +166,17 @@ __global__ void __launch_bounds__(ROWS_BLK, 6) k_rows_m(int64_t r0, int64_t r1, 
         for (int u = 0; u < U; ++u) acc[0] += vals[u] * (A)xv[u];
       }
     } else {
-      // U entries from the chunk's position jj on; ALL: all of them exist
-      auto take = [&](int cc, A vv, int jj, int cnt, auto ALLc) {
+      // entries src[u] of the chunk, those with got[u] (the same for the whole
+      // group; ALL: all of them)
+      auto take = [&](int cc, A vv, const int (&src)[U], const bool (&got)[U], auto ALLc) {
         constexpr bool ALL = decltype(ALLc)::value;
         A vals[U];
         X xv[U][KPL];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const bool got = ALL || jj + u < cnt;  // the same for the whole group
-          const int col = __shfl_sync(mask, cc, got ? jj + u : 0, W);
-          const A val = __shfl_sync(mask, vv, got ? jj + u : 0, W);
-          const bool in = got && (!FIRST || col < r0);
+          const bool in = ALL || got[u];
+          const int col = __shfl_sync(mask, cc, src[u], W);
+          const A val = __shfl_sync(mask, vv, src[u], W);
           vals[u] = in ? val : A(0);
           const X* xr = x + (int64_t)col * k;
           if constexpr (VEC) {
@@ -197,14 +197,47 @@ __global__ void __launch_bounds__(ROWS_BLK, 6) k_rows_m(int64_t r0, int64_t r1, 
 #pragma unroll
           for (int q = 0; q < KPL; ++q) acc[q] += vals[u] * (A)xv[u][q];
       };
-      for (int base = b + pidx * W; base < e; base += spl * W) {
-        const int my = base + lane;
-        const int cc = my < e ? ci[my] : 0;
-        const A vv = my < e ? as<A>(va[my]) : A(0);
+      // the next chunk's pairs are loaded before this one's are used
+      int base = b + pidx * W;
+      int cc = base + lane < e ? ci[base + lane] : 0;
+      A vv = base + lane < e ? as<A>(va[base + lane]) : A(0);
+      while (base < e) {
         const int cnt = min(W, e - base);
-        int jj = 0;
-        for (; jj + U <= cnt; jj += U) take(cc, vv, jj, cnt, std::true_type());
-        if (jj < cnt) take(cc, vv, jj, cnt, std::false_type());
+        base += spl * W;
+        const int ncc = base + lane < e ? ci[base + lane] : 0;
+        const A nvv = base + lane < e ? as<A>(va[base + lane]) : A(0);
+        int src[U];
+        bool got[U];
+        if constexpr (FIRST) {  // the chunk's entries below r0, from lane to lane
+          unsigned keep = __ballot_sync(mask, lane < cnt && cc < r0);
+          if (W < 32) keep = (keep >> ((threadIdx.x & 31) & ~(W - 1))) & ((1u << (W & 31)) - 1u);
+          while (keep) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              got[u] = keep != 0;
+              src[u] = got[u] ? __ffs(keep) - 1 : 0;
+              keep &= keep - 1;
+            }
+            take(cc, vv, src, got, std::false_type());
+          }
+        } else {
+          int jj = 0;
+          for (; jj + U <= cnt; jj += U) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) src[u] = jj + u;
+            take(cc, vv, src, got, std::true_type());
+          }
+          if (jj < cnt) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              got[u] = jj + u < cnt;
+              src[u] = got[u] ? jj + u : 0;
+            }
+            take(cc, vv, src, got, std::false_type());
+          }
+        }
+        cc = ncc;
+        vv = nvv;
       }
     }
   }
