@@ -80,11 +80,13 @@ __device__ __forceinline__ T group_sum(T s) {
 // the other entries two dependent loads behind the wait: 2D P1 256^2 15.5 ms a
 // solve against 14.4, P2 100^2 34.5 against 30.7.)  FP32 takes one or two more
 // for the rows above the mean, P2 100^2 mixed 18.6 ms against 20.3, 3D P1 32^3
-// 2.98 against 3.26; in FP64 their registers cost what they gain.
+// 2.98 against 3.26; in FP64, and at 32 lanes (10 pairs: P2 20^3 mixed 16.8 ms
+// against 16.1, 3D P1 64^3 14.75 against 14.55), their registers cost what they gain.
 template <int VEC, class V>
 constexpr int prefetch_depth() {
-  if (sizeof(V) == 8) return VEC >= 32 ? 8 : 4;
-  return VEC >= 32 ? 10 : VEC >= 16 ? 6 : VEC >= 4 ? 5 : 4;
+  if (VEC >= 32) return 8;
+  if (sizeof(V) == 8) return 4;
+  return VEC >= 16 ? 6 : VEC >= 4 ? 5 : 4;
 }
 
 template <int VEC, class V>
