@@ -399,12 +399,12 @@ __device__ __forceinline__ int find_slot(const int* c, int R, int key, int row) 
 // G lanes per coarse row, 32 / G rows side by side in a warp: FP64
 // instructions cost a warp 16 clocks however few lanes use them, so lanes
 // idle past the end of short P^T rows (4 entries on the finest level, 13 on
-// the next) are what this pass would otherwise wait for: 25 ms for the
+// the next) are what this pass would otherwise wait for: 19 ms for the
 // 31,833-row product of a 64^3 hierarchy and 1.5 ms for the 139,878-row one; a
 // warp per row with one product in flight and a binary search each took 70
-// and 6 ms.  The warp's groups run in lockstep: each takes the next up to G pairs (a, b) of its row, one
-// per lane, then all go through them U at a time -- columns and weights of U
-// rows of P^T loaded, their slots found and products formed, and only then
+// and 6 ms.  The warp's groups run in lockstep: each takes the next up to G
+// pairs (a, b) of its row, one per lane, then all go through them U at a time
+// -- columns and weights of U rows of P^T loaded, their slots found and products formed, and only then
 // added one row of P^T after the other.
 // A column's slot is its rank in the row: with RANK a bitmap over the row's
 // column window with the words' prefix counts (two shared loads; window <=
@@ -687,8 +687,12 @@ void galerkin_product(const afp_context* ctx, int64_t n_c, int64_t n_f, const in
   const int rmax = extent.first, window = extent.second;
   AFP_REQUIRE(rmax <= (BLOCK_CAP * 3) / 4, AFP_ERR_UNSUPPORTED,
               "Galerkin product row longer than the block-level table");
-  // Lanes per coarse row: the power of two that holds a mean row of P^T.  A
-  // slot is found by rank where the row windows' bitmaps fit 12 KB a group
+  // Lanes per coarse row.  Few where rows of P^T are short: mean 3.4 entries
+  // 0.42, 0.49 and 0.59 ms with 8, 16 and 32 lanes (2D P2 121^2), 4.3 2.4, 2.3
+  // and 3.4 (64^3), 5.8 0.92, 0.82 and 0.94, 6.8 2.8, 2.3 and 2.6 (3D P2 20^3).
+  // Long rows of the product take a warp: their accumulators and bitmaps in
+  // shared memory bound the groups of an SM (285 entries a row, mean 13: 27 ms
+  // with 32 lanes, 33 with 16, 46 with 8; both phases).  A slot is found by rank where the row windows' bitmaps fit 12 KB a group
   // (64K columns; 0.3 KB for the lattice numbering of a 64^3 mesh), else by
   // binary search.  A group's accumulator is the longest row; blocks of 4, 2
   // or 1 warps, so that two blocks fit an SM, and wider groups if not even
@@ -708,7 +712,7 @@ void galerkin_product(const afp_context* ctx, int64_t n_c, int64_t n_f, const in
   const size_t gb = ((size_t)acc_cap * sizeof(double) + search_bytes + 15) / 16 * 16;
   const bool gacc = gb > NUM_SMEM_MAX;
   const size_t group_bytes = gacc ? (rank ? (search_bytes + 15) / 16 * 16 : 16) : gb;
-  int G = mean <= 8.0 ? 8 : mean <= 16.0 ? 16 : 32;
+  int G = mean <= 5.0 ? 8 : mean <= 16.0 && out.nnz <= 200 * n_c ? 16 : 32;
   while (G < 32 && (size_t)(32 / G) * group_bytes > NUM_SMEM_MAX / 2) G *= 2;
   if (gacc) G = 32;
   int warps = 4;
