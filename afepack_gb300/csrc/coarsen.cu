@@ -119,9 +119,10 @@ __device__ __forceinline__ void push_rows(bool push, int i, int* list, int* coun
 // that changed it, C by the decrement that reached zero (a row held by a C
 // point never gets there, since that point does not count down).  The lists
 // and counts are read past the L1 cache, and the cluster barrier orders a
-// step's writes before the next step's reads.  G lanes take a row: a step is
-// a chain of dependent loads, so short rows go four to a warp.
-template <int G>
+// step's writes before the next step's reads.  A warp takes a row, short ones
+// too: a step waits for its longest row (35,237 rows of 14 entries: the whole
+// splitting 1.94 ms, with 8 lanes a row 2.52; only on steps of thousands of
+// rows do 8 lanes gain, 274,625 rows of 15: 3.60 and 3.33).
 __global__ void __launch_bounds__(kWaveThreads) k_cf_pass1_wave(int m, const int* __restrict__ rp,
                                                                 const int* __restrict__ ci,
                                                                 const double* __restrict__ va,
@@ -146,13 +147,13 @@ __global__ void __launch_bounds__(kWaveThreads) k_cf_pass1_wave(int m, const int
     int* next = list + (size_t)((step + 1) & 1) * m;
     int* ncount = counts + (step + 1) % 3;
     if (tid == 0) counts[(step + 2) % 3] = 0;
-    for (int w = warp * (32 / G); w < n; w += nw * (32 / G)) {
-      const int at = w + lane / G;
-      const int j = at < n ? __ldcg(cur + at) : -1;
-      const bool is_c = j >= 0 && __ldcg(st + j) == -1;
-      const double bj = j >= 0 ? beta[j] : 0.0;
-      const int e1 = j >= 0 ? rp[j + 1] : 0;
-      for (int e = j >= 0 ? rp[j] + 1 + lane % G : 0; __any_sync(0xffffffffu, e < e1); e += G) {
+    for (int w = warp; w < n; w += nw) {
+      const int j = __ldcg(cur + w);
+      const bool is_c = __ldcg(st + j) == -1;
+      const double bj = beta[j];
+      const int e1 = rp[j + 1];
+      for (int e0 = rp[j] + 1; e0 < e1; e0 += 32) {
+        const int e = e0 + lane;
         const int i = e < e1 ? ci[e] : -1;
         bool push = false;
         if (i > j && strong(va[e], bj)) {
@@ -532,7 +533,10 @@ __global__ void k_cf_weights(int m, const int* __restrict__ rp, const int* __res
 // chunk are passed round in order.  Rows of P^T longer than kPtCap accumulate
 // and search in global memory.
 constexpr int kPtCap = 256;
-constexpr double kWarpWeightsLen = 24.0;  // mean row length above which a warp takes a row
+// Mean row length above which a warp takes a row: of 131 entries the whole
+// splitting 2.7 ms against 10 (18,476 rows of a 3D P2 20^3 hierarchy);
+// of 7 to 15 a thread each 3.33 against 3.67 (64^3), 2.14 against 2.27 (48^3).
+constexpr double kWarpWeightsLen = 24.0;
 
 // acc + the values v of the lanes in `which`, added in lane order
 __device__ __forceinline__ double add_in_order(double acc, double v, unsigned which) {
@@ -711,8 +715,8 @@ int gpu_project(const afp_context* ctx, int64_t m64, const int* rp, const int* c
   waves.zero();
   k_cf_count_in<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), cnt.get());
   const double len = (double)nnz / (double)m;  // mean row
-  launch_wave(ctx, "C/F pass 1", 0, len <= 24.0 ? k_cf_pass1_wave<8> : k_cf_pass1_wave<32>, m, rp, ci, va,
-              (const double*)beta.get(), st1.get(), cnt.get(), list.get(), waves.get(), waves.get() + 6);
+  launch_wave(ctx, "C/F pass 1", 0, k_cf_pass1_wave, m, rp, ci, va, (const double*)beta.get(), st1.get(), cnt.get(),
+              list.get(), waves.get(), waves.get() + 6);
   k_cf_pass2_candidates<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), st1.get(), s2.get());
   k_cf_pass2_count<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), s2.get(), cnt.get());
   launch_wave(ctx, "C/F pass 2", kWaveThreads / 32 * kSet * sizeof(int), k_cf_pass2_wave, m, rp, ci, va, (const double*)beta.get(), (const int*)st1.get(),
