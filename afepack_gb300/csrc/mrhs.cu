@@ -2,7 +2,7 @@
 // and hierarchy, all advanced by the same launches.
 //
 // Blocks are n x k row-major (the k values of one DOF are contiguous).  Every
-// row kernel gives a matrix row to one warp whose lanes own the columns: a
+// row kernel gives a matrix row to a group of lanes that own the columns: a
 // stored entry a_ij is read once and applied to all k columns of row j of the
 // block, a 128/256-byte coalesced segment.  Relative to k single solves the
 // matrix traffic drops k-fold and the arithmetic per matrix byte grows k-fold.
@@ -650,8 +650,13 @@ float* blk<float>(MultiState& S, int which, int l) {
   return (which == 0 ? S.X32 : which == 1 ? S.R32 : S.T32)[l].get();
 }
 
-// Rows from which the dense tail is a digit product.
-constexpr int64_t kDigitTail = 128;
+// Rows from which the dense tail is a digit product.  CG of 64 columns with a
+// tail of 525 rows: 9.4 ms in mixed precision and 13.4 in FP64, against 10.1 and
+// 14.0 with the row kernels; with 1,572 rows 6.9 and 10.0 against 10.9 and 14.7.
+// Of 7 columns in FP64: 9.2 against 9.6, and 6.8 against 10.0.  In mixed
+// precision up to 8 columns are cheap in the row kernel: 8.7 ms against its 8.3
+// at 525 rows, 5.9 against 6.0 at 1,572.
+int64_t digit_tail_rows(bool mixed, int k) { return mixed && k <= 8 ? 1024 : 128; }
 
 // the tail product's error word, in row 5 of the column scalars
 int* tail_error(MultiState& S) { return reinterpret_cast<int*>(S.scal.get() + 5 * MAXK); }
@@ -772,10 +777,10 @@ void ensure_state(afp_amg* h, int k) {
   S->scal.alloc(ctx, 8 * MAXK + (int64_t)RED_GRID * MAXK + 1);  // scalars, partials, retire counter
   S->scal.zero();
   S->active.alloc(ctx, MAXK);
-  // The dense tail by digits from kDigitTail rows on.  Where the device has no
+  // The dense tail by digits from digit_tail_rows on.  Where the device has no
   // room for them (14 or 18 bytes an entry), and below, the row kernels.
   const Level& T = h->lv[h->t];
-  if (h->tail_dense && T.n >= kDigitTail) {
+  if (h->tail_dense && T.n >= digit_tail_rows(mixed, k)) {
     try {
       if (!h->tail_digits) {
         auto D = std::make_unique<TailDigits>();
