@@ -2,12 +2,11 @@
 // src/AMGSolver.cpp:384-639, and the CG of
 // examples/FAST/src/poisson_solver_comparison_afepack.cpp:197-253).
 //
-// Setup reproduces the reference hierarchy: per level the host runs the C/F
-// splitting (host_project) on the level matrix, the GPU forms P A P^T
-// (galerkin_product), and the coarse matrix comes back to the host for the
-// next splitting, until the reference's stop rule holds -- or, GB300-side,
-// until a level is small enough (opts.dense_tail) to be solved through a
-// dense inverse, the reference's own coarsest-level treatment.
+// Setup reproduces the reference hierarchy: per level the C/F splitting and
+// P (gpu_project, or host_project) and P A P^T (galerkin_product), until the
+// reference's stop rule holds -- or, GB300-side, until a level is small enough
+// (opts.dense_tail) to be solved through a dense inverse, the reference's own
+// coarsest-level treatment.  Host threads colour the levels meanwhile.
 //
 // For the solve every smoothed level is colour-permuted: rows are grouped by
 // greedy colour class so that a Gauss-Seidel class is a contiguous row

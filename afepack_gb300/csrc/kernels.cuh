@@ -61,8 +61,8 @@ struct DevCSR {
 };
 
 // Project() on the GPU (coarsen.cu): flags and P, P^T bitwise the host
-// routine's; cf[i] = 1 for C points, 0 for F points; rounds of the two
-// passes for the trace.
+// routine's; cf[i] = 1 for C points, 0 for F points; steps of the two
+// passes' waves for the trace.
 struct GpuProjection {
   DevCSR P, Pt;
   DevBuf<int> cf;

@@ -193,10 +193,11 @@ typedef struct afp_amg_opts {
                            with at most 16384 rows and at least 5% of its
                            entries nonzero; that level is solved with a dense
                            inverse instead of smoothed (0 keeps the
-                           reference's full depth).  The inverse costs 2 n^3
-                           FP64 operations (0.1 s at 4096 rows), so a sparse
-                           level of more rows (a 33K-DOF 2D problem's
-                           7,644-row third level: 1 s) is coarsened further
+                           reference's full depth).  The inverse costs n^3
+                           operations and n^2 memory (11 ms at 4096 rows, 35
+                           at 6,744 when the matrix is symmetric positive
+                           definite; some twenty times that otherwise), so a
+                           sparse level of more rows is coarsened further
                            instead; dense coarse levels of 3D and 2D P2
                            hierarchies (6,744 rows at 12%, 12,588 at 11%)
                            stop by density */
@@ -217,7 +218,7 @@ typedef struct afp_amg_opts {
   int fused_vcycle;     /* mixed precision: run each V-cycle as one persistent
                            kernel (1) instead of a chain of ~100 PDL launches
                            (0, default: on the 3D P1 64^3 hierarchy the chain
-                           takes 0.80 ms per V-cycle and the persistent kernel
+                           takes 0.63 ms per V-cycle and the persistent kernel
                            0.93 ms -- both are bound by ~100 dependent steps,
                            a launch or a grid-wide wait of ~2.5 us each).  The kernel keeps one CTA per SM and
                            streams every CTA's share of the level operators
@@ -253,8 +254,8 @@ typedef struct afp_solve_info {
 void afp_amg_default_opts(afp_amg_opts *opts);
 
 /* AMGSolver::reinit (src/AMGSolver.cpp:384-438): the C/F splitting of
- * Project (:18-226) runs on the host, the Galerkin product P A P^T of
- * getPMPt (:288-358) on the GPU, level by level, until the reference's stop
+ * Project (:18-226) (opts.gpu_coarsen = 0: on the host) and the Galerkin
+ * product P A P^T of getPMPt (:288-358) run on the GPU, level by level, until the reference's stop
  * rule (order <= max_coarse and density >= min_density) holds. */
 afp_status afp_amg_setup(afp_matrix *a, const afp_amg_opts *opts, afp_amg **out);
 /* AMGSolver::lazyReinit on a fresh solver, i.e. lazyInit (src/AMGSolver.cpp:442-503):
