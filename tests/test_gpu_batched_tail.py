@@ -22,7 +22,8 @@ def _spd(n, seed):
 
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("n,ks", [(100, (3,)), (127, (5, 64)), (128, (1, 16, 17)), (129, (33,)), (511, (2, 64)),
-                                  (512, (32, 31)), (513, (64, 7)), (1000, (15,)), (1153, (64, 48))])
+                                  (512, (32, 31)), (513, (64, 7)), (1000, (15,)), (1023, (8, 9)), (1024, (8, 9)),
+                                  (1153, (64, 48))])
 def test_batched_tail(ctx, n, ks, precision):
     import scipy.sparse as sp
     from afepack_gb300.amg import AMGSolver
