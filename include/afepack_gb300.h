@@ -218,7 +218,7 @@ typedef struct afp_amg_opts {
   int fused_vcycle;     /* mixed precision: run each V-cycle as one persistent
                            kernel (1) instead of a chain of ~100 PDL launches
                            (0, default: on the 3D P1 64^3 hierarchy the chain
-                           takes 0.63 ms per V-cycle and the persistent kernel
+                           takes 0.61 ms per V-cycle and the persistent kernel
                            0.93 ms -- both are bound by ~100 dependent steps,
                            a launch or a grid-wide wait of ~2.5 us each).  The kernel keeps one CTA per SM and
                            streams every CTA's share of the level operators
