@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kProdThreads, 1) k_spd_product(const __nv_bflo
 #pragma unroll
           for (int q = 0; q < kKC / 16; ++q)
             mma(tmem + min(i + j, kAcc - 1) * kTN, mat_desc(ab + i * kABytes + q * 256), mat_desc(bb + j * kBBytes + q * 256),
-                instr_desc(kTM, kTN), kc > 0 || i > 0 || q > 0);
+                instr_desc(kTM, kTN), kc > 0 || i > 0 || j >= kAcc || q > 0);  // each accumulator's first product overwrites
       mma_commit(&empty[st]);
     }
     mma_commit(&done);

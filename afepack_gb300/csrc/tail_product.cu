@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tail_product(int64_t n, int64_t
 #pragma unroll
             for (int q = 0; q < kKC / 16; ++q)
               mma(tmem + min(i + j, ACC - 1) * N, mat_desc(ab + i * Sh::kA + q * 256),
-                  mat_desc(bb + j * Sh::kBb + q * 256), instr_desc(kTM, N), kc > 0 || i > 0 || q > 0);
+                  mat_desc(bb + j * Sh::kBb + q * 256), instr_desc(kTM, N),
+                  kc > 0 || i > 0 || j >= ACC || q > 0);  // each accumulator's first product overwrites
         mma_commit(&empty[b]);
       }
       mma_commit(&done);

@@ -1,0 +1,137 @@
+"""The tensor-core digit products, entry by entry, on matrices whose entries and inverses span many decades.
+
+The matrices are 7-point operators with a random coefficient a cell, of a given contrast: M-matrices, whose inverse
+has positive entries only.  A hierarchy whose stop rule holds on the fine matrix itself is one dense level, so a V-cycle
+from zero is x = T b with T the inverse as the library holds it (for a unit vector b: a column of T, exactly in FP64),
+and one step of batched CG from zero gives alpha_c T B per column.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+M = 9
+N_ROWS = M ** 3  # 729: three panels of the inverse, two chunks of the batched product
+
+
+def cells(contrast, seed, m=M):
+    """Dense 7-point matrix of m^3 unknowns with a coefficient 10^U(0, log10 contrast) in every cell."""
+    rng = np.random.default_rng(seed)
+    k = 10.0 ** rng.uniform(0.0, np.log10(contrast), (m + 2,) * 3)
+    idx = np.arange(m ** 3).reshape(m, m, m)
+    A = np.zeros((m ** 3, m ** 3))
+    diag = np.zeros((m, m, m))
+    inner = (slice(1, -1),) * 3
+    for axis in range(3):
+        for step in (-1, 1):
+            near = np.roll(k, -step, axis)[inner]
+            w = 2.0 * k[inner] * near / (k[inner] + near)
+            diag += w
+            here = [slice(None)] * 3
+            there = [slice(None)] * 3
+            here[axis] = slice(1, None) if step < 0 else slice(None, -1)
+            there[axis] = slice(None, -1) if step < 0 else slice(1, None)
+            A[idx[tuple(here)].ravel(), idx[tuple(there)].ravel()] = -w[tuple(here)].ravel()
+    A[np.arange(m ** 3), np.arange(m ** 3)] = diag.ravel()
+    return (A + A.T) / 2
+
+
+def hierarchy(ctx, A, precision=0):
+    from afepack_gb300.amg import AMGSolver
+    from afepack_gb300.fem import SparseMatrix
+    n = len(A)
+    rp, ci, va = [0], [], []
+    for i in range(n):
+        js = [i] + [j for j in np.nonzero(A[i])[0] if j != i]
+        ci += js
+        va += list(A[i, js])
+        rp.append(len(ci))
+    K = SparseMatrix.from_csr(ctx, np.array(rp, np.int32), np.array(ci, np.int32), np.array(va))
+    amg = AMGSolver(K, nmpo=n + 1, nmpsd=0.0, precision=precision)
+    assert amg.solve_levels() == 1
+    return amg
+
+
+def held_inverse(amg, n, columns=None):
+    """Columns of the FP64 inverse that the hierarchy holds."""
+    columns = range(n) if columns is None else columns
+    out = []
+    for j in columns:
+        b, x = np.zeros(n), np.zeros(n)
+        b[j] = 1.0
+        amg.solve(x, b, step=0)
+        out.append(x)
+    return np.stack(out, axis=1)
+
+
+def one_step(native, amg, B):
+    """alpha_c T B_c: the iterate after one CG step from zero (whether it converged or not)."""
+    from afepack_gb300 import _native as N
+    X = np.zeros_like(B)
+    infos = (N.SolveInfo * B.shape[1])()
+    st = native.afp_pcg_solve_multi(amg.handle, N.ptr(X), N.ptr(B), B.shape[1], 1e-300, 1, infos)
+    assert st in (0, 5), native.afp_last_error()  # converged, or out of steps
+    return X
+
+
+def long_product(T, B):
+    return T.astype(np.longdouble) @ B.astype(np.longdouble)
+
+
+def right_hand_sides(A, k, seed):
+    """Half of the columns A x (graded as the matrix is), half of one size."""
+    rng = np.random.default_rng(seed)
+    B = rng.standard_normal((len(A), k))
+    B[:, ::2] = A @ B[:, ::2]
+    return B
+
+
+@pytest.mark.parametrize("contrast", [1e4])
+@pytest.mark.parametrize("k", [5, 16, 24, 64])
+def test_fp64_tail_is_as_good_as_fp64_sums(native, ctx, k, contrast):
+    """The batched product against the held inverse times B, per entry, within the classical bound of FP64 sums of
+    n terms, n eps sum |T||B|."""
+    A = cells(contrast, 11)
+    amg = hierarchy(ctx, A)
+    T = held_inverse(amg, N_ROWS)
+    B = right_hand_sides(A, k, 12)
+    X = one_step(native, amg, B)
+    want = long_product(T, B)
+    size = np.abs(T) @ np.abs(B)
+    for c in range(k):
+        alpha = np.median(X[:, c] / want[:, c])  # the step length, 1 to rounding
+        assert abs(alpha - 1) < 1e-9
+        err = np.abs(X[:, c] / alpha - want[:, c])
+        assert (err <= N_ROWS * EPS * size[:, c]).all(), (c, float((err / size[:, c]).max()))
+
+
+def refined_columns(A, columns):
+    """Columns of the inverse to beyond FP64: iterative refinement with residuals in long double."""
+    inv = np.linalg.inv(A)
+    rows, cols = np.nonzero(A)
+    vals = A[rows, cols].astype(np.longdouble)[:, None]
+    X = inv[:, columns].astype(np.longdouble)
+    for _ in range(4):
+        R = np.zeros(X.shape, np.longdouble)
+        R[columns, range(len(columns))] = 1
+        np.subtract.at(R, rows, vals * X[cols])
+        X = X + (inv @ R.astype(np.float64)).astype(np.longdouble)
+    return X
+
+
+def worst_of_median_row(T, want):
+    return float(np.median((np.abs(T - want) / np.abs(want)).max(axis=1)))
+
+
+@pytest.mark.parametrize("contrast", [1e2, 1e4])
+def test_inverse_entry_by_entry(ctx, contrast):
+    """The inverse of an M-matrix by elimination has small relative errors in every entry; entries span six decades a
+    row at contrast 1e4.  The worst entry of the median row is within n eps, a rounding per pivot."""
+    A = cells(contrast, 11)
+    amg = hierarchy(ctx, A)
+    cols = list(range(0, N_ROWS, 4))
+    T = held_inverse(amg, N_ROWS, cols)
+    assert worst_of_median_row(T, refined_columns(A, cols)) <= N_ROWS * EPS
