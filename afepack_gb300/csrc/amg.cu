@@ -455,7 +455,7 @@ void build_solve_layout(afp_amg* h, Built& built, const afp_matrix* A0) {
   Level& T = h->lv[t];
   if (h->tail_dense) {
     h->tail_inv.alloc(ctx, T.n * T.n);
-    if (!dense_inverse(ctx, T.A<double>(), h->tail_inv.get()))
+    if (!dense_inverse(ctx, T.A<double>(), h->tail_inv.get(), &h->tail_spd))
       fail(AFP_ERR_SINGULAR, "coarsest matrix is singular");
     if (mixed) {
       // FP32 pair with FP64-class accuracy: a plain FP32 inverse summed in

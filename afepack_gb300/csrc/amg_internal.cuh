@@ -174,6 +174,7 @@ struct afp_amg {
   std::shared_ptr<afp::Pattern> pat0;     // the fine matrix's pattern object (lazy re-setup check)
   afp::DevBuf<double> tail_inv;           // FP64 dense inverse (FP64 precision)
   afp::DevBuf<float> tail_hi, tail_lo;    // the same as an FP32 pair hi + lo (mixed precision)
+  bool tail_spd = false;                  // the tail is symmetric positive definite
   int64_t tail_ld = 0;                    // row stride of hi / lo (a multiple of 4 floats)
   std::unique_ptr<afp::TailDigits> tail_digits;  // the inverse's digits, made by the first batched solve
   // solver vectors (level-0 solve order)

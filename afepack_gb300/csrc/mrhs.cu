@@ -777,20 +777,24 @@ void ensure_state(afp_amg* h, int k) {
   S->scal.alloc(ctx, 8 * MAXK + (int64_t)RED_GRID * MAXK + 1);  // scalars, partials, retire counter
   S->scal.zero();
   S->active.alloc(ctx, MAXK);
-  // The dense tail by digits from digit_tail_rows on.  Where the device has no
-  // room for them (14 or 18 bytes an entry), and below, the row kernels.
+  // The dense tail by digits from digit_tail_rows on, if it is symmetric
+  // positive definite: its diagonal then bounds its entries, and scaling by it
+  // keeps their digits.  Other tails, smaller ones, and where the device has no
+  // room for the digits (20 bytes an entry), the row kernels.
   const Level& T = h->lv[h->t];
-  if (h->tail_dense && T.n >= digit_tail_rows(mixed, k)) {
+  if (h->tail_dense && h->tail_spd && T.n >= digit_tail_rows(mixed, k)) {
     try {
       if (!h->tail_digits) {
         auto D = std::make_unique<TailDigits>();
-        tail_digits(ctx, T.n, mixed ? nullptr : h->tail_inv.get(), h->tail_hi.get(), h->tail_lo.get(),
-                    mixed ? h->tail_ld : T.n, *D);
-        h->tail_digits = std::move(D);
+        if (tail_digits(ctx, T.n, mixed ? nullptr : h->tail_inv.get(), h->tail_hi.get(), h->tail_lo.get(),
+                        mixed ? h->tail_ld : T.n, *D))
+          h->tail_digits = std::move(D);
       }
-      auto W = std::make_unique<TailWork>();
-      tail_work(ctx, *h->tail_digits, k, *W);
-      S->tail = std::move(W);
+      if (h->tail_digits) {
+        auto W = std::make_unique<TailWork>();
+        tail_work(ctx, *h->tail_digits, k, *W);
+        S->tail = std::move(W);
+      }
     } catch (const Error& e) {
       if (e.status != AFP_ERR_OUT_OF_MEMORY) throw;
       cudaGetLastError();

@@ -863,7 +863,7 @@ void copy2d(const afp_context* ctx, int64_t rows, int64_t cols, const double* sr
 //   P <- P^-1,  R <- P^-1 R,  S <- S - C P^-1 R,  C <- -C P^-1,
 // which after every panel leaves the inverse; rows are pivoted within a
 // pivot block only.
-bool dense_inverse(const afp_context* ctx, const CSRView<double>& A, double* inv) {
+bool dense_inverse(const afp_context* ctx, const CSRView<double>& A, double* inv, bool* spd) {
   constexpr int64_t kPanel = 512;
   const int64_t n = A.m;
   auto fill = [&](double* M) {
@@ -872,7 +872,8 @@ bool dense_inverse(const afp_context* ctx, const CSRView<double>& A, double* inv
     check_launch(ctx, "dense copy");
   };
   fill(inv);
-  if (spd_inverse(ctx, n, inv)) return true;
+  *spd = spd_inverse(ctx, n, inv);
+  if (*spd) return true;
   if (n <= kPanel) {
     DevBuf<double> M(ctx, n * n);
     fill(M.get());

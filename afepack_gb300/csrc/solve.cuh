@@ -99,6 +99,7 @@ void l1_diag(const afp_context* ctx, const CSRView<double>& A, int64_t r0, int64
 // (spd_inverse.cu); false, with M undefined, when it is not.
 bool spd_inverse(const afp_context* ctx, int64_t n, double* M);
 // Dense inverse of the n x n CSR matrix; returns false when it is singular.
-bool dense_inverse(const afp_context* ctx, const CSRView<double>& A, double* inv);
+// *spd: whether the matrix turned out to be symmetric positive definite.
+bool dense_inverse(const afp_context* ctx, const CSRView<double>& A, double* inv, bool* spd);
 
 }  // namespace afp

@@ -12,17 +12,11 @@
 //
 // FP64 arithmetic runs at 2 multiply-adds a clock and SM here, so the n^3
 // part of a 6,744-row inverse is at least 0.25 s in FP64 even with symmetry.
-// The two products of a panel are therefore formed from kS = 9 digits of 7
-// bits (digits.cuh).  On grid matrices of 576 rows with coefficients of
-// contrast 1, 1e4 and 1e8 the inverse is as far from an extended-precision one
-// as the same sweep with FP64 products: 2.2e-15, 8e-14 and 2e-11 of its norm
-// on either side; with 8 digits the small entries of the last two were 40 and
-// more times worse.
+// The two products of a panel are therefore formed from digits (digits.cuh).
 //
-// Measured (GB300, whole inverse): 6,744 rows 35 ms against 706 ms with the
+// Measured (GB300, whole inverse): 6,744 rows 34.5 ms against 706 ms with the
 // pivoted FP64 sweep of solve.cu (two launches per pivot, FP64 products);
-// 2,048 rows 3.6 ms, 256 rows 0.39 ms.  At 6,744 rows the trailing updates
-// take 24 of the 35 ms, the panels' own inverses 7.
+// 2,200 rows 4.0 ms, 256 rows 0.39 ms.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -37,10 +31,8 @@ namespace afp {
 namespace {
 
 constexpr int kB = 256;         // panel width
-constexpr int kS = 9;           // digits per number
-constexpr int kAcc = 8;         // accumulators of an output tile
 constexpr int kNK = kB / kKC;   // stages of one product
-constexpr int kTM = 128, kTN = 64;  // output tile of a block: kAcc accumulators of kTN columns fill tensor memory
+constexpr int kTN = 64;         // columns of an output tile: its accumulators fill tensor memory
 constexpr int kSub = 16;        // pivots per step of the panel's own inverse
 
 // ------------------------------------------------------------- eligibility
@@ -193,7 +185,7 @@ __global__ void __launch_bounds__(256) k_spd_cut_panel(int64_t n, int64_t k0, in
       v[0][e] = (on && j < pb) ? M[row * n + k0 + j] : 0.0;
     }
   }
-  cut_row<kS>(v, lane, groups, row, 0, dig, scale + row);
+  cut_row(v, lane, groups, row, 0, dig, scale + row);
 }
 
 // A dense `rows` x kB array cut into digits; with M, its rows also go back
@@ -209,7 +201,7 @@ __global__ void __launch_bounds__(256) k_spd_cut_dense(int64_t n, int64_t k0, in
   double v[1][8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) v[0][e] = Z[row * kB + 8 * lane + e];
-  cut_row<kS>(v, lane, groups, row, 0, dig, scale + row);
+  cut_row(v, lane, groups, row, 0, dig, scale + row);
   if (M == nullptr) return;
 #pragma unroll
   for (int e = 0; e < 8; ++e) tile[w][8 * lane + e] = v[0][e];
@@ -250,96 +242,44 @@ __global__ void k_spd_mirror(int64_t n, double* __restrict__ M) {
 }
 
 // -------------------------------------------------------- the digit product
-constexpr uint32_t kABytes = kTM * kKC * 2, kBBytes = kTN * kKC * 2;  // one digit's tile of a stage
-constexpr uint32_t kStageBytes = kS * (kABytes + kBBytes);
-constexpr int kStages = 2;
-constexpr size_t kProdSmem = kStages * kStageBytes + 1024;
-constexpr int kProdThreads = 192;
+constexpr size_t kProdSmem = DigitTile<kTN>::kSmem;
 
-// The exact sums over digit pairs of a kTM x kTN tile of A B^T (A, B digit
-// arrays of kB inner indices).  UPDATE: subtracted from (rows >= k0) or added
-// to the tiles of the lower triangle of `out` (row stride ld) that the panel
-// [k0, k0 + kB) does not own; otherwise stored to `out`.  One tile per block:
-// warp 4 streams the digits, warp 5 issues the products, warps 0-3 put the
-// sums together.  A tile is 720 products of 128 x 64 x 16, which read 6 KB of
-// shared memory each (48 clocks, 35K in all), and then 8,192 entries of six
-// FP64 operations (25K clocks); the accumulators fill tensor memory, so the
-// two do not overlap: 46 us a tile.  (73 us with integer conversions in place
-// of the fraction trick and the entries to update read after the products.)
+// The sums over digit pairs of a kTM x kTN tile of A B^T (A, B digit arrays of
+// kB inner indices).  UPDATE: subtracted from (rows >= k0) or added to the
+// tiles of the lower triangle of `out` (row stride ld) that the panel
+// [k0, k0 + kB) does not own; otherwise stored to `out`.  One tile per block
+// (digits.cuh).  A tile is 880 products of 128 x 64 x 16, which read 6 KB of
+// shared memory each (48 clocks, 42K in all), and then 8,192 entries of six
+// FP64 operations (25K clocks); the accumulators fill tensor memory, so the two
+// do not overlap.
 template <bool UPDATE>
-__global__ void __launch_bounds__(kProdThreads, 1) k_spd_product(const __nv_bfloat16* __restrict__ A, int64_t groups_a,
-                                                              const double* __restrict__ sa,
-                                                              const __nv_bfloat16* __restrict__ B, int64_t groups_b,
-                                                              const double* __restrict__ sb, int64_t rows,
-                                                              int64_t cols, int64_t k0, double* __restrict__ out,
-                                                              int64_t ld, int* __restrict__ error) {
+__global__ void __launch_bounds__(kDigitThreads, 1) k_spd_product(const __nv_bfloat16* __restrict__ A, int64_t groups_a,
+                                                               const double* __restrict__ sa,
+                                                               const __nv_bfloat16* __restrict__ B, int64_t groups_b,
+                                                               const double* __restrict__ sb, int64_t rows,
+                                                               int64_t cols, int64_t k0, double* __restrict__ out,
+                                                               int64_t ld, int* __restrict__ error) {
   const int64_t i0 = (int64_t)blockIdx.x * kTM, j0 = (int64_t)blockIdx.y * kTN;
   if (UPDATE) {
     if (j0 > i0 + kTM - 1) return;
     if ((i0 >= k0 && i0 < k0 + kB) || (j0 >= k0 && j0 < k0 + kB)) return;
   }
   extern __shared__ unsigned char prod_raw[];
-  __shared__ uint64_t full[kStages], empty[kStages], done;
-  __shared__ uint32_t tmem_slot;
+  __shared__ DigitPipe pipe;
   const uint32_t base = (smem_u32(prod_raw) + 1023u) & ~1023u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      bar_init(&full[s], 1);
-      bar_init(&empty[s], 1);
-    }
-    bar_init(&done, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = pipe_begin<kTN>(pipe);
   if (warp == 4 && lane == 0) {
-    int issued = 0;
-    for (int kc = 0; kc < kNK; ++kc) {
-      const int st = kc % kStages;
-      if (kc >= kStages && !bar_wait(&empty[st], ((kc / kStages) - 1) & 1)) {
-        atomicOr(error, 2);
-        break;
-      }
-      bar_expect(&full[st], kStageBytes);
-      const uint32_t dst = base + st * kStageBytes;
-      for (int s = 0; s < kS; ++s) {
-        bulk_load(dst + s * kABytes, A + (((size_t)kc * kS + s) * groups_a + i0 / 8) * (kKC * 8), kABytes, &full[st]);
-        bulk_load(dst + kS * kABytes + s * kBBytes, B + (((size_t)kc * kS + s) * groups_b + j0 / 8) * (kKC * 8),
-                  kBBytes, &full[st]);
-      }
-      ++issued;
-    }
-    // copies in flight end before the block does
-    for (int kc = issued > kStages ? issued - kStages : 0; kc < issued; ++kc)
-      if (!bar_wait(&full[kc % kStages], (kc / kStages) & 1)) atomicOr(error, 2);
+    int it = 0;
+    while (it < kNK && pipe_load<kTN>(pipe, base, it, A + digit_offset(groups_a, it, 0, i0, 0), groups_a * (kKC * 8),
+                                      B + digit_offset(groups_b, it, 0, j0, 0), groups_b * (kKC * 8)))
+      ++it;
+    if (!pipe_drain(pipe, it) || it < kNK) atomicOr(error, 2);
   } else if (warp == 5 && lane == 0) {
-    for (int kc = 0; kc < kNK; ++kc) {
-      const int st = kc % kStages;
-      if (!bar_wait(&full[st], (kc / kStages) & 1)) {
-        atomicOr(error, 2);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t ab = base + st * kStageBytes, bb = ab + kS * kABytes;
-#pragma unroll 1
-      for (int i = 0; i < kS; ++i)
-        for (int j = 0; i + j < kS; ++j)
-#pragma unroll
-          for (int q = 0; q < kKC / 16; ++q)
-            mma(tmem + min(i + j, kAcc - 1) * kTN, mat_desc(ab + i * kABytes + q * 256), mat_desc(bb + j * kBBytes + q * 256),
-                instr_desc(kTM, kTN), kc > 0 || i > 0 || j >= kAcc || q > 0);  // each accumulator's first product overwrites
-      mma_commit(&empty[st]);
-    }
-    mma_commit(&done);
+    int it = 0;
+    while (it < kNK && pipe_issue<kTN>(pipe, base, tmem, it, it == 0)) ++it;
+    if (it < kNK) atomicOr(error, 2);
+    mma_commit(&pipe.done);
   } else if (warp < 4) {
     // the entries to update, read while the products run: lane l holds columns l and 32 + l of its warp's 32 rows
     const int64_t ja = j0 + lane, jb = j0 + 32 + lane, iw = i0 + warp * 32;
@@ -352,31 +292,25 @@ __global__ void __launch_bounds__(kProdThreads, 1) k_spd_product(const __nv_bflo
         old[r][1] = i < rows && jb <= i ? out[i * ld + jb] : 0.0;
       }
     }
-    const double rs = sa[iw + lane] * (UPDATE && i0 >= k0 ? -0x1p-68 : 0x1p-68);  // 2^-12 of the digits' scale, 2^-56 of lo's units
+    const double rs = sa[iw + lane] * (UPDATE && i0 >= k0 ? -0x1p-62 : 0x1p-62);  // put_together's unit
     const double ca = sb[ja], cb = sb[jb];
-    const bool ok = bar_wait(&done, 0);
-    if (!ok) {
+    if (!bar_wait(&pipe.done, 0)) {
       if (lane == 0) atomicOr(error, 2);
     } else {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // the stages are free: warp w puts its rows' (hi, lo) there
+      // the stages are free: warp w puts its rows' sums there
       double2* tile = reinterpret_cast<double2*>(prod_raw + (base - smem_u32(prod_raw))) + warp * 32 * (kTN + 1);
 #pragma unroll 1
       for (int c = 0; c < kTN; c += 8) {
         float v[kAcc][8];
-#pragma unroll
-        for (int s = 0; s < kAcc; ++s) tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + s * kTN + c, v[s]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        pipe_read8<kTN>(tmem, c, v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          int w[kAcc];
+          float w[kAcc];
 #pragma unroll
-          for (int s = 0; s < 7; ++s) w[s] = __float2int_rn(v[s][e] * __int_as_float((127 + 7 * s) << 23));
-          w[7] = __float2int_rn(v[7][e] * 0x1p56f);
-          // hi = the weights 0..3 in units of weight 3, lo = the rest in units of weight 8: |hi| < 2^43, |lo| < 2^51
-          const long long hi = (long long)(w[0] * 128 + w[1]) * 16384 + (w[2] * 128 + w[3]);
-          const long long lo = (long long)(w[4] * 128 + w[5]) * 2097152 + ((long long)w[6] * 16384 + w[7]);
-          tile[lane * (kTN + 1) + c + e] = make_double2(exact_double(hi), exact_double(lo));
+          for (int s = 0; s < kAcc; ++s) w[s] = v[s][e];
+          const DigitSum sum = put_together(w);
+          tile[lane * (kTN + 1) + c + e] = make_double2(sum.hi, sum.lo);
         }
       }
       __syncwarp();
@@ -386,20 +320,15 @@ __global__ void __launch_bounds__(kProdThreads, 1) k_spd_product(const __nv_bflo
         const double s = __shfl_sync(0xffffffffu, rs, r);
         const double2 ta = tile[r * (kTN + 1) + lane], tb = tile[r * (kTN + 1) + 32 + lane];
         const double sca = s * ca, scb = s * cb;
-        const double va = fma(ta.y, sca, fma(ta.x, sca * 0x1p35, UPDATE ? old[r][0] : 0.0));
-        const double vb = fma(tb.y, scb, fma(tb.x, scb * 0x1p35, UPDATE ? old[r][1] : 0.0));
+        const double va = fma(ta.y, sca, fma(ta.x, sca * 0x1p34, UPDATE ? old[r][0] : 0.0));
+        const double vb = fma(tb.y, scb, fma(tb.x, scb * 0x1p34, UPDATE ? old[r][1] : 0.0));
         if (i < rows && (UPDATE ? ja <= i : ja < cols)) out[i * ld + ja] = va;
         if (i < rows && (UPDATE ? jb <= i : jb < cols)) out[i * ld + jb] = vb;
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
-  __syncthreads();
-  if (warp == 5) {
-    __syncwarp();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
-  }
+  pipe_end<kTN>(tmem);
 }
 
 }  // namespace
@@ -423,9 +352,9 @@ bool spd_inverse(const afp_context* ctx, int64_t n, double* M) {
     sc.alloc(ctx, np);
     sz.alloc(ctx, np);
     sq.alloc(ctx, kB);
-    dc.alloc(ctx, (size_t)np * kB * kS);
-    dz.alloc(ctx, (size_t)np * kB * kS);
-    dq.alloc(ctx, (size_t)kB * kB * kS);
+    dc.alloc(ctx, (size_t)np * kB * kDigits);
+    dz.alloc(ctx, (size_t)np * kB * kDigits);
+    dq.alloc(ctx, (size_t)kB * kB * kDigits);
     AFP_CUDA(cudaFuncSetAttribute(k_spd_product<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdSmem));
     AFP_CUDA(cudaFuncSetAttribute(k_spd_product<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProdSmem));
   }
@@ -444,12 +373,12 @@ bool spd_inverse(const afp_context* ctx, int64_t n, double* M) {
       check_launch(ctx, "spd cut pivot inverse");
       k_spd_cut_panel<<<(unsigned)groups, 256, 0, ctx->stream>>>(n, k0, pb, M, groups, dc.get(), sc.get());
       check_launch(ctx, "spd cut panel");
-      k_spd_product<false><<<dim3((unsigned)(np / kTM), kB / kTN), kProdThreads, kProdSmem, ctx->stream>>>(
+      k_spd_product<false><<<dim3((unsigned)(np / kTM), kB / kTN), kDigitThreads, kProdSmem, ctx->stream>>>(
           dc.get(), groups, sc.get(), dq.get(), kB / 8, sq.get(), np, kB, k0, Z.get(), kB, flag.get() + 1);
       check_launch(ctx, "spd panel product");
       k_spd_cut_dense<<<(unsigned)groups, 256, 0, ctx->stream>>>(n, k0, pb, Z.get(), M, groups, dz.get(), sz.get());
       check_launch(ctx, "spd cut panel product");
-      k_spd_product<true><<<dim3((unsigned)(np / kTM), (unsigned)(np / kTN)), kProdThreads, kProdSmem, ctx->stream>>>(
+      k_spd_product<true><<<dim3((unsigned)(np / kTM), (unsigned)(np / kTN)), kDigitThreads, kProdSmem, ctx->stream>>>(
           dz.get(), groups, sz.get(), dc.get(), groups, sc.get(), n, n, k0, M, n, flag.get() + 1);
       check_launch(ctx, "spd update");
     }

@@ -1,19 +1,25 @@
 // X = T R for the dense coarsest solve of the batched V-cycle: T the n x n
-// inverse, R an n x k block, by digit products on the tensor cores
-// (digits.cuh).  T is cut once per hierarchy, R every time, both with a scale
-// per row (column) and 512 inner indices, so that every 512 inner indices'
-// exact sums are put together and added up in FP64.  FP64 hierarchies take 9
-// digits a number, mixed-precision ones 7: 49 bits for an inverse held as a
-// pair of 48 and a residual of 24.
+// inverse of a symmetric positive definite matrix, R an n x k block, by digit
+// products on the tensor cores (digits.cuh).  T's rows and columns are scaled
+// by powers of two to a diagonal near one, which bounds its other entries, and
+// R's rows against it (exact); T is cut once per hierarchy, R every time, both
+// with a scale per row (column) and 512 inner indices, so that every 512 inner
+// indices' sums are put together and added up in FP64.
+//
+// Error against extended precision, the largest entry in units of sum |T||R|
+// (GB300, 729 rows, 7-point matrices with random cell coefficients of contrast
+// 1e2, 1e4 and 1e8): 1.3e-16, 2.0e-16 and 2.1e-15; the FP64 sums of the row
+// kernel 2.7e-15, 4.7e-15 and 4.8e-15.  In mixed precision (T a pair of 48 bits, R
+// FP32) the same digits: the result's own rounding to FP32 is all that shows.
+// With nine digits, unscaled, it was 1e-11 at 1e8, with seven for mixed precision
+// 2e-7 of the entries at 1e4 and 1e-4 at 1e8.
 //
 // One block takes 128 rows, all columns (N >= k, 16, 32 or 64) and a run of
 // 512-index chunks; partial sums of the runs meet in k_tail_add in order.  A
 // product of 128 x N x 16 reads 4 KB of T's digits and 32 N bytes of R's from
-// shared memory, 36 to 48 clocks; a chunk is 45 (28) x 32 of them and then
-// 128 N entries of five FP64 operations (20K clocks at N = 64).
-//
-// Measured (GB300), against a double-float product on the FP32 pipe (11
-// operations a term) and, in FP64, a warp per row: see tail_product().
+// shared memory, 36 to 48 clocks; a chunk is 55 x 32 of them and then 128 N
+// entries of five FP64 operations (20K clocks at N = 64).  Times against the row
+// kernels: digit_tail_rows in mrhs.cu.
 #include <algorithm>
 
 #include "common.cuh"
@@ -24,34 +30,48 @@
 namespace afp {
 namespace {
 
-constexpr int kTM = 128;
 constexpr int kChunk = 512, kChunkStages = kChunk / kKC;
-constexpr int kStages = 2;
-constexpr int kThreads = 192;
 
-template <int S>
+// e[i] with 2^e T_ii 2^e in [1/2, 2) (T from inv, or from hi + lo);
+// *flag = 1 unless every T_ii is a number in [2^-400, 2^400].
+__global__ void k_tail_exponents(int64_t n, const double* __restrict__ inv, const float* __restrict__ hi,
+                                 const float* __restrict__ lo, int64_t ld, int* __restrict__ e,
+                                 int* __restrict__ flag) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t q = i * ld + i;
+  const double d = inv != nullptr ? inv[q] : (double)hi[q] + (double)lo[q];
+  if (!(d >= 0x1p-400 && d <= 0x1p400)) *flag = 1;
+  e[i] = balance(d);
+}
+
+// T scaled and cut: rows and columns by 2^e; the rows' own 2^-e into their scales
 __global__ void __launch_bounds__(256) k_tail_cut(int64_t n, int64_t np, const double* __restrict__ inv,
                                                   const float* __restrict__ hi, const float* __restrict__ lo,
-                                                  int64_t ld, __nv_bfloat16* __restrict__ dig,
-                                                  double* __restrict__ scale) {
+                                                  int64_t ld, const int* __restrict__ ex,
+                                                  __nv_bfloat16* __restrict__ dig, double* __restrict__ scale) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), chunk = blockIdx.y;
+  const int er = row < n ? ex[row] : 0;
   double v[2][8];
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int64_t j = chunk * kChunk + 256 * h + 8 * lane + e;
-      const bool on = row < n && j < n;
-      v[h][e] = !on ? 0.0 : inv != nullptr ? inv[row * ld + j] : (double)hi[row * ld + j] + (double)lo[row * ld + j];
+      v[h][e] = 0.0;
+      if (row < n && j < n) {
+        const double t = inv != nullptr ? inv[row * ld + j] : (double)hi[row * ld + j] + (double)lo[row * ld + j];
+        v[h][e] = t * pow2(er + ex[j]);
+      }
     }
-  cut_row<S>(v, lane, np / 8, row, chunk * kChunkStages, dig, scale + chunk * np + row);
+  cut_row(v, lane, np / 8, row, chunk * kChunkStages, dig, scale + chunk * np + row, -er);
 }
 
-// The columns of R as rows of N: a warp per column and chunk
-template <int S, class X>
+// The columns of R as rows of N, its rows scaled by 2^-e: a warp per column and chunk
+template <class X>
 __global__ void __launch_bounds__(256) k_tail_cut_rhs(int64_t n, int k, int N, const X* __restrict__ R,
-                                                      __nv_bfloat16* __restrict__ dig, double* __restrict__ scale) {
+                                                      const int* __restrict__ ex, __nv_bfloat16* __restrict__ dig, double* __restrict__ scale) {
   const int lane = threadIdx.x & 31;
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int64_t chunk = blockIdx.y;
@@ -61,166 +81,81 @@ __global__ void __launch_bounds__(256) k_tail_cut_rhs(int64_t n, int k, int N, c
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int64_t j = chunk * kChunk + 256 * h + 8 * lane + e;
-      v[h][e] = c < k && j < n ? (double)R[j * k + c] : 0.0;
+      v[h][e] = c < k && j < n ? (double)R[j * k + c] * pow2(-ex[j]) : 0.0;
     }
-  cut_row<S>(v, lane, N / 8, c, chunk * kChunkStages, dig, scale + chunk * N + c);
+  cut_row(v, lane, N / 8, c, chunk * kChunkStages, dig, scale + chunk * N + c);
 }
 
-template <int S, int N>
-struct Shape {
-  static constexpr int kAcc = S < 8 ? S : 8;
-  static constexpr uint32_t kA = kTM * kKC * 2, kBb = N * kKC * 2;  // a digit's tile of a stage
-  static constexpr uint32_t kStage = S * (kA + kBb);
-  static constexpr uint32_t kCols = N >= 64 ? 512 : N >= 32 ? 256 : 128;  // tensor memory columns
-  static constexpr size_t kSmem = kStages * kStage + 1024;
-};
-
-// Digit sums of one accumulator set -> the entry, times 2^55 (S = 9) or 2^42
-// (S = 7).  At 512 inner indices a sum of weight s < 7 is an integer of at most
-// (s + 1) 2^21 units; the last accumulator of S = 9 holds the weights 7 and 8,
-// rounded here to half a unit of weight 8 (at most 2^30.1 of those).
-template <int S, int ACC>
-__device__ __forceinline__ double put_together(const float (&v)[ACC]) {
-  int w[ACC];
-#pragma unroll
-  for (int s = 0; s < ACC; ++s)
-    w[s] = __float2int_rn(v[s] * __int_as_float((127 + (S == 9 && s == 7 ? 55 : 7 * s)) << 23));
-  const long long four = (long long)(w[0] * 128 + w[1]) * 16384 + (long long)(w[2] * 128 + w[3]);  // < 2^42.1
-  if constexpr (S == 9) {
-    const long long hi = four * 128 + w[4];                                                // < 2^49.1
-    const long long lo = (long long)w[5] * 1048576 + ((long long)w[6] * 8192 + w[7]);      // < 2^44
-    return fma(exact_double(hi), 0x1p27, exact_double(lo));
-  } else {
-    const long long lo = (long long)(w[4] * 128 + w[5]) * 128 + w[6];
-    return fma(exact_double(four), 0x1p21, exact_double(lo));
-  }
-}
-
-template <int S, int N>
-__global__ void __launch_bounds__(kThreads, 1) k_tail_product(int64_t n, int64_t np, int k, int chunks, int splits,
-                                                              const __nv_bfloat16* __restrict__ T,
-                                                              const double* __restrict__ st,
-                                                              const __nv_bfloat16* __restrict__ R,
-                                                              const double* __restrict__ sr,
-                                                              double* __restrict__ part, int* __restrict__ error) {
-  using Sh = Shape<S, N>;
-  constexpr int ACC = Sh::kAcc;
+template <int N>
+__global__ void __launch_bounds__(kDigitThreads, 1) k_tail_product(int64_t n, int64_t np, int k, int chunks, int splits,
+                                                                const __nv_bfloat16* __restrict__ T,
+                                                                const double* __restrict__ st,
+                                                                const __nv_bfloat16* __restrict__ R,
+                                                                const double* __restrict__ sr,
+                                                                double* __restrict__ part, int* __restrict__ error) {
   const int64_t i0 = (int64_t)blockIdx.x * kTM;
   const int split = blockIdx.y;
   const int ch0 = split * chunks / splits, ch1 = (split + 1) * chunks / splits;
-  const int64_t groups = np / 8;
   extern __shared__ unsigned char tail_raw[];
-  __shared__ uint64_t full[kStages], empty[kStages], done, flushed;
-  __shared__ uint32_t tmem_slot;
+  __shared__ DigitPipe pipe;
   const uint32_t base = (smem_u32(tail_raw) + 1023u) & ~1023u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // stages of a chunk: the last one's end with n
   auto stages_of = [&](int ch) { return (int)min((int64_t)kChunkStages, (n - (int64_t)ch * kChunk + kKC - 1) / kKC); };
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      bar_init(&full[s], 1);
-      bar_init(&empty[s], 1);
-    }
-    bar_init(&done, 1);
-    bar_init(&flushed, 128);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "n"(Sh::kCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = pipe_begin<N>(pipe);
   if (warp == 4 && lane == 0) {
     int it = 0;
     bool ok = true;
     for (int ch = ch0; ch < ch1 && ok; ++ch) {
       const int ns = stages_of(ch);
-      for (int kc = 0; kc < ns; ++kc, ++it) {
-        const int b = it % kStages;
-        if (it >= kStages && !bar_wait(&empty[b], ((it / kStages) - 1) & 1)) {
-          atomicOr(error, 1);
-          ok = false;
-          break;
-        }
-        bar_expect(&full[b], Sh::kStage);
-        const uint32_t dst = base + b * Sh::kStage;
-        const size_t stage = (size_t)ch * kChunkStages + kc;
-        for (int s = 0; s < S; ++s) {
-          bulk_load(dst + s * Sh::kA, T + ((stage * S + s) * groups + i0 / 8) * (kKC * 8), Sh::kA, &full[b]);
-          bulk_load(dst + S * Sh::kA + s * Sh::kBb, R + (stage * S + s) * (N / 8) * (kKC * 8), Sh::kBb, &full[b]);
-        }
+      for (int kc = 0; kc < ns && ok; ++kc) {
+        const int64_t stage = (int64_t)ch * kChunkStages + kc;
+        ok = pipe_load<N>(pipe, base, it, T + digit_offset(np / 8, stage, 0, i0, 0), np * kKC,
+                          R + digit_offset(N / 8, stage, 0, 0, 0), N * kKC);
+        it += ok;
       }
     }
-    // copies in flight end before the block does
-    for (int q = it > kStages ? it - kStages : 0; q < it; ++q)
-      if (!bar_wait(&full[q % kStages], (q / kStages) & 1)) atomicOr(error, 1);
+    if (!pipe_drain(pipe, it) || !ok) atomicOr(error, 1);
   } else if (warp == 5 && lane == 0) {
     int it = 0;
     bool ok = true;
     for (int ch = ch0; ch < ch1; ++ch) {
-      const int ns = stages_of(ch);
       // the accumulators of the chunk before have been read
-      if (ok && ch > ch0 && !bar_wait(&flushed, (ch - ch0 - 1) & 1)) {
-        atomicOr(error, 1);
-        ok = false;
-      }
-      if (ok) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int kc = 0; kc < ns && ok; ++kc, ++it) {
-        const int b = it % kStages;
-        if (!bar_wait(&full[b], (it / kStages) & 1)) {
-          atomicOr(error, 1);
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t ab = base + b * Sh::kStage, bb = ab + S * Sh::kA;
-#pragma unroll 1
-        for (int i = 0; i < S; ++i)
-          for (int j = 0; i + j < S; ++j)
-#pragma unroll
-            for (int q = 0; q < kKC / 16; ++q)
-              mma(tmem + min(i + j, ACC - 1) * N, mat_desc(ab + i * Sh::kA + q * 256),
-                  mat_desc(bb + j * Sh::kBb + q * 256), instr_desc(kTM, N),
-                  kc > 0 || i > 0 || j >= ACC || q > 0);  // each accumulator's first product overwrites
-        mma_commit(&empty[b]);
-      }
-      mma_commit(&done);
+      if (ok && ch > ch0) ok = bar_wait(&pipe.flushed, (ch - ch0 - 1) & 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int ns = stages_of(ch);
+      for (int kc = 0; kc < ns && ok; ++kc, ++it) ok = pipe_issue<N>(pipe, base, tmem, it, kc == 0);
+      mma_commit(&pipe.done);
     }
+    if (!ok) atomicOr(error, 1);
   } else if (warp < 4) {
     const int64_t row = i0 + warp * 32 + lane;
     double acc[N];
 #pragma unroll
     for (int c = 0; c < N; ++c) acc[c] = 0.0;
     for (int ch = ch0; ch < ch1; ++ch) {
-      const double rs = st[(int64_t)ch * np + row] * (S == 9 ? 0x1p-67 : 0x1p-54);  // 2^-12 of the digits' scale, the sums' unit
+      const double rs = st[(int64_t)ch * np + row] * 0x1p-62;  // put_together's unit
       const double* cs = sr + (int64_t)ch * N;
-      if (!bar_wait(&done, (ch - ch0) & 1)) {
+      if (!bar_wait(&pipe.done, (ch - ch0) & 1)) {
         atomicOr(error, 1);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int c = 0; c < N; c += 8) {
-        float v[ACC][8];
-#pragma unroll
-        for (int s = 0; s < ACC; ++s) tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + s * N + c, v[s]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float v[kAcc][8];
+        pipe_read8<N>(tmem, c, v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          float w[ACC];
+          float w[kAcc];
 #pragma unroll
-          for (int s = 0; s < ACC; ++s) w[s] = v[s][e];
-          acc[c + e] = fma(put_together<S, ACC>(w), rs * cs[c + e], acc[c + e]);
+          for (int s = 0; s < kAcc; ++s) w[s] = v[s][e];
+          const DigitSum sum = put_together(w);
+          acc[c + e] = fma(fma(sum.hi, 0x1p34, sum.lo), rs * cs[c + e], acc[c + e]);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&flushed)) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&pipe.flushed)) : "memory");
     }
     if (row < n) {
       double* o = part + ((int64_t)split * n + row) * k;
@@ -230,12 +165,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tail_product(int64_t n, int64_t
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
-  __syncthreads();
-  if (warp == 5) {
-    __syncwarp();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(Sh::kCols) : "memory");
-  }
+  pipe_end<N>(tmem);
 }
 
 template <class X>
@@ -249,48 +179,33 @@ __global__ void k_tail_add(int64_t nk, int parts, const double* __restrict__ par
 
 int pad_cols(int k) { return k <= 16 ? 16 : k <= 32 ? 32 : 64; }
 
-template <int S, class X>
-void product(const afp_context* ctx, const TailDigits& D, TailWork& W, const X* R, X* out, int k, int* error) {
-  const int N = pad_cols(k);
-  k_tail_cut_rhs<S, X><<<dim3(N / 8, D.chunks), 256, 0, ctx->stream>>>(D.n, k, N, R, W.dig.get(), W.scale.get());
-  check_launch(ctx, "tail right-hand side digits");
-  auto go = [&](auto Nc) {
-    constexpr int NN = decltype(Nc)::value;
-    AFP_CUDA(cudaFuncSetAttribute(k_tail_product<S, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)Shape<S, NN>::kSmem));
-    k_tail_product<S, NN><<<dim3((unsigned)(D.np / kTM), W.splits), kThreads, Shape<S, NN>::kSmem, ctx->stream>>>(
-        D.n, D.np, k, D.chunks, W.splits, D.dig.get(), D.scale.get(), W.dig.get(), W.scale.get(), W.part.get(),
-        error);
-  };
-  if (N == 16) go(std::integral_constant<int, 16>());
-  else if (N == 32) go(std::integral_constant<int, 32>());
-  else go(std::integral_constant<int, 64>());
-  check_launch(ctx, "tail product");
-  k_tail_add<X><<<grid_for(D.n * k, 256), 256, 0, ctx->stream>>>(D.n * k, W.splits, W.part.get(), out);
-  check_launch(ctx, "tail sums");
-}
-
 }  // namespace
 
-void tail_digits(const afp_context* ctx, int64_t n, const double* inv, const float* hi, const float* lo, int64_t ld,
+bool tail_digits(const afp_context* ctx, int64_t n, const double* inv, const float* hi, const float* lo, int64_t ld,
                  TailDigits& D) {
   D.n = n;
   D.np = (n + kTM - 1) / kTM * kTM;
   D.chunks = (int)((n + kChunk - 1) / kChunk);
-  D.digits = inv != nullptr ? 9 : 7;
-  D.dig.alloc(ctx, (size_t)D.np * D.chunks * kChunk * D.digits);
+  D.ex.alloc(ctx, n);
+  DevBuf<int> flag(ctx, 1);
+  flag.zero();
+  k_tail_exponents<<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, inv, hi, lo, ld, D.ex.get(), flag.get());
+  check_launch(ctx, "tail exponents");
+  int bad = 0;
+  flag.download(&bad, 1);
+  sync(ctx);
+  if (bad) return false;
+  D.dig.alloc(ctx, (size_t)D.np * D.chunks * kChunk * kDigits);
   D.scale.alloc(ctx, (size_t)D.np * D.chunks);
-  const dim3 grid((unsigned)(D.np / 8), (unsigned)D.chunks);
-  if (D.digits == 9)
-    k_tail_cut<9><<<grid, 256, 0, ctx->stream>>>(n, D.np, inv, hi, lo, ld, D.dig.get(), D.scale.get());
-  else
-    k_tail_cut<7><<<grid, 256, 0, ctx->stream>>>(n, D.np, inv, hi, lo, ld, D.dig.get(), D.scale.get());
+  k_tail_cut<<<dim3((unsigned)(D.np / 8), (unsigned)D.chunks), 256, 0, ctx->stream>>>(
+      n, D.np, inv, hi, lo, ld, D.ex.get(), D.dig.get(), D.scale.get());
   check_launch(ctx, "tail digits");
+  return true;
 }
 
 void tail_work(const afp_context* ctx, const TailDigits& D, int k, TailWork& W) {
   const int N = pad_cols(k);
-  W.dig.alloc(ctx, (size_t)N * D.chunks * kChunk * D.digits);
+  W.dig.alloc(ctx, (size_t)N * D.chunks * kChunk * kDigits);
   W.scale.alloc(ctx, (size_t)N * D.chunks);
   // runs of chunks: as many as give the fewest chunks one after the other on
   // an SM (a block fills one), then the fewest
@@ -308,15 +223,28 @@ void tail_work(const afp_context* ctx, const TailDigits& D, int k, TailWork& W) 
   W.part.alloc(ctx, (size_t)W.splits * D.n * k);
 }
 
-template <>
-void tail_product<double>(const afp_context* ctx, const TailDigits& D, TailWork& W, const double* R, double* X, int k,
-                          int* error) {
-  product<9, double>(ctx, D, W, R, X, k, error);
+template <class X>
+void tail_product(const afp_context* ctx, const TailDigits& D, TailWork& W, const X* R, X* out, int k, int* error) {
+  const int N = pad_cols(k);
+  k_tail_cut_rhs<X><<<dim3(N / 8, D.chunks), 256, 0, ctx->stream>>>(D.n, k, N, R, D.ex.get(), W.dig.get(),
+                                                                    W.scale.get());
+  check_launch(ctx, "tail right-hand side digits");
+  auto go = [&](auto Nc) {
+    constexpr int NN = decltype(Nc)::value;
+    constexpr size_t smem = DigitTile<NN>::kSmem;
+    AFP_CUDA(cudaFuncSetAttribute(k_tail_product<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_tail_product<NN><<<dim3((unsigned)(D.np / kTM), W.splits), kDigitThreads, smem, ctx->stream>>>(
+        D.n, D.np, k, D.chunks, W.splits, D.dig.get(), D.scale.get(), W.dig.get(), W.scale.get(), W.part.get(),
+        error);
+  };
+  if (N == 16) go(std::integral_constant<int, 16>());
+  else if (N == 32) go(std::integral_constant<int, 32>());
+  else go(std::integral_constant<int, 64>());
+  check_launch(ctx, "tail product");
+  k_tail_add<X><<<grid_for(D.n * k, 256), 256, 0, ctx->stream>>>(D.n * k, W.splits, W.part.get(), out);
+  check_launch(ctx, "tail sums");
 }
-template <>
-void tail_product<float>(const afp_context* ctx, const TailDigits& D, TailWork& W, const float* R, float* X, int k,
-                         int* error) {
-  product<7, float>(ctx, D, W, R, X, k, error);
-}
+template void tail_product<double>(const afp_context*, const TailDigits&, TailWork&, const double*, double*, int, int*);
+template void tail_product<float>(const afp_context*, const TailDigits&, TailWork&, const float*, float*, int, int*);
 
 }  // namespace afp

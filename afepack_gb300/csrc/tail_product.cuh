@@ -7,11 +7,13 @@
 
 namespace afp {
 
-// The n x n inverse cut into digits (2 bytes each, 9 a number in FP64, 7 in
-// mixed precision), laid out once per hierarchy for the tensor cores.
+// The n x n inverse cut into digits (ten of 2 bytes a number, rows padded to
+// 128 and columns to 512), laid out once per hierarchy for the tensor cores;
+// ex: row and column i scaled by 2^ex[i] first.
 struct TailDigits {
   int64_t n = 0, np = 0;
-  int chunks = 0, digits = 0;
+  int chunks = 0;
+  DevBuf<int> ex;
   DevBuf<__nv_bfloat16> dig;
   DevBuf<double> scale;
 };
@@ -23,13 +25,15 @@ struct TailWork {
   DevBuf<double> scale, part;
 };
 
-// From the FP64 inverse (row stride ld), or from its FP32 pair hi + lo.
-void tail_digits(const afp_context* ctx, int64_t n, const double* inv, const float* hi, const float* lo, int64_t ld,
+// From the inverse of a symmetric positive definite matrix in FP64 (row stride
+// ld), or from its FP32 pair hi + lo.  False, with nothing allocated that
+// counts, if its diagonal is not positive or of extreme size.
+bool tail_digits(const afp_context* ctx, int64_t n, const double* inv, const float* hi, const float* lo, int64_t ld,
                  TailDigits& D);
 void tail_work(const afp_context* ctx, const TailDigits& D, int k, TailWork& W);
 
 // X = T R for n x k row-major blocks, k <= 64; *error |= 1 if a bounded wait
-// ran out.  FP64 digits take double blocks, mixed-precision ones float blocks.
+// ran out.
 template <class X>
 void tail_product(const afp_context* ctx, const TailDigits& D, TailWork& W, const X* R, X* out, int k, int* error);
 

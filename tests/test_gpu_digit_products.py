@@ -89,7 +89,7 @@ def right_hand_sides(A, k, seed):
     return B
 
 
-@pytest.mark.parametrize("contrast", [1e4])
+@pytest.mark.parametrize("contrast", [1e4, 1e8])
 @pytest.mark.parametrize("k", [5, 16, 24, 64])
 def test_fp64_tail_is_as_good_as_fp64_sums(native, ctx, k, contrast):
     """The batched product against the held inverse times B, per entry, within the classical bound of FP64 sums of
@@ -106,6 +106,50 @@ def test_fp64_tail_is_as_good_as_fp64_sums(native, ctx, k, contrast):
         assert abs(alpha - 1) < 1e-9
         err = np.abs(X[:, c] / alpha - want[:, c])
         assert (err <= N_ROWS * EPS * size[:, c]).all(), (c, float((err / size[:, c]).max()))
+
+
+def pair(T):
+    """T as the mixed-precision hierarchy holds it."""
+    hi = T.astype(np.float32)
+    lo = (T - hi).astype(np.float32)
+    return hi.astype(np.float64) + lo.astype(np.float64)
+
+
+def assert_mixed_product(X, T, B, k):
+    """Z is rounded to FP32 and so is, in effect, the step length taken from it (two roundings, 2^-22.5 with the
+    division); the sums themselves are good to 2^-40 of sum |T||R|: 729 terms of a double-float sum, whose low part
+    rounds at 2^-48 of the sum each."""
+    R = B.astype(np.float32).astype(np.float64)
+    want = long_product(T, R)
+    size = np.abs(T) @ np.abs(R)
+    for c in range(k):
+        alpha = np.median(X[:, c] / want[:, c])
+        err = np.abs(X[:, c] / alpha - want[:, c])
+        bound = 2.0 ** -22.5 * np.abs(want[:, c]) + 2.0 ** -40 * size[:, c]
+        assert (err <= bound).all(), (c, float((err / bound).max()))
+
+
+@pytest.mark.parametrize("contrast", [1e4, 1e8])
+@pytest.mark.parametrize("k", [5, 9, 33, 64])
+def test_mixed_tail_is_as_good_as_double_float_sums(native, ctx, k, contrast):
+    A = cells(contrast, 11)
+    T = pair(held_inverse(hierarchy(ctx, A), N_ROWS))
+    B = right_hand_sides(A, k, 13)
+    assert_mixed_product(one_step(native, hierarchy(ctx, A, 1), B), T, B, k)
+
+
+@pytest.mark.parametrize("kind", ["nonsymmetric", "indefinite"])
+@pytest.mark.parametrize("k", [16, 40])
+def test_mixed_tail_of_other_matrices(native, ctx, k, kind):
+    """Tails that are not symmetric positive definite, whose diagonal says nothing about their entries."""
+    A = cells(1e4, 14)
+    if kind == "nonsymmetric":
+        A = np.triu(A) + 0.5 * np.tril(A, -1)
+    else:
+        A[np.arange(0, N_ROWS, 2), np.arange(0, N_ROWS, 2)] *= -1
+    T = pair(held_inverse(hierarchy(ctx, A), N_ROWS))
+    B = right_hand_sides(A, k, 15)
+    assert_mixed_product(one_step(native, hierarchy(ctx, A, 1), B), T, B, k)
 
 
 def refined_columns(A, columns):
