@@ -16,6 +16,9 @@
 // A row's scale is that of its largest entry, so an entry that is 2^-17 of it
 // still has FP64's 53 bits and a smaller one fewer; callers scale rows and
 // columns of graded matrices first (by powers of two, which is exact).
+//
+// A row that holds an infinity or a NaN gets a NaN for its scale, so that every
+// result made from it is NaN.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -71,14 +74,15 @@ __device__ __forceinline__ int balance(double d) { return -((((__double2hiint(d)
 template <int H>
 __device__ __forceinline__ void cut_row(const double (&v)[H][8], int lane, int64_t groups, int64_t row, int64_t kc0,
                                         __nv_bfloat16* __restrict__ dig, double* __restrict__ scale, int shift = 0) {
-  int top = 0;  // high word of the largest |v|
+  int top = 0;  // high word of the largest |v|; infinities and NaNs are above all numbers
 #pragma unroll
   for (int h = 0; h < H; ++h)
 #pragma unroll
     for (int e = 0; e < 8; ++e) top = max(top, __double2hiint(v[h][e]) & 0x7fffffff);
   top = __reduce_max_sync(0xffffffffu, top) >> 20;
+  const bool finite = top < 0x7ff;
   // 2^ex > |v|; a row below 2^-900 counts as zeros
-  const int ex = min(900, max(-900, top - 1022));
+  const int ex = finite ? max(-900, top - 1022) : 0;
   constexpr double magic = 0x1.8p52;
   const double up = pow2(27 - ex), down = pow2(ex - 27), up2 = pow2(7 * kDigits - 1 - ex);
 #pragma unroll
@@ -87,7 +91,7 @@ __device__ __forceinline__ void cut_row(const double (&v)[H][8], int lane, int64
     long long lo[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const double x = v[h][e];
+      const double x = finite ? v[h][e] : 0.0;
       const double t = fma(x, up, magic);
       hi[e] = __double2loint(t);
       lo[e] = __double_as_longlong(fma(fma(-(t - magic), down, x), up2, magic)) - __double_as_longlong(magic);
@@ -116,7 +120,7 @@ __device__ __forceinline__ void cut_row(const double (&v)[H][8], int lane, int64
           *reinterpret_cast<const uint4*>(d);
     }
   }
-  if (lane == 0) *scale = pow2(ex - 6 + shift);
+  if (lane == 0) *scale = finite ? pow2(ex - 6 + shift) : __longlong_as_double(0x7ff8000000000000LL);
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

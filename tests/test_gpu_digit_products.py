@@ -190,3 +190,25 @@ def test_inverse_of_a_graded_matrix(ctx):
     T = held_inverse(amg, N_ROWS, cols)
     want = refined_columns(A, cols)
     assert worst_of_median_row(T, want) <= 4 * worst_of_median_row(np.linalg.inv(A)[:, cols], want)
+
+
+BREAKDOWN, TIMEOUT = 6, 8
+
+
+def solve_status(native, amg, B):
+    from afepack_gb300 import _native as N
+    X = np.zeros_like(B)
+    infos = (N.SolveInfo * B.shape[1])()
+    return native.afp_pcg_solve_multi(amg.handle, N.ptr(X), N.ptr(B), B.shape[1], 1e-8, 200, infos)
+
+
+def test_infinity_in_the_tail_is_a_breakdown(native, ctx):
+    """An entry that FP32 cannot hold is an infinity in the V-cycle: the solve breaks down, as it does where the
+    product is summed entry by entry, and does not go on with a number made of it."""
+    A = cells(1e2, 16)
+    amg = hierarchy(ctx, A, 1)
+    B = right_hand_sides(A, 48, 17)
+    bad = B.copy()
+    bad[5, 3] = 1e39
+    assert solve_status(native, amg, bad) == BREAKDOWN, native.afp_last_error()
+    assert solve_status(native, amg, B) == 0
