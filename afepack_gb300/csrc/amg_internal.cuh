@@ -72,6 +72,7 @@ struct MultiState {
   DevBuf<double> scal;                      // column scalars, 8 x k (row 5: error word of the tail product)
   DevBuf<int> active;                       // k flags
   std::unique_ptr<TailWork> tail;           // set when the dense tail is a digit product
+  bool injected = false;                    // the test's one failed product of this width has been reported
   cudaGraphExec_t graph = nullptr;
   int64_t graph_nodes = 0;
   ~MultiState() {

@@ -658,8 +658,18 @@ float* blk<float>(MultiState& S, int which, int l) {
 // at 525 rows, 5.9 against 6.0 at 1,572.
 int64_t digit_tail_rows(bool mixed, int k) { return mixed && k <= 8 ? 1024 : 128; }
 
-// the tail product's error word, in row 5 of the column scalars
+// The tail product's error word, in row 5 of the column scalars: cleared when
+// a solve or a server starts, and read with every iteration's scalars before
+// they are, since a product that gave up leaves any residual behind.
 int* tail_error(MultiState& S) { return reinterpret_cast<int*>(S.scal.get() + 5 * MAXK); }
+void clear_tail_error(const afp_context* ctx, MultiState& S) {
+  AFP_CUDA(cudaMemsetAsync(tail_error(S), 0, sizeof(int), ctx->stream));
+}
+void check_tail_error(const double* scalars) {
+  int e;
+  std::memcpy(&e, scalars + 5 * MAXK, sizeof(int));
+  if (e) fail(AFP_ERR_TIMEOUT, "batched dense tail: a bounded wait ran out");
+}
 
 template <class X, class PV>
 void vcycle_m(afp_amg* h, MultiState& S) {
@@ -839,6 +849,10 @@ void precondition_m(afp_amg* h) {
   }
   AFP_CUDA(cudaGraphLaunch(S.graph, ctx->stream));
   ctx->launches.n += S.graph_nodes;
+  if (h->opts.inject_barrier_stall == 2 && S.tail && !S.injected) {  // fault injection for tests
+    AFP_CUDA(cudaMemsetAsync(tail_error(S), 1, sizeof(int), ctx->stream));
+    S.injected = true;
+  }
 }
 
 }  // namespace
@@ -853,8 +867,9 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
   MultiState& S = *h->multi;
   const Level& L0 = h->lv[0];
   const int64_t n = L0.n, nk = n * k;
-  double* sc = S.scal.get();  // rows: 0 rz_a, 1 pq, 2 rr, 3 rz_b, 4 bb
+  double* sc = S.scal.get();  // rows: 0 rz_a, 1 pq, 2 rr, 3 rz_b, 4 bb, 5 the tail's error word
   double* partials = sc + 8 * MAXK;
+  clear_tail_error(ctx, S);
   cudaEvent_t e0, e1;
   AFP_CUDA(cudaEventCreate(&e0));
   AFP_CUDA(cudaEventCreate(&e1));
@@ -880,10 +895,14 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
     k_col_dot<KPL, VEC><<<rg, BLK, 0, ctx->stream>>>(n, S.Rs.get(), S.Rs.get(), k, partials, sc + 2 * MAXK);
     check_launch(ctx, "mrhs dot");
   });
-  std::vector<double> hb(k), hr(k), init(k), rel(k);
-  copy(ctx, hb.data(), sc + 4 * MAXK, sizeof(double) * k);
-  copy(ctx, hr.data(), sc + 2 * MAXK, sizeof(double) * k);
-  sync(ctx);
+  std::vector<double> host(6 * MAXK), init(k), rel(k);
+  const double *hr = host.data() + 2 * MAXK, *hb = host.data() + 4 * MAXK;
+  auto fetch = [&] {
+    copy(ctx, host.data(), sc, sizeof(double) * host.size());
+    sync(ctx);
+    check_tail_error(host.data());
+  };
+  fetch();
   std::vector<double> bn(k);
   int n_active = 0;
   std::vector<int> iters(k, 0);
@@ -918,8 +937,7 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
                                                       sc + 2 * MAXK);
         check_launch(ctx, "mrhs update x r");
       });
-      copy(ctx, hr.data(), sc + 2 * MAXK, sizeof(double) * k);
-      sync(ctx);
+      fetch();
       n_active = 0;
       for (int c = 0; c < k; ++c) {
         if (!act[c]) continue;
@@ -949,13 +967,7 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
   check_launch(ctx, "mrhs scatter x");
   AFP_CUDA(cudaEventRecord(e1, ctx->stream));
   copy(ctx, X_user, S.Tmp.get(), sizeof(double) * nk);
-  int tail_err = 0;
-  copy(ctx, &tail_err, tail_error(S), sizeof(int));
   sync(ctx);
-  if (tail_err) {
-    S.scal.zero();
-    fail(AFP_ERR_TIMEOUT, "batched dense tail: a bounded wait ran out");
-  }
   float ms = 0;
   AFP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
   cudaEventDestroy(e0);
@@ -1119,6 +1131,7 @@ void batch_driver(afp_batch_server* s) {
     AFP_CUDA(cudaMemsetAsync(S.P.get(), 0, sizeof(double) * n * k, ctx->stream));
     AFP_CUDA(cudaMemsetAsync(S.B.get(), 0, sizeof(double) * n * k, ctx->stream));
     S.active.upload(act.data(), k);
+    clear_tail_error(ctx, S);
     sync(ctx);
     for (;;) {
       // ---- admission: queued requests into free columns
@@ -1190,9 +1203,7 @@ void batch_driver(afp_batch_server* s) {
       sync(ctx);
       // ---- retire converged (or failed) columns
       const double* host = pin.scal;
-      int tail_err;
-      std::memcpy(&tail_err, host + 5 * MAXK, sizeof(int));
-      if (tail_err) fail(AFP_ERR_TIMEOUT, "batched dense tail: a bounded wait ran out");
+      check_tail_error(host);
       bool retired = false;
       for (int c = 0; c < k; ++c) {
         if (!act[c]) continue;

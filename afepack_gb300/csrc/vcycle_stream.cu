@@ -925,7 +925,7 @@ void fused_vcycle(afp_amg* h, const double* r64, double* z64) {
   a.nb = F.nb.get();
   a.nb_off = F.nb_off.get();
   a.limit_ns = (long long)(h->opts.wait_limit_s * 1e9);
-  a.stall = h->opts.inject_barrier_stall;
+  a.stall = h->opts.inject_barrier_stall != 0 && h->opts.inject_barrier_stall != 2;
   a.r64 = r64;
   a.z64 = z64;
   a.trace = F.trace.size() ? F.trace.get() : nullptr;

@@ -234,10 +234,12 @@ typedef struct afp_amg_opts {
                            barriers, neighbour waits, shared-memory slots);
                            past it the kernel stops and the call returns
                            AFP_ERR_TIMEOUT (default 2 s, at most 60) */
-  int inject_barrier_stall; /* fault injection for tests: the first grid
+  int inject_barrier_stall; /* fault injection for tests.  1: the first grid
                            barrier of each persistent V-cycle waits for one
                            arrival more than the grid has, so every wait runs
-                           out after wait_limit_s (default 0) */
+                           out after wait_limit_s.  2: the first dense tail
+                           product of each batch width is reported as one
+                           whose wait ran out (default 0) */
   int gpu_coarsen;      /* classical hierarchy: C/F splitting and P on the GPU
                            (1, default), with the host routine's flags and P
                            bit for bit, or on the host (0) */

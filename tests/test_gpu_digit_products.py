@@ -212,3 +212,31 @@ def test_infinity_in_the_tail_is_a_breakdown(native, ctx):
     bad[5, 3] = 1e39
     assert solve_status(native, amg, bad) == BREAKDOWN, native.afp_last_error()
     assert solve_status(native, amg, B) == 0
+
+
+@pytest.mark.parametrize("entry", [0.0, 1e39])
+def test_a_failed_tail_product_is_reported_once(native, ctx, entry):
+    """The first product of the width reports a wait that ran out (set from the host).  The call fails for that and
+    not for what the residual looks like then, and the next one on the same hierarchy is not blamed for it."""
+    A = cells(1e2, 16)
+    amg = hierarchy(ctx, A, 1)
+    amg.opts.inject_barrier_stall = 2
+    amg.reinit(amg.matrix)
+    B = right_hand_sides(A, 48, 17)
+    first = B.copy()
+    first[5, 3] += entry
+    assert solve_status(native, amg, first) == TIMEOUT, native.afp_last_error()
+    assert solve_status(native, amg, B) == 0, native.afp_last_error()
+
+
+def test_a_failed_tail_product_ends_the_server_and_nothing_after_it(native, ctx):
+    from afepack_gb300.serve import BatchServer
+    A = cells(1e2, 16)
+    amg = hierarchy(ctx, A, 1)
+    amg.opts.inject_barrier_stall = 2
+    amg.reinit(amg.matrix)
+    B = right_hand_sides(A, 48, 17)
+    with BatchServer(amg, width=48) as srv:
+        _, res = srv.wait(srv.submit(np.ascontiguousarray(B[:, 0])))
+    assert res["status"] == TIMEOUT
+    assert solve_status(native, amg, B) == 0, native.afp_last_error()
