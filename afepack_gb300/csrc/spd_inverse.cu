@@ -94,15 +94,6 @@ __global__ void k_spd_pivot_block(int64_t n, int64_t k0, int pb, const double* _
   P[t] = v;
 }
 
-// 1/p for a normal p by Newton-Raphson from the hardware's approximation
-__device__ __forceinline__ double newton_reciprocal(double p) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
-#pragma unroll
-  for (int i = 0; i < 2; ++i) y = fma(y, fma(-p, y, 1.0), y);
-  return y;
-}
-
 // One step of the block Gauss-Jordan inverse of P: kSub pivots, from `in` to
 // `out`.  A block owns 32 rows x kSub columns; its first warp inverts the
 // kSub x kSub pivot itself, in registers (lane l: row l / 2, eight columns),
@@ -131,7 +122,7 @@ __global__ void __launch_bounds__(128) k_spd_sweep(int kk, const double* __restr
       const double p = __shfl_sync(0xffffffffu, d[qc], 2 * q + h);
       const double f = __shfl_sync(0xffffffffu, d[qc], (tid & ~1) + h);
       bad |= !(p > 0.0);
-      const double y = newton_reciprocal(p);
+      const double y = 1.0 / p;
       const double g = row == q ? -y : f * y;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {

@@ -240,3 +240,13 @@ def test_a_failed_tail_product_ends_the_server_and_nothing_after_it(native, ctx)
         _, res = srv.wait(srv.submit(np.ascontiguousarray(B[:, 0])))
     assert res["status"] == TIMEOUT
     assert solve_status(native, amg, B) == 0, native.afp_last_error()
+
+
+def test_inverse_of_a_diagonal_matrix_is_its_reciprocal(ctx):
+    """Pivots alone: every entry within an ulp of the quotient, over the range of scales that the sweep takes."""
+    rng = np.random.default_rng(18)
+    d = rng.uniform(1.0, 2.0, 300) * 2.0 ** rng.integers(-390, 390, 300)
+    amg = hierarchy(ctx, np.diag(d))
+    x = np.zeros(300)
+    amg.solve(x, np.ones(300), step=0)
+    assert (np.abs(x - 1.0 / d) <= np.spacing(1.0 / d)).all()
