@@ -548,8 +548,8 @@ void setup(afp_amg* h, afp_matrix* A, bool lazy) {
     // after all (the next splitting needs getPMPt's values).  Whether a
     // level above dense_tail rows can reach the density rule is first
     // estimated from the symbolic count of an evenly spaced sample of its
-    // rows (with a margin), so that sparse levels never build the
-    // n_f x n_c intermediate.
+    // rows (with a margin), so that sparse levels never build the dense
+    // n_c x n_c product.
     bool dense_done = false;
     bool try_dense = o.dense_tail > 0 && P.m <= kDenseTailMax;
     if (try_dense && P.m > (int64_t)o.dense_tail) {
@@ -1093,7 +1093,9 @@ afp_status afp_amg_time_kernel(afp_amg* h, int kind, int level, int reps, double
       for (int l = 0; l < h->t; ++l) {
         const Level& Q = h->lv[l];
         const double m = (double)Q.nnz * (v + 4) + 4.0 * (Q.n + 1);
-        b += (2 * s + 1) * m + 2 * s * 3 * Q.n * v + 2 * Q.n * v;
+        // sweeps and residual: r, x, out; the first sweep reads no row of x that it has not written, so none of the
+        // last class (without sweeps x is filled with zeros)
+        b += (2 * s + 1) * (m + 3.0 * Q.n * v) + (s > 0 ? -(double)(Q.n - Q.cls[Q.cls.size() - 2]) : (double)Q.n) * v;
         b += 2.0 * Q.pnnz * (vp + 4) + 4.0 * (h->lv[l + 1].n + 1) + 4.0 * (Q.n + 1) + 3.0 * Q.n * v +
              2.0 * h->lv[l + 1].n * v;
       }

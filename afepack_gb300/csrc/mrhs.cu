@@ -1435,11 +1435,13 @@ void time_multi(afp_amg* h, int kind, int level, int reps, double* ms, double* b
   for (int l = 0; l < h->t; ++l) {
     const Level& Q = h->lv[l];
     const double nn = (double)Q.n, nc = (double)h->lv[l + 1].n;
-    b += (2 * s + 1) * pass(Q) + 2.0 * nn * v * k;                          // sweeps, residual, zero
+    // sweeps and residual; the first sweep reads no row of the iterate that it has not written, so none of the last
+    // class (without sweeps the iterate is filled with zeros)
+    b += (2 * s + 1) * pass(Q) + (s > 0 ? -(nn - (double)Q.cls[Q.cls.size() - 2]) : nn) * v * k;
     b += 2.0 * Q.pnnz * (vp + 4) + 4.0 * (nc + 1) + 4.0 * (nn + 1) + 3.0 * nn * v * k + 2.0 * nc * v * k;  // P, P^T
   }
   const double nt = (double)h->lv[h->t].n;
-  b += h->tail_dense ? nt * nt * 8.0 + 2.0 * nt * v * k : 0.0;
+  b += h->tail_dense ? nt * nt * (S.tail ? kTailEntryBytes : 8.0) + 2.0 * nt * v * k : 0.0;
   *bytes = b;
 }
 }  // namespace afp

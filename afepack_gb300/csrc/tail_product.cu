@@ -31,6 +31,7 @@ namespace afp {
 namespace {
 
 constexpr int kChunk = 512, kChunkStages = kChunk / kKC;
+static_assert(kTailEntryBytes == 2.0 * kDigits, "kTailEntryBytes");
 
 // e[i] with 2^e T_ii 2^e in [1/2, 2) (T from inv, or from hi + lo);
 // *flag = 1 unless every T_ii is a number in [2^-400, 2^400].

@@ -18,6 +18,8 @@ struct TailDigits {
   DevBuf<double> scale;
 };
 
+constexpr double kTailEntryBytes = 20.0;  // of an entry's digits
+
 // Work space of one batch width: the block's digits and the partial sums.
 struct TailWork {
   int splits = 1;

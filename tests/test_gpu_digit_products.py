@@ -250,3 +250,14 @@ def test_inverse_of_a_diagonal_matrix_is_its_reciprocal(ctx):
     x = np.zeros(300)
     amg.solve(x, np.ones(300), step=0)
     assert (np.abs(x - 1.0 / d) <= np.spacing(1.0 / d)).all()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_bytes_of_a_batched_vcycle(ctx, precision):
+    """The reported bytes are those of the code that runs: a tail product reads the digits, two bytes each."""
+    k = 48
+    A = cells(1e2, 16)
+    amg = hierarchy(ctx, A, precision)
+    amg.pcg_multi(right_hand_sides(A, k, 17), 1e-6, 50)
+    _, nbytes = amg.time_kernel(4, 0, 1)
+    assert nbytes == N_ROWS ** 2 * 2 * 10 + 2 * N_ROWS * k * (4 if precision else 8)
