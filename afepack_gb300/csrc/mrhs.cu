@@ -650,13 +650,19 @@ float* blk<float>(MultiState& S, int which, int l) {
   return (which == 0 ? S.X32 : which == 1 ? S.R32 : S.T32)[l].get();
 }
 
-// Rows from which the dense tail is a digit product.  CG of 64 columns with a
-// tail of 525 rows: 9.4 ms in mixed precision and 13.4 in FP64, against 10.1 and
-// 14.0 with the row kernels; with 1,572 rows 6.9 and 10.0 against 10.9 and 14.7.
-// Of 7 columns in FP64: 9.2 against 9.6, and 6.8 against 10.0.  In mixed
-// precision up to 8 columns are cheap in the row kernel: 8.7 ms against its 8.3
-// at 525 rows, 5.9 against 6.0 at 1,572.
-int64_t digit_tail_rows(bool mixed, int k) { return mixed && k <= 8 ? 1024 : 128; }
+// Rows from which the dense tail is a digit product.  That takes some 70 us
+// whatever the width as long as one block has all the rows' chunks, the row
+// kernels' time grows with rows and columns.  The tail alone (us, digits and
+// rows): FP64, 2 columns 72 and 70 at 525 rows; 4 columns 41 and 41 at 200, 51
+// and 61 at 300; 64 columns 57 and 57 at 200, 66 and 80 at 300, 88 and 409 at
+// 1,572.  Mixed precision, 4 columns 74 and 57 at 1,572, 74 and 114 at 3,000; 7
+// columns 74 and 76 at 1,572; 16 columns 74 and 72 at 1,024 (53 and 27 at 300);
+// 32 columns 80 and 66 at 525, 79 and 94 at 800; 64 columns 68 and 68 at 300, 90
+// and 321 at 1,572.
+int64_t digit_tail_rows(bool mixed, int k) {
+  if (!mixed) return k <= 2 ? 512 : 256;
+  return k <= 4 ? 2048 : k <= 8 ? 1536 : k <= 16 ? 1024 : k <= 32 ? 640 : 320;
+}
 
 // The tail product's error word, in row 5 of the column scalars: cleared when
 // a solve or a server starts, and read with every iteration's scalars before

@@ -261,3 +261,17 @@ def test_bytes_of_a_batched_vcycle(ctx, precision):
     amg.pcg_multi(right_hand_sides(A, k, 17), 1e-6, 50)
     _, nbytes = amg.time_kernel(4, 0, 1)
     assert nbytes == N_ROWS ** 2 * 2 * 10 + 2 * N_ROWS * k * (4 if precision else 8)
+
+
+@pytest.mark.parametrize("n_side,k,precision,digits", [(5, 64, 0, False), (6, 2, 0, False), (7, 3, 0, True),
+                                                       (9, 2, 0, True), (6, 64, 1, False), (7, 64, 1, True),
+                                                       (7, 16, 1, False), (8, 32, 1, False), (9, 32, 1, True),
+                                                       (11, 16, 1, True), (11, 8, 1, False)])
+def test_route_of_the_batched_tail(ctx, n_side, k, precision, digits):
+    """Small and narrow tails are summed row by row, the others by digits (by the bytes that a V-cycle reports)."""
+    A = cells(1e2, 19, n_side)
+    n = len(A)
+    amg = hierarchy(ctx, A, precision)
+    amg.pcg_multi(right_hand_sides(A, k, 20), 1e-6, 50)
+    _, nbytes = amg.time_kernel(4, 0, 1)
+    assert nbytes == n * n * (20 if digits else 8) + 2 * n * k * (4 if precision else 8)
