@@ -9,6 +9,8 @@
 //
 // Reductions are deterministic: each block writes a partial sum and the last
 // block to finish adds the partials in block order.
+#include <cstdlib>
+
 #include "df32.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
@@ -23,8 +25,19 @@ namespace afp {
 // 4, 6 and this: FP64 22.9, 19.8 and 19.2 ms, mixed 10.0, 9.3 and 9.4; on the
 // P2 100^2 one (11, 21, 54) 30.7, 32.1 and 30.7 ms in FP64.  Two lanes for the
 // rows of 7 of a 2D P1 level instead of four: 256^2 FP64 12.8 against 13.7 ms,
-// mixed 9.9 against 10.6; one lane gains nothing more.
+// mixed 9.9 against 10.6; one lane gains nothing more.  AFP_ENTRIES_PER_LANE in
+// the environment sets the limit for every row instead, at four lanes or more
+// (A/B timing).
 int pick_vec(double avg) {
+  static const double limit = [] {
+    const char* e = std::getenv("AFP_ENTRIES_PER_LANE");
+    return e ? std::atof(e) : 0.0;
+  }();
+  if (limit > 0.0) {
+    int vec = 4;
+    while (vec < 32 && vec * limit < avg) vec *= 2;
+    return vec;
+  }
   int vec = 2;
   while (vec < 32 && vec * (vec < 16 ? 4.0 : 6.0) < avg) vec *= 2;
   return vec;
