@@ -31,7 +31,7 @@ namespace {
 constexpr int BLK = 256;
 constexpr int WPB = BLK / 32;
 constexpr int MAXK = 64;
-constexpr int RED_GRID = 912;  // blocks of a column reduction: six per SM
+constexpr int RED_GRID = 912;  // blocks of a column reduction at most (red_blocks): six per SM
 
 template <class X>
 struct AccT {
@@ -92,7 +92,7 @@ __global__ void k_dense_gemm(int64_t n, const X* __restrict__ M, const X* __rest
 // loads).  spl groups share one row, group p taking the row's entries in chunks
 // p, p + spl, ... of W (long coarse-level rows: enough groups in flight to
 // cover the gather latency).  A chunk's (column, value) pairs are loaded one
-// per lane and broadcast with shuffles; the gathers of the x rows of U = 4
+// per lane and broadcast with shuffles; the gathers of the x rows of U
 // entries are issued before any of their products is summed.  The groups'
 // partial sums meet in shared memory and are added in group order, so the
 // result does not depend on timing.
@@ -103,7 +103,13 @@ __global__ void k_dense_gemm(int64_t n, const X* __restrict__ M, const X* __rest
 // hierarchy with 64 columns took 7.76 ms with 8 entries in flight and nothing
 // ahead, 6.05 with 4 entries and six blocks an SM, 5.65 with fewer groups per
 // row (rows_m); the tail aside, loading the next chunk ahead at four blocks (64
-// registers) is another 0.15 ms less than six blocks without.  The l1-Jacobi
+// registers) is another 0.15 ms less than six blocks without.  That holds for
+// vector gathers and for groups of up to four lanes, whose chunk is no longer
+// than that; scalar groups of eight lanes and more keep eight entries in flight,
+// as does one FP32 lane.  One V-cycle of a 36^3 P1 hierarchy in mixed precision
+// with 1, 3, 5, 12 and 33 columns: 0.85, 1.16, 1.08, 1.48 and 2.23 ms; with four
+// everywhere 0.95, 1.18, 1.43, 1.88 and 2.92; with eight everywhere 0.89, 2.04,
+// 1.11, 1.52 and 2.29.  The l1-Jacobi
 // class of a 48^3 second level now runs at 76% of L1's throughput.
 enum RowOp { RO_SPMM = 0, RO_SPMM_ADD, RO_RES, RO_GS, RO_JAC };
 
@@ -151,7 +157,8 @@ __global__ void __launch_bounds__(ROWS_BLK, 4) k_rows_m(int64_t r0, int64_t r1, 
       diag = as<A>(va[b]);
       ++b;
     }
-    constexpr int U = 4;
+    // entries in flight (see above; an FP64 lane pays for entries that are not there)
+    constexpr int U = !VEC && (W >= 8 || (W == 1 && sizeof(X) == 4)) ? 8 : 4;
     if (W == 1) {
       for (int j0 = b + pidx * U; j0 < e; j0 += spl * U) {
         A vals[U];
@@ -168,7 +175,7 @@ __global__ void __launch_bounds__(ROWS_BLK, 4) k_rows_m(int64_t r0, int64_t r1, 
     } else {
       // entries src[u] of the chunk, those with got[u] (the same for the whole
       // group; ALL: all of them)
-      auto take = [&](int cc, A vv, const int (&src)[U], const bool (&got)[U], auto ALLc) {
+      auto take = [&](int cc, A vv, const int* src, const bool* got, auto ALLc) {
         constexpr bool ALL = decltype(ALLc)::value;
         A vals[U];
         X xv[U][KPL];
@@ -249,7 +256,22 @@ __global__ void __launch_bounds__(ROWS_BLK, 4) k_rows_m(int64_t r0, int64_t r1, 
 #pragma unroll
     for (int q = 0; q < KPL; ++q) {
       A s = part[grp][lane][q];
-      for (int p = 1; p < spl; ++p) s += part[grp + p][lane][q];
+      // FP32: all the groups' sums are read at once (64 columns 1.82 -> 1.71 ms a V-cycle of that hierarchy); FP64
+      // pays for every addition, those of no group included
+      if constexpr (sizeof(X) == 4) {
+        auto add = [&](auto Nc) {
+          constexpr int N = decltype(Nc)::value < GPB ? decltype(Nc)::value : GPB;
+          A t[N];
+#pragma unroll
+          for (int p = 1; p < N; ++p) t[p] = part[min(grp + p, GPB - 1)][lane][q];
+#pragma unroll
+          for (int p = 1; p < N; ++p) s = p < spl ? s + t[p] : s;
+        };
+        if (spl <= 4) add(std::integral_constant<int, 4>());
+        else add(std::integral_constant<int, 16>());
+      } else {
+        for (int p = 1; p < spl; ++p) s += part[grp + p][lane][q];
+      }
       acc[q] = s;
     }
   }
@@ -425,6 +447,20 @@ __global__ void k_rows_scatter(int64_t n, int k, const int* __restrict__ perm, c
 }
 
 // ------------------------------------------------------ column reductions
+unsigned rows_grid(const afp_context* ctx, int64_t rows) {
+  const int64_t want = (rows + WPB - 1) / WPB;
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * 16));
+}
+
+// Blocks of a column reduction: the last one to finish adds all their partial
+// sums up, so two per SM unless the block is large.  12 iterations of CG, 304
+// blocks and 912: 22,801 rows 5 columns 5.3 and 6.1 ms; 117,649 rows 64 columns
+// (7.5M entries) 29.9 and 30.1; 160,801 rows 64 columns (10M) 24.7 and 24.4;
+// 274,625 rows 64 columns (18M) 64.5 and 63.8.
+unsigned red_blocks(const afp_context* ctx, int64_t n, int k) {
+  return std::min<unsigned>(n * k >= (int64_t)8 << 20 ? RED_GRID : RED_GRID / 3, rows_grid(ctx, n));
+}
+
 // Per-column sums of a.b over n x k blocks; deterministic (block partials,
 // last block adds them in a fixed order).  Lane l owns the columns l and
 // l + 32, or with VEC (an even k above 32) 2 l and 2 l + 1, which it reads as
@@ -538,7 +574,7 @@ __global__ void __launch_bounds__(BLK, 4) k_spmm_dot(int64_t m, const int* __res
       const int cc = my < e ? ci[my] : 0;
       const double vv = my < e ? va[my] : 0.0;
       const int cnt = min(32, e - base);
-      constexpr int U = 4;
+      constexpr int U = KPL == 1 ? 8 : 4;  // 50,653 rows, one load a lane: 88 us with 8, 104 with 4
       for (int jj = 0; jj < cnt; jj += U) {
         double vals[U], pv[U][KPL];
 #pragma unroll
@@ -623,11 +659,6 @@ __global__ void k_update_p(int64_t n, int k, const double* __restrict__ num, con
       if (act[t]) vp[t] = vz[t] + beta[t] * vp[t];
     row_store<KPL, VEC>(p + row * k, lane, k, vp);
   }
-}
-
-unsigned rows_grid(const afp_context* ctx, int64_t rows) {
-  const int64_t want = (rows + WPB - 1) / WPB;
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * 16));
 }
 
 // f(columns per lane, whether as one 16-byte load)
@@ -890,7 +921,7 @@ bool pcg_multi(afp_amg* h, double* X_user, const double* B_user, int nrhs, doubl
   std::vector<int> act(k, 1);
   S.active.upload(act.data(), k);
   const CSRView<double> A = L0.A<double>();
-  const unsigned rg = std::min<unsigned>(RED_GRID, rows_grid(ctx, n));
+  const unsigned rg = red_blocks(ctx, n, k);
   rows_m<double, double, RO_RES>(ctx, 0, n, A.rowptr, A.cols, A.vals, S.Xs.get(), S.Rs.get(), S.B.get(), nullptr, k,
                                  (double)L0.nnz / n, "mrhs residual");
   with_kpl(k, [&](auto KPLc, auto VECc) {
@@ -1132,7 +1163,7 @@ void batch_driver(afp_batch_server* s) {
     double* sc = S.scal.get();  // rows: 0 rz (old), 1 pq, 2 rr, 3 rz (new), 4 bb
     double* partials = sc + 8 * MAXK;
     const CSRView<double> A = L0.A<double>();
-    const unsigned rg = std::min<unsigned>(RED_GRID, rows_grid(ctx, n));
+    const unsigned rg = red_blocks(ctx, n, k);
     AFP_CUDA(cudaMemsetAsync(S.Rs.get(), 0, sizeof(double) * n * k, ctx->stream));
     AFP_CUDA(cudaMemsetAsync(S.P.get(), 0, sizeof(double) * n * k, ctx->stream));
     AFP_CUDA(cudaMemsetAsync(S.B.get(), 0, sizeof(double) * n * k, ctx->stream));
