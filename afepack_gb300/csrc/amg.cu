@@ -320,7 +320,10 @@ double l1_residual(afp_amg* h, const double* x, const double* r) {
 // The colouring of a level, on a host thread of its own: it needs nothing but
 // the level's host copy, so it runs beside the device's work on the levels
 // below.  (On a 64^3 hierarchy the three colourings took 0.19 s of the setup
-// one after the other at its end.)
+// one after the other at its end.)  Levels below kColorInline entries are
+// coloured when they are asked for: a thread costs more than that (16 rows,
+// lazy setup: 0.42 ms without one, 0.52 with).
+constexpr int64_t kColorInline = 4096;
 struct Coloring {
   int cap = 0, classes = 0;
   std::vector<int> color;
@@ -333,6 +336,7 @@ std::future<Coloring> start_coloring(const afp_amg_opts& o, int level, const Hos
     c.classes = host_color(ref, cap, c.color);
     return c;
   };
+  if (H.nnz() < kColorInline) return std::async(std::launch::deferred, work);
   try {
     return std::async(std::launch::async, work);
   } catch (const std::system_error&) {  // no thread to be had: when it is asked for
