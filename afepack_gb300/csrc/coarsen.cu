@@ -309,7 +309,7 @@ __global__ void k_cf_pass2_count(int m, const int* __restrict__ rp, const int* _
 // k_cf_pass2_round.  Lists and counts as in k_cf_pass1_wave.  A warp takes a
 // row, or a whole block while a step has no more than `block_rows` rows: on
 // levels of long rows (285 entries: 55 us a row to one warp, and 250 steps
-// one after the other) a row's own time is what a step waits for.
+// one after the other) a row's own time is what a step waits for (wave_block_rows).
 __global__ void __launch_bounds__(kWaveThreads) k_cf_pass2_wave(int m, const int* __restrict__ rp,
                                                                 const int* __restrict__ ci,
                                                                 const double* __restrict__ va,
@@ -533,10 +533,11 @@ __global__ void k_cf_weights(int m, const int* __restrict__ rp, const int* __res
 // chunk are passed round in order.  Rows of P^T longer than kPtCap accumulate
 // and search in global memory.
 constexpr int kPtCap = 256;
-// Mean row length above which a warp takes a row: of 131 entries the whole
-// splitting 2.7 ms against 10 (18,476 rows of a 3D P2 20^3 hierarchy);
-// of 7 to 15 a thread each 3.33 against 3.67 (64^3), 2.14 against 2.27 (48^3).
-constexpr double kWarpWeightsLen = 24.0;
+// Mean row length above which a warp takes a row.  The whole splitting with a
+// warp and with a thread (ms): 7.0 entries 8.99 and 8.66 (361,201 rows), 14.5 2.31
+// and 2.19 (48^3), 14.6 4.03 and 3.69 (64^3); 21 1.86 and 1.97 (2D P2 220^2), 24
+// 0.98 and 1.29 (121^2), 41 1.39 and 2.07, 131 2.7 and 10.2 (3D P2 20^3).
+constexpr double kWarpWeightsLen = 18.0;
 
 // acc + the values v of the lanes in `which`, added in lane order
 __device__ __forceinline__ double add_in_order(double acc, double v, unsigned which) {
@@ -668,6 +669,13 @@ int run_rounds(const afp_context* ctx, int m, DevBuf<int>& counter, F launch, co
   }
 }
 
+// Pass 2: a step of at most so many rows gives each a whole block.  The whole
+// splitting with 0, 96 and 512 (ms), by mean row length: 15 entries 2.18, 2.66
+// and 4.37 (48^3), 28 2.17, 2.29 and 2.80 (3D P2 20^3), 56 2.83, 2.83 and 2.94;
+// 68 1.77, 1.64 and 1.80, 73 3.56, 3.40 and 3.83 (40^3), 76 8.6, 8.9 and 9.2 (64^3),
+// 131 2.67, 2.69 and 3.01; 273 14.0, 10.7 and 10.9 (48^3), 285 20.2, 17.5 and 17.9.
+int wave_block_rows(double len) { return len > 64.0 ? 96 : 0; }
+
 // Launches a wave kernel as one cluster, of 16 blocks where the device can
 // place one that large, else of the portable 8.
 template <class... K, class... Args>
@@ -720,7 +728,7 @@ int gpu_project(const afp_context* ctx, int64_t m64, const int* rp, const int* c
   k_cf_pass2_candidates<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), st1.get(), s2.get());
   k_cf_pass2_count<<<warp_grid, 256, 0, s>>>(m, rp, ci, va, beta.get(), s2.get(), cnt.get());
   launch_wave(ctx, "C/F pass 2", kWaveThreads / 32 * kSet * sizeof(int), k_cf_pass2_wave, m, rp, ci, va, (const double*)beta.get(), (const int*)st1.get(),
-              s2.get(), cnt.get(), list.get(), waves.get() + 3, waves.get() + 7, waves.get() + 8, len > 64.0 ? 96 : 0);
+              s2.get(), cnt.get(), list.get(), waves.get() + 3, waves.get() + 7, waves.get() + 8, wave_block_rows(len));
   int hw[3] = {0, 0, 0};
   copy(ctx, hw, waves.get() + 6, sizeof(hw));
   sync(ctx);

@@ -687,12 +687,13 @@ void galerkin_product(const afp_context* ctx, int64_t n_c, int64_t n_f, const in
   const int rmax = extent.first, window = extent.second;
   AFP_REQUIRE(rmax <= (BLOCK_CAP * 3) / 4, AFP_ERR_UNSUPPORTED,
               "Galerkin product row longer than the block-level table");
-  // Lanes per coarse row.  Few where rows of P^T are short: mean 3.4 entries
-  // 0.42, 0.49 and 0.59 ms with 8, 16 and 32 lanes (2D P2 121^2), 4.3 2.4, 2.3
-  // and 3.4 (64^3), 5.8 0.92, 0.82 and 0.94, 6.8 2.8, 2.3 and 2.6 (3D P2 20^3).
-  // Long rows of the product take a warp: their accumulators and bitmaps in
-  // shared memory bound the groups of an SM (285 entries a row, mean 13: 27 ms
-  // with 32 lanes, 33 with 16, 46 with 8; both phases).  A slot is found by rank where the row windows' bitmaps fit 12 KB a group
+  // Lanes per coarse row, by the mean row of P^T: all lanes of a group take one
+  // such row's entries.  Both phases with 8, 16 and 32 lanes (ms): mean 3.3
+  // 0.45, 0.50 and 0.60 (2D P2 121^2), 4.2 0.59, 0.65 and 0.93 (40^3), 4.3 2.4,
+  // 2.3 and 3.4 (64^3); 5.8 1.9, 1.7 and 2.2 (2D P2 220^2), 6.9 4.9, 3.7 and 4.3
+  // (3D P2 24^3); 10.6 3.0, 3.3 and 2.7 (2D P1 300^2), 11.6 6.0, 4.9 and 3.8, 12.9
+  // 46, 33 and 27 (64^3), 20.1 14.4, 10.5 and 10.2.  A slot is found by rank where
+  // the row windows' bitmaps fit 12 KB a group
   // (64K columns; 0.3 KB for the lattice numbering of a 64^3 mesh), else by
   // binary search.  A group's accumulator is the longest row; blocks of 4, 2
   // or 1 warps, so that two blocks fit an SM, and wider groups if not even
@@ -712,7 +713,7 @@ void galerkin_product(const afp_context* ctx, int64_t n_c, int64_t n_f, const in
   const size_t gb = ((size_t)acc_cap * sizeof(double) + search_bytes + 15) / 16 * 16;
   const bool gacc = gb > NUM_SMEM_MAX;
   const size_t group_bytes = gacc ? (rank ? (search_bytes + 15) / 16 * 16 : 16) : gb;
-  int G = mean <= 5.0 ? 8 : mean <= 16.0 && out.nnz <= 200 * n_c ? 16 : 32;
+  int G = mean <= 5.0 ? 8 : mean <= 10.0 ? 16 : 32;
   while (G < 32 && (size_t)(32 / G) * group_bytes > NUM_SMEM_MAX / 2) G *= 2;
   if (gacc) G = 32;
   int warps = 4;
