@@ -275,3 +275,21 @@ def test_route_of_the_batched_tail(ctx, n_side, k, precision, digits):
     amg.pcg_multi(right_hand_sides(A, k, 20), 1e-6, 50)
     _, nbytes = amg.time_kernel(4, 0, 1)
     assert nbytes == n * n * (20 if digits else 8) + 2 * n * k * (4 if precision else 8)
+
+
+@pytest.mark.parametrize("first_bad", [0, 250, 300, 520])
+def test_pivot_that_turns_out_not_positive(ctx, first_bad):
+    """Symmetric, unit diagonal, no entry above it, yet indefinite from row first_bad on (in the first panel of the
+    symmetric sweep, across its edge, in the second and in the third): the pivoted sweep takes over from the start."""
+    n = 600
+    A = np.eye(n)
+    i = np.arange(n - 1)
+    A[i, i + 1] = A[i + 1, i] = np.where(i >= first_bad, -0.6, -0.3)
+    amg = hierarchy(ctx, A)
+    b = np.random.default_rng(21).uniform(-1.0, 1.0, n)
+    x = np.zeros(n)
+    amg.solve(x, b, step=0)
+    want = np.linalg.solve(A, b)
+    assert np.linalg.eigvalsh(A)[0] < -0.1
+    # two sweeps without pivoting across panels, each with growth of a few units
+    assert np.linalg.norm(x - want) <= 100 * n * EPS * np.linalg.cond(A) * np.linalg.norm(want)
