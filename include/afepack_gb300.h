@@ -314,7 +314,12 @@ afp_status afp_pcg_solve(afp_amg *amg, double *x, const double *b, double tol, i
                          afp_solve_info *info);
 /* nrhs systems with the same matrix; X and B are n x nrhs row-major.  One
  * batched launch per kernel serves all right-hand sides; every column has
- * its own CG recurrences and stopping test. info may be NULL or nrhs long. */
+ * its own CG recurrences and stopping test. info may be NULL or nrhs long.
+ * The first batched solve of a hierarchy (or its batch server) cuts a large
+ * dense tail's inverse into digits for the tensor cores: 20 bytes an entry
+ * (rows padded to 128, columns to 512; 1.0 GB at 6,744 rows) beside the
+ * inverse's own 8, held until the hierarchy is set up again or destroyed.
+ * Where they do not fit, the row kernels are used. */
 afp_status afp_pcg_solve_multi(afp_amg *amg, double *X, const double *B, int nrhs, double tol,
                                int maxit, afp_solve_info *info);
 
