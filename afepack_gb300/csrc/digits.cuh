@@ -120,7 +120,9 @@ __device__ __forceinline__ void cut_row(const double (&v)[H][8], int lane, int64
           *reinterpret_cast<const uint4*>(d);
     }
   }
-  if (lane == 0) *scale = finite ? pow2(ex - 6 + shift) : __longlong_as_double(0x7ff8000000000000LL);
+  // (a scale beyond the range of normal numbers is taken to its end: below it the row counts for nothing either way)
+  if (lane == 0)
+    *scale = finite ? pow2(min(1023, max(-1022, ex - 6 + shift))) : __longlong_as_double(0x7ff8000000000000LL);
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

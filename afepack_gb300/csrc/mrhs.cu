@@ -826,8 +826,9 @@ void ensure_state(afp_amg* h, int k) {
   S->active.alloc(ctx, MAXK);
   // The dense tail by digits from digit_tail_rows on, if it is symmetric
   // positive definite: its diagonal then bounds its entries, and scaling by it
-  // keeps their digits.  Other tails, smaller ones, and where the device has no
-  // room for the digits (20 bytes an entry), the row kernels.
+  // keeps their digits, as long as it spans no more than 2^34.  Other tails,
+  // smaller ones, and where the device has no room for the digits (20 bytes an
+  // entry), the row kernels.
   const Level& T = h->lv[h->t];
   if (h->tail_dense && h->tail_spd && T.n >= digit_tail_rows(mixed, k)) {
     try {

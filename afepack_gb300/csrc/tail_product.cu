@@ -33,8 +33,15 @@ namespace {
 constexpr int kChunk = 512, kChunkStages = kChunk / kKC;
 static_assert(kTailEntryBytes == 2.0 * kDigits, "kTailEntryBytes");
 
-// e[i] with 2^e T_ii 2^e in [1/2, 2) (T from inv, or from hi + lo);
-// *flag = 1 unless every T_ii is a number in [2^-400, 2^400].
+// The largest difference of the rows' exponents with which the digits are used.
+// A residual whose entries are of their matrix rows' size spreads, scaled, by as
+// many bits as the exponents do; a column's digits count from its largest
+// entry, and of their 70 bits FP64's 53 are to be left to the smallest.
+constexpr int kSpread = 7 * kDigits - 53;
+
+// e[i] with 2^e T_ii 2^e in [1/2, 2) (T from inv, or from hi + lo).  *flag (3
+// words, zeros): not zero unless every T_ii is a number in [2^-400, 2^400]; the
+// largest of 512 + e and of 512 - e.
 __global__ void k_tail_exponents(int64_t n, const double* __restrict__ inv, const float* __restrict__ hi,
                                  const float* __restrict__ lo, int64_t ld, int* __restrict__ e,
                                  int* __restrict__ flag) {
@@ -42,8 +49,11 @@ __global__ void k_tail_exponents(int64_t n, const double* __restrict__ inv, cons
   if (i >= n) return;
   const int64_t q = i * ld + i;
   const double d = inv != nullptr ? inv[q] : (double)hi[q] + (double)lo[q];
-  if (!(d >= 0x1p-400 && d <= 0x1p400)) *flag = 1;
-  e[i] = balance(d);
+  if (!(d >= 0x1p-400 && d <= 0x1p400)) flag[0] = 1;
+  const int b = balance(d);
+  e[i] = b;
+  atomicMax(flag + 1, 512 + b);
+  atomicMax(flag + 2, 512 - b);
 }
 
 // T scaled and cut: rows and columns by 2^e; the rows' own 2^-e into their scales
@@ -188,14 +198,14 @@ bool tail_digits(const afp_context* ctx, int64_t n, const double* inv, const flo
   D.np = (n + kTM - 1) / kTM * kTM;
   D.chunks = (int)((n + kChunk - 1) / kChunk);
   D.ex.alloc(ctx, n);
-  DevBuf<int> flag(ctx, 1);
+  DevBuf<int> flag(ctx, 3);
   flag.zero();
   k_tail_exponents<<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, inv, hi, lo, ld, D.ex.get(), flag.get());
   check_launch(ctx, "tail exponents");
-  int bad = 0;
-  flag.download(&bad, 1);
+  int hf[3] = {0, 0, 0};
+  flag.download(hf, 3);
   sync(ctx);
-  if (bad) return false;
+  if (hf[0] || hf[1] + hf[2] - 1024 > kSpread) return false;
   D.dig.alloc(ctx, (size_t)D.np * D.chunks * kChunk * kDigits);
   D.scale.alloc(ctx, (size_t)D.np * D.chunks);
   k_tail_cut<<<dim3((unsigned)(D.np / 8), (unsigned)D.chunks), 256, 0, ctx->stream>>>(

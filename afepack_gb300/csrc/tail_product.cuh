@@ -29,7 +29,8 @@ struct TailWork {
 
 // From the inverse of a symmetric positive definite matrix in FP64 (row stride
 // ld), or from its FP32 pair hi + lo.  False, with nothing allocated that
-// counts, if its diagonal is not positive or of extreme size.
+// counts, if its diagonal is not positive, of extreme size or of too wide a
+// range (a factor above 2^34) for a column's digits.
 bool tail_digits(const afp_context* ctx, int64_t n, const double* inv, const float* hi, const float* lo, int64_t ld,
                  TailDigits& D);
 void tail_work(const afp_context* ctx, const TailDigits& D, int k, TailWork& W);

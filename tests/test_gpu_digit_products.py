@@ -293,3 +293,24 @@ def test_pivot_that_turns_out_not_positive(ctx, first_bad):
     assert np.linalg.eigvalsh(A)[0] < -0.1
     # two sweeps without pivoting across panels, each with growth of a few units
     assert np.linalg.norm(x - want) <= 100 * n * EPS * np.linalg.cond(A) * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("exponent,digits", [(-390, False), (-240, False), (-9, False), (-8, True), (0, True),
+                                             (8, True), (9, False), (240, False), (390, False)])
+def test_tail_with_rows_of_two_sizes(native, ctx, exponent, digits):
+    """Rows of size 2^(2 exponent) and of 2^(-2 exponent), coupled by 2^-905 of their diagonals alone: for a solution
+    of one size their residuals' scaled entries are 2^(2 exponent) apart, and a chunk that holds nothing but such a
+    coupling has a scale far from its row's.  Digits up to a spread of 2^34, row by row beyond; in either case the
+    product is good to rounding in both kinds of rows."""
+    n, k = 1100, 5
+    i = np.arange(400)
+    e = 2 * exponent if abs(exponent) < 100 else exponent
+    d = np.where(np.arange(n) < 550, 2.0 ** e, 2.0 ** -e)
+    A = np.diag(8.0 * d)
+    A[i, i + 600] = A[i + 600, i] = -(2.0 ** -905)
+    amg = hierarchy(ctx, A)
+    want = np.random.default_rng(22).uniform(-1.0, 1.0, (n, k))
+    X = one_step(native, amg, want * 8.0 * d[:, None])  # the coupling is far below rounding
+    assert np.abs(X - want).max() <= 8 * n * EPS
+    _, nbytes = amg.time_kernel(4, 0, 1)
+    assert nbytes == n * n * (20 if digits else 8) + 2 * n * k * 8
